@@ -180,6 +180,17 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long *b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
 }
 
+// F[row, col0 .. col0 + NC) -= v (real rows of the factor), rows and columns inside the given ends.
+template <int NC>
+__device__ __forceinline__ void subtract_direct(const JobDev &J, int row, int col0, int row_end, int col_end,
+                                                const uint32_t (&v)[NC]) {
+  if (row >= row_end) return;
+  float *f = static_cast<float *>(J.F) + row;
+#pragma unroll
+  for (int j = 0; j < NC; ++j)
+    if (col0 + j < col_end) f[(size_t)(col0 + j) * 2 * J.ld] -= __uint_as_float(v[j]);
+}
+
 // Persistent: one CTA per SM loops over the launch's tiles.  Warp 0 (one thread) streams the
 // operand chunks through a 2-stage ring; warp 1 owns TMEM (2 x 256 columns) and issues the MMAs
 // of tile i into accumulator i % 2; warps 2..5 drain the other accumulator meanwhile (tcgen05.ld ->
@@ -303,7 +314,9 @@ __global__ void __launch_bounds__(192, 1)
     // F by one TMA reduce-add (cp.reduce.async.bulk.tensor .add.f32): the read-modify-write of the
     // C tile happens in L2, asynchronously to the SM.  Rows/columns of a tile beyond the trailing
     // block land in F's padding (rows/columns N..ld-1, never read) or are clipped at the tensor
-    // bounds.
+    // bounds.  After a job's last step k + kb = n, and an odd n (an odd number of (lmax + 1)^2 = 9
+    // blocks) would start the reduce-add on 8 bytes, off its 16-byte boundary: such a tile is added
+    // element by element from the registers, only inside the trailing block.
     const int q = warp & 3;
     const int rl = q * 32 + lane;  // real row within the tile
     const bool issuer = (warp == 2 && lane == 0);
@@ -326,8 +339,10 @@ __global__ void __launch_bounds__(192, 1)
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (!sm.ep_ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int fx = 2 * (k + kb) + row0;  // float row coordinate in F (multiple of 4)
+      const int fx = 2 * (k + kb) + row0;  // float row coordinate in F
       const int fy = k + kb + col0;        // column coordinate in F
+      const bool aligned = (fx & 3) == 0;
+      const JobDev &J = jobs[z];
       for (int piece = 0; piece < kTN / kPieceCols; ++piece, ++pcount) {
         float *ps = sm.ep[pcount & 1];
         if (issuer) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // ps is free again
@@ -346,13 +361,18 @@ __global__ void __launch_bounds__(192, 1)
               : "r"(taddr)
               : "memory");
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (aligned) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) ps[(c16 + j) * kTM + rl] = -__uint_as_float(v[j]);
+            for (int j = 0; j < 16; ++j) ps[(c16 + j) * kTM + rl] = -__uint_as_float(v[j]);
+          } else {
+            subtract_direct<16>(J, fx + rl, fy + piece * kPieceCols + c16, 2 * J.N, J.N, v);
+            __syncwarp();
+          }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (issuer) {
-          asm volatile(
+          if (aligned) asm volatile(
               "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
                   &tF),
               "r"(fx), "r"(fy + piece * kPieceCols), "r"(z), "r"(su32(ps))
@@ -730,6 +750,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
       const bool rows_in = wr0 < 2 * rest;
       const int fx = 2 * (k + kb) + wr0;
       const int fy = k + kb + col0;
+      const bool aligned = (fx & 3) == 0;  // (as in the single-CTA kernel)
       for (int piece = 0; piece < kTN / kPieceCols; ++piece, ++pcount) {
         float *ps = wbuf[pcount & 1];
         if (lead) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // ps is free again
@@ -747,15 +768,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
             : "r"(taddr)
             : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (aligned) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) ps[j * 32 + lane] = -__uint_as_float(v[j]);
+          for (int j = 0; j < 32; ++j) ps[j * 32 + lane] = -__uint_as_float(v[j]);
+        } else {
+          subtract_direct<32>(jobs[z], fx + lane, fy + piece * kPieceCols, 2 * jobs[z].N, jobs[z].N, v);
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         // pieces wholly outside the trailing block (this warp's rows past it, or columns past it)
         // are not written; their group is committed empty, so that the wait above always covers
         // the reduce that last read the staging buffer
         if (lead) {
-          if (rows_in && col0 + piece * kPieceCols < rest)
+          if (aligned && rows_in && col0 + piece * kPieceCols < rest)
             asm volatile(
                 "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
                     &tFw),
