@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "cplx.cuh"
+#include "dmma.cuh"
 #include "gj.cuh"
 
 namespace b200 {
@@ -26,9 +27,8 @@ namespace {
 
 using namespace cx;
 
-constexpr int kT = 64;   // GEMM tile
-constexpr int kKc = 16;  // K chunk
-enum { kOverwrite = 0, kSubtract = 1 };
+using dm::kOverwrite;
+using dm::kSubtract;
 
 struct GemmView {
   const double2 *A;
@@ -38,85 +38,23 @@ struct GemmView {
   int m, n, K;
 };
 
-// C (m x n) = A B  [kOverwrite, C may alias B: a CTA reads all of its B tile before writing]
+// C (m x n) = A B  [kOverwrite, C may alias B: one row of tiles, so a CTA reads all of its columns of
+// B before it writes them]
 // C (m x n) -= A B [kSubtract]
-// 64 x 64 complex tile per CTA, 256 threads, 4 x 4 FP64 complex accumulators per thread, operands
-// double-buffered through shared memory in K chunks of 16.
-template <class Op, int MODE>
-__global__ void __launch_bounds__(256) zgemm_view_kernel(const JobDev *__restrict__ jobs, int k, Op op) {
+// Tiles of 16 WM x 16 WN on the FP64 tensor cores (dmma.cuh), in columns of `len`.
+template <class Op, int WM, int WN, int MODE>
+__global__ void __launch_bounds__(dm::kThreads, WM == 4 ? 3 : 4)
+    zgemm_view_kernel(const JobDev *__restrict__ jobs, int k, Op op, int len) {
+  extern __shared__ __align__(16) double2 vsm64[];
+  using TL = dm::Tile<WM, WN>;
   const JobDev &J = jobs[blockIdx.z];
   GemmView g;
   if (!op(J, k, g)) return;
-  const int row0 = blockIdx.y * kT, col0 = blockIdx.x * kT;
+  const int row0 = blockIdx.y * len * TL::kRows, col0 = blockIdx.x * TL::kCols;
   if (row0 >= g.m || col0 >= g.n) return;
-  const int m = min(kT, g.m - row0), n = min(kT, g.n - col0), K = g.K;
-  const double2 *__restrict__ Ab = g.A + row0;
-  const double2 *__restrict__ Bb = g.B + (size_t)col0 * g.ldb;
-  double2 *Cb = g.C + row0 + (size_t)col0 * g.ldc;
-  extern __shared__ __align__(16) unsigned char zsm[];
-  double2(*As)[kKc][kT] = reinterpret_cast<double2(*)[kKc][kT]>(zsm);  // As[buf][kk][row]
-  double2(*Bs)[kKc][kT] = reinterpret_cast<double2(*)[kKc][kT]>(zsm + 2 * kKc * kT * sizeof(double2));
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const double2 zero = make_double2(0.0, 0.0);
-  double2 acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = zero;
-  double2 ra[4], rb[4];
-  auto load_chunk = [&](int kc) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + q * 256;
-      const int ar = e & 63, ak = e >> 6;
-      ra[q] = (ar < m && kc + ak < K) ? Ab[(size_t)ar + (size_t)(kc + ak) * g.lda] : zero;
-      const int bk = e & 15, bc = e >> 4;
-      rb[q] = (bc < n && kc + bk < K) ? Bb[(size_t)(kc + bk) + (size_t)bc * g.ldb] : zero;
-    }
-  };
-  auto store_chunk = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + q * 256;
-      As[buf][e >> 6][e & 63] = ra[q];
-      Bs[buf][e & 15][e >> 4] = rb[q];
-    }
-  };
-  const int nchunks = (K + kKc - 1) / kKc;
-  load_chunk(0);
-  store_chunk(0);
-  __syncthreads();
-  for (int ch = 0; ch < nchunks; ++ch) {
-    const int buf = ch & 1;
-    if (ch + 1 < nchunks) load_chunk((ch + 1) * kKc);
-#pragma unroll
-    for (int kk = 0; kk < kKc; ++kk) {
-      double2 a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[buf][kk][tx + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[buf][kk][ty + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = cfma(a[i], b[j], acc[i][j]);
-    }
-    if (ch + 1 < nchunks) store_chunk(buf ^ 1);
-    __syncthreads();
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int c = ty + 16 * j;
-    if (c >= n) continue;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = tx + 16 * i;
-      if (r >= m) continue;
-      double2 *dst = Cb + (size_t)r + (size_t)c * g.ldc;
-      *dst = MODE == kOverwrite ? acc[i][j] : csub(*dst, acc[i][j]);
-    }
-  }
+  dm::zgemm_column<WM, WN, MODE>(g.A + row0, g.lda, g.B + (size_t)col0 * g.ldb, g.ldb,
+                                 g.C + row0 + (size_t)col0 * g.ldc, g.ldc, min(len * TL::kRows, g.m - row0),
+                                 min(TL::kCols, g.n - col0), g.K, vsm64);
 }
 
 // --- the passes of V = M^-1 = U^-1 S^-1 L^-1 over the block factors in F (positions order) ---
@@ -219,16 +157,26 @@ __global__ void __launch_bounds__(256) schur_inverse_kernel(const JobDev *__rest
   }
 }
 
+template <class Op, int WM, int WN, int MODE>
+cudaError_t gemm_launch_tile(const JobDev *jobs, int njobs, int k, int max_m, int max_n, cudaStream_t s) {
+  using TL = dm::Tile<WM, WN>;
+  const cudaError_t e = ensure_smem(zgemm_view_kernel<Op, WM, WN, MODE>, TL::kSmem);
+  if (e != cudaSuccess) return e;
+  const int tx = (max_n + TL::kCols - 1) / TL::kCols, ty = (max_m + TL::kRows - 1) / TL::kRows;
+  const int len = dm::column_tiles((long)tx * ty * njobs);
+  zgemm_view_kernel<Op, WM, WN, MODE>
+      <<<dim3(tx, (ty + len - 1) / len, njobs), dm::kThreads, TL::kSmem, s>>>(jobs, k, Op(), len);
+  return cudaGetLastError();
+}
+
+// kOverwrite: at most 64 rows, one row of 64 x 32 tiles.  kSubtract: 32 x 32 tiles, as in the
+// elimination's update.
 template <class Op, int MODE>
 cudaError_t gemm_launch(const JobDev *jobs, int njobs, int k, int max_m, int max_n, cudaStream_t s,
                         long *launches) {
   if (max_m <= 0 || max_n <= 0) return cudaSuccess;
-  const int smem = 4 * kKc * kT * (int)sizeof(double2);
-  cudaError_t e = ensure_smem(zgemm_view_kernel<Op, MODE>, smem);
-  if (e != cudaSuccess) return e;
-  zgemm_view_kernel<Op, MODE><<<dim3((max_n + kT - 1) / kT, (max_m + kT - 1) / kT, njobs), 256, smem, s>>>(jobs, k, Op());
   if (launches) *launches += 1;
-  return cudaGetLastError();
+  return gemm_launch_tile<Op, MODE == kOverwrite ? 4 : 2, 2, MODE>(jobs, njobs, k, max_m, max_n, s);
 }
 
 // One CTA per (LIZ position p, job): with G in M's storage, X refined and V = M^-1,

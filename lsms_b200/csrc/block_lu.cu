@@ -9,9 +9,10 @@
 // Here M is stored with the central site last and eliminated top-down in 64-column steps on the
 // factor storage F (FP64 or FP32):
 //   diag_inverse_kernel   D = A11^-1, Gauss-Jordan with partial pivoting inside the block (FP64)
-//   zgemm_tile<kOverwrite> W = D A12 in place over the block row
-//   zgemm_tile<kSubtract>  A22 -= A21 W over the trailing matrix (the O(N^3) part; the mixed path
-//                          replaces this launch by the tensor-core kernel in tc_update.cu)
+//   W = D A12 in place over the block row
+//   A22 -= A21 W over the trailing matrix (the O(N^3) part)
+// FP64 factors take both as tiles on the FP64 tensor cores (dmma.cuh); FP32 factors as FP32 tiles
+// (zgemm_tile_kernel), or the update on the TF32 tensor cores (tc_update.cu).
 // After n = N - b columns the trailing b x b block holds S = 1 - Delta and F holds, in place, the
 // block factors {D_k in the diagonal blocks, A21_k below them, W_k to their right}.
 // Without refinement, finalize solves S tau00 = t0.  With refinement (the reference's zcgesv /
@@ -28,16 +29,13 @@
 
 #include "common.cuh"
 #include "cplx.cuh"
+#include "dmma.cuh"
 #include "gj.cuh"
 
 namespace b200 {
 namespace {
 
 using namespace cx;
-
-template <typename S> struct Vec2;
-template <> struct Vec2<double> { using t = double2; };
-template <> struct Vec2<float> { using t = float2; };
 
 // ---------------------------------------------------------------------------------------------
 // In-place inverse of the kb x kb diagonal block at (k, k) of F, kb <= 64: FP64 Gauss-Jordan with
@@ -228,16 +226,16 @@ void launch_diag_inverse(bool packed, const JobDev *jobs, int njobs, int k, int 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Complex GEMM tile on F (SIMT), C (m x n) = A (m x K) B (K x n)  [kOverwrite, in place over B]
-//                                C (m x n) -= A (m x K) B (K x n) [kSubtract]
-// 64 x 64 complex tile per CTA, 256 threads, 4 x 4 complex accumulators per thread in the storage
-// precision S; operands double-buffered through shared memory in K-chunks of 16.  Thread (tx, ty)
+// Complex GEMM tile on FP32 factors (SIMT), C (m x n) = A (m x K) B (K x n)  [kOverwrite, in place over B]
+//                                           C (m x n) -= A (m x K) B (K x n) [kSubtract]
+// 64 x 64 complex tile per CTA, 256 threads, 4 x 4 complex accumulators per thread; operands double-buffered through shared memory in K-chunks of 16.  Thread (tx, ty)
 // owns rows tx + 16 i and columns ty + 16 j so consecutive lanes touch consecutive rows of the
 // column-major matrix.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTile = 64;
 constexpr int kKc = 16;
-enum { kOverwrite = 0, kSubtract = 1 };
+using dm::kOverwrite;
+using dm::kSubtract;
 
 // Optional second output of the W = D A12 tiles (FP32, tensor-core path): W's hi/lo TF32 split in
 // the K-major operand layout of the trailing update (column c of the trailing block at
@@ -258,10 +256,10 @@ __device__ __forceinline__ float tf32_round(float x) {
   return __uint_as_float(r);
 }
 
-template <typename S, int MODE>
+template <int MODE>
 __device__ __forceinline__ void zgemm_tile_body(const JobDev &J, int k, int bx, int by, int bx0, int by0,
                                                 const PackB &pk = PackB(), int z = 0) {
-  using T = typename Vec2<S>::t;
+  using T = float2;
   const int N = J.N, ld = J.ld;
   if (k >= J.n || J.inactive) return;
   const int kb = min(kNb, J.n - k);
@@ -293,7 +291,7 @@ __device__ __forceinline__ void zgemm_tile_body(const JobDev &J, int k, int bx, 
   T(*Bs)[kKc][kTile] = reinterpret_cast<T(*)[kKc][kTile]>(zsm + 2 * kKc * kTile * sizeof(T));
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
-  const T zero = {S(0), S(0)};
+  const T zero = make_float2(0.f, 0.f);
 
   T acc[4][4];
 #pragma unroll
@@ -358,12 +356,12 @@ __device__ __forceinline__ void zgemm_tile_body(const JobDev &J, int k, int bx, 
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = tx + 16 * i;
-      if (MODE == kOverwrite && sizeof(S) == 4 && pk.hi != nullptr) {
+      if (MODE == kOverwrite && pk.hi != nullptr) {
         // rows past kb pack as zero
         const int shift = pk.shift_k >= 0 ? min(kNb, J.n - pk.shift_k) : 0;
         const int prow = (bx + bx0) * kTile + c - shift;
         if (prow >= 0) {
-          const float wr = r < m ? (float)acc[i][j].x : 0.f, wi = r < m ? (float)acc[i][j].y : 0.f;
+          const float wr = r < m ? acc[i][j].x : 0.f, wi = r < m ? acc[i][j].y : 0.f;
           const float hr = tf32_round(wr), hi = tf32_round(wi);
           const size_t o = (size_t)z * pk.slot + (size_t)prow * kTcKMax + pk.k_off;
           reinterpret_cast<float2 *>(pk.hi + o)[r] = make_float2(hr, hi);
@@ -382,40 +380,92 @@ __device__ __forceinline__ void zgemm_tile_body(const JobDev &J, int k, int bx, 
   }
 }
 
-// One output tile per (bx, by, job).  Launched either with that 3-D grid, or with a smaller 1-D
-// grid whose CTAs loop over the tiles (the FP64 re-solve of a mixed wave, where most jobs are
-// inactive and a full grid would spend its time launching CTAs that exit at once).
-// Two resident CTAs per SM: with K = 64 per step each CTA runs only four K-chunks, so its operand
-// prologue and C read-modify-write latencies are hidden by the other CTA's FMAs.
-// Tiles start at column tile bx0 and row tile by0 of the step's trailing block.
-template <typename S, int MODE>
-__global__ void __launch_bounds__(256, 2) zgemm_tile_kernel(const JobDev *__restrict__ jobs, int k, int tx, int ty,
-                                                            int nj, PackB pk, int bx0, int by0 = 0) {
-  if (gridDim.z == (unsigned)nj && gridDim.x == (unsigned)tx && gridDim.y == (unsigned)ty) {
-    zgemm_tile_body<S, MODE>(jobs[blockIdx.z], k, blockIdx.x, blockIdx.y, bx0, by0, pk, blockIdx.z);
-    return;
-  }
-  // looping grid: jobs one after another (an inactive job costs one check), its tiles spread
-  // over the CTAs
-  const int nblk = gridDim.x * gridDim.y * gridDim.z;
-  const int b0 = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  for (int bz = 0; bz < nj; ++bz) {
-    const JobDev &J = jobs[bz];
-    if (J.inactive || k >= J.n) continue;
-    for (int vb = b0; vb < tx * ty; vb += nblk) zgemm_tile_body<S, MODE>(J, k, vb % tx, vb / tx, bx0, by0);
-  }
+// One output tile per (bx, by, job).  Two resident CTAs per SM: with K = 64 per step each CTA runs
+// only four K-chunks, so its operand prologue and C read-modify-write latencies are hidden by the
+// other CTA's FMAs.  Tiles start at column tile bx0 and row tile by0 of the step's trailing block.
+template <int MODE>
+__global__ void __launch_bounds__(256, 2) zgemm_tile_kernel(const JobDev *__restrict__ jobs, int k, PackB pk, int bx0,
+                                                            int by0 = 0) {
+  zgemm_tile_body<MODE>(jobs[blockIdx.z], k, blockIdx.x, blockIdx.y, bx0, by0, pk, blockIdx.z);
 }
-
 
 // Step k's update of the two strips a paired step k2 = k + 64 needs before its own W (block
 // pivoting): block column k2 below its diagonal block (CTAs x < t1: row tiles 1 .. t1) and block
 // row k2 right of it (x >= t1: column tiles 1 .. t1), one grid of 2 t1 x njobs CTAs, so that the
 // last wave of one strip shares the GPU with the other.
-template <typename S>
 __global__ void __launch_bounds__(256, 2) zgemm_strips_kernel(const JobDev *__restrict__ jobs, int k, int t1) {
   const int x = blockIdx.x;
-  if (x < t1) zgemm_tile_body<S, kSubtract>(jobs[blockIdx.z], k, 0, x, 0, 1);
-  else zgemm_tile_body<S, kSubtract>(jobs[blockIdx.z], k, x - t1, 0, 1, 0);
+  if (x < t1) zgemm_tile_body<kSubtract>(jobs[blockIdx.z], k, 0, x, 0, 1);
+  else zgemm_tile_body<kSubtract>(jobs[blockIdx.z], k, x - t1, 0, 1, 0);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same products on FP64 factors, tiles on the FP64 tensor cores (dmma.cuh):
+// step k's W = D A12 (kOverwrite) and A22 -= A21 W (kSubtract).
+// ---------------------------------------------------------------------------------------------
+// A column of `len` tiles of step k's trailing block from tile (bx, by) down.
+__device__ __forceinline__ void update64_column(const JobDev &J, int k, int bx, int by, int len, double2 *sm) {
+  constexpr int R = dm::Tile<2, 2>::kRows, C = dm::Tile<2, 2>::kCols;
+  const int N = J.N, ld = J.ld;
+  const int kb = min(kNb, J.n - k);
+  double2 *F = static_cast<double2 *>(J.F);
+  const int col0 = k + kb + bx * C, row0 = k + kb + by * R;
+  if (col0 >= N || row0 >= N) return;
+  dm::zgemm_column<2, 2, kSubtract>(F + (size_t)row0 + (size_t)k * ld, ld, F + (size_t)k + (size_t)col0 * ld, ld,
+                                      F + (size_t)row0 + (size_t)col0 * ld, ld, min(len * R, N - row0),
+                                      min(C, N - col0), kb, sm);
+}
+
+// Which tiles of the trailing block an update launch covers: all, the ones of its first 64 x 64
+// (the next step's diagonal block), or the others.
+enum { kAllTiles = 0, kFirstBlock = 1, kOtherTiles = 2 };
+
+// W = D A12 overwrites its own operand, so a CTA takes all kb rows of its columns.
+template <int WN>
+__global__ void __launch_bounds__(dm::kThreads, 2) zgemm64_w_kernel(const JobDev *__restrict__ jobs, int k) {
+  extern __shared__ __align__(16) double2 zsm64[];
+  const JobDev &J = jobs[blockIdx.z];
+  if (k >= J.n || J.inactive) return;
+  const int ld = J.ld, kb = min(kNb, J.n - k);
+  double2 *F = static_cast<double2 *>(J.F);
+  const int col0 = k + kb + blockIdx.x * dm::Tile<4, WN>::kCols;
+  if (col0 >= J.N) return;
+  double2 *A12 = F + (size_t)k + (size_t)col0 * ld;
+  dm::zgemm_column<4, WN, kOverwrite>(F + (size_t)k + (size_t)k * ld, ld, A12, ld, A12, ld, kb,
+                                      min(dm::Tile<4, WN>::kCols, J.N - col0), kb, zsm64);
+}
+
+// 32 x 32 tiles in columns of `len`: tx columns of tiles, ty rows of columns.  Four CTAs of four warps
+// on an SM: 31 jobs of N = 2160 took 32.3 ms of updates with 64 x 64 tiles at two CTAs, 28.4 with
+// 64 x 32 at three, 27.9 with these at four (48.2 -> 30.0 ms for the whole elimination, from DFMA tiles
+// without look-ahead).
+__global__ void __launch_bounds__(dm::kThreads, 4) zgemm64_update_kernel(const JobDev *__restrict__ jobs, int k, int tx,
+                                                                         int ty, int nj, int part, int len) {
+  extern __shared__ __align__(16) double2 zsm64[];
+  using TL = dm::Tile<2, 2>;
+  if (gridDim.z == (unsigned)nj) {
+    const JobDev &J = jobs[blockIdx.z];
+    const int bx = blockIdx.x;
+    int by = blockIdx.y * len, l = len;
+    if (k >= J.n || J.inactive) return;
+    if (part == kOtherTiles && bx * TL::kCols < kNb) {  // without the first 64 rows
+      const int skip = max(0, min(l, kNb / TL::kRows - by));
+      by += skip;
+      l -= skip;
+      if (l <= 0) return;
+    }
+    update64_column(J, k, bx, by, l, zsm64);
+    return;
+  }
+  // a 1-D grid smaller than the tiles (the FP64 re-solve of a mixed wave, where most jobs are
+  // inactive and a full grid would spend its time launching CTAs that exit at once): jobs one
+  // after another (an inactive job costs one check), its columns spread over the CTAs
+  for (int z = 0; z < nj; ++z) {
+    const JobDev &J = jobs[z];
+    if (J.inactive || k >= J.n) continue;
+    for (int v = blockIdx.x; v < tx * ty; v += gridDim.x)
+      update64_column(J, k, v % tx, (v / tx) * len, len, zsm64);
+  }
 }
 
 // out = tau00 (out_mode 1) or rotate(tau00 - t0) (out_mode 0), tau00 in A[r][b + c].
@@ -531,14 +581,6 @@ __host__ __device__ constexpr int residual_smem_bytes() {
   return kResStages * kResK * (residual_rows<BC>() + BC) * (int)sizeof(double2);
 }
 
-// D (8 x 8) += A (8 x 4) B (4 x 8) in FP64 on the tensor cores, per warp: lane l holds
-// a = A[l / 4][l % 4], b = B[l % 4][l / 4] and D[l / 4][2 (l % 4) + i] in d_i.
-__device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-      : "+d"(d0), "+d"(d1)
-      : "d"(a), "d"(b));
-}
-
 // The jobs of a wave still refining: list[0] = their number, list[1..] their indices in order.
 // One warp.
 __global__ void active_list_kernel(const JobDev *__restrict__ jobs, int njobs, int *list) {
@@ -631,10 +673,10 @@ __global__ void __launch_bounds__(kResThreads, 4) residual_kernel(const JobDev *
         const double2 mv = Ms[st][ks + t][wrow + 8 * r + g];
 #pragma unroll
         for (int j = 0; j < NB; ++j) {
-          dmma_884(ar[r][j][0], ar[r][j][1], mv.x, xv[j].x);
-          dmma_884(ar[r][j][0], ar[r][j][1], mv.y, -xv[j].y);
-          dmma_884(ai[r][j][0], ai[r][j][1], mv.x, xv[j].y);
-          dmma_884(ai[r][j][0], ai[r][j][1], mv.y, xv[j].x);
+          dm::mma_884(ar[r][j][0], ar[r][j][1], mv.x, xv[j].x);
+          dm::mma_884(ar[r][j][0], ar[r][j][1], mv.y, -xv[j].y);
+          dm::mma_884(ai[r][j][0], ai[r][j][1], mv.x, xv[j].y);
+          dm::mma_884(ai[r][j][0], ai[r][j][1], mv.y, xv[j].x);
         }
       }
     }
@@ -699,12 +741,11 @@ constexpr int kSparseGrid = 2 * 148;
 // every row), the second stream also runs the next step's row selection and applies its row moves to
 // the columns left of the other tiles, and the main stream applies them to the other columns once
 // their update is done.
-template <typename T, typename S>
 cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int max_N, int *info, cudaStream_t s,
                                 long *launches, KernelTimer *timer, const TcMaps &tc, int *err, const Lookahead &la,
                                 int smem_diag, int smem_gemm, bool panel) {
   cudaError_t e;
-  const FactorKind fk = sizeof(T) == sizeof(double2) ? kFactorFP64 : kFactorFP32;
+  const FactorKind fk = kFactorFP32;
   // SMs left to the second stream's work during the interior update.  The update is a persistent
   // kernel with a fixed share of tiles per CTA, so a CTA of it that cannot start (an inverse took
   // its SM) delays the whole launch: without panel pivoting the inverses, which the scheduler may
@@ -712,7 +753,7 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
   // SM) runs first on the second stream, in waves over the SMs left to it, and the inverses then
   // pack at their occupancy: one wave of those is enough, and the update keeps more SMs.
   int per_sm = 1;
-  if (panel && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, diag_inverse_kernel<T, 2>, kDiagThreads,
+  if (panel && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, diag_inverse_kernel<float2, 2>, kDiagThreads,
                                                                smem_diag) != cudaSuccess ||
                 per_sm < 1)) {
     cudaGetLastError();
@@ -724,7 +765,7 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
     if ((e = launch_panel_select(fk, jobs, njobs, 0, max_n, s, launches)) != cudaSuccess) return e;
     if ((e = launch_row_moves(fk, jobs, njobs, 0, 0, max_N, max_N, s, launches)) != cudaSuccess) return e;
   }
-  launch_diag_inverse<T>(panel, jobs, njobs, 0, info, smem_diag, s);
+  launch_diag_inverse<float2>(panel, jobs, njobs, 0, info, smem_diag, s);
   if (launches) *launches += 1;
   for (int k = 0; k < max_n; k += kNb) {
     const int rest = max_N - k - 1;
@@ -750,28 +791,25 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
       pk0.lo = tc.b_lo;
       pk0.slot = tc.b_slot;
       pk0.shift_k = k2;
-      zgemm_tile_kernel<S, kOverwrite><<<dim3(tiles, 1, njobs), 256, smem_gemm, s>>>(jobs, k, tiles, 1, njobs, pk0, 0);
+      zgemm_tile_kernel<kOverwrite><<<dim3(tiles, 1, njobs), 256, smem_gemm, s>>>(jobs, k, pk0, 0);
       // step k on block column k2, every row below step k (the diagonal block included)
-      zgemm_tile_kernel<S, kSubtract><<<dim3(1, tiles, njobs), 256, smem_gemm, s>>>(jobs, k, 1, tiles, njobs,
-                                                                                   PackB(), 0, 0);
+      zgemm_tile_kernel<kSubtract><<<dim3(1, tiles, njobs), 256, smem_gemm, s>>>(jobs, k, PackB(), 0, 0);
       if ((e = launch_panel_select(fk, jobs, njobs, k2, max_n, s, launches)) != cudaSuccess) return e;
       if ((e = launch_row_moves(fk, jobs, njobs, k2, 0, max_N, max_N, s, launches)) != cudaSuccess) return e;
       // the inverse of the moved diagonal block beside step k's update of block row k2
       if ((e = cudaEventRecord(la.panel, s)) != cudaSuccess) return e;
       if ((e = cudaStreamWaitEvent(la.s2, la.panel, 0)) != cudaSuccess) return e;
-      launch_diag_inverse<T>(true, jobs, njobs, k2, info, smem_diag, la.s2);
+      launch_diag_inverse<float2>(true, jobs, njobs, k2, info, smem_diag, la.s2);
       if ((e = cudaEventRecord(la.diag, la.s2)) != cudaSuccess) return e;
       if (tiles > 1)
-        zgemm_tile_kernel<S, kSubtract><<<dim3(tiles - 1, 1, njobs), 256, smem_gemm, s>>>(jobs, k, tiles - 1, 1,
-                                                                                         njobs, PackB(), 1, 0);
+        zgemm_tile_kernel<kSubtract><<<dim3(tiles - 1, 1, njobs), 256, smem_gemm, s>>>(jobs, k, PackB(), 1, 0);
       if ((e = cudaStreamWaitEvent(s, la.diag, 0)) != cudaSuccess) return e;
       PackB pk1;  // W(k2) -> K half 1
       pk1.hi = tc.b_hi;
       pk1.lo = tc.b_lo;
       pk1.slot = tc.b_slot;
       pk1.k_off = 2 * kNb;
-      zgemm_tile_kernel<S, kOverwrite><<<dim3(tiles2, 1, njobs), 256, smem_gemm, s>>>(jobs, k2, tiles2, 1, njobs,
-                                                                                     pk1, 0);
+      zgemm_tile_kernel<kOverwrite><<<dim3(tiles2, 1, njobs), 256, smem_gemm, s>>>(jobs, k2, pk1, 0);
       const bool timed = timer && timer->used + 2 <= timer->cap;
       if (timed) cudaEventRecord(timer->ev[timer->used++], s);
       if ((e = launch_tc_pack(tc, jobs, njobs, k, 2, k2, max_N, s, false)) != cudaSuccess) return e;
@@ -782,7 +820,7 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
       if ((e = launch_panel_select(fk, jobs, njobs, k2 + kNb, max_n, la.s2, launches)) != cudaSuccess) return e;
       if ((e = launch_row_moves(fk, jobs, njobs, k2 + kNb, 0, split2, max_N, la.s2, launches)) != cudaSuccess)
         return e;
-      launch_diag_inverse<T>(true, jobs, njobs, k2 + kNb, info, smem_diag, la.s2);
+      launch_diag_inverse<float2>(true, jobs, njobs, k2 + kNb, info, smem_diag, la.s2);
       if ((e = cudaEventRecord(la.diag, la.s2)) != cudaSuccess) return e;
       if ((e = launch_tc_update(tc, jobs, njobs, k2, max_N, err, s, 4, tc_num_sms() - free_sms, 2)) != cudaSuccess)
         return e;
@@ -805,24 +843,23 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
       pk0.lo = tc.b_lo;
       pk0.slot = tc.b_slot;
       pk0.shift_k = k2;
-      zgemm_tile_kernel<S, kOverwrite><<<dim3(tiles, 1, njobs), 256, smem_gemm, s>>>(jobs, k, tiles, 1, njobs, pk0, 0);
+      zgemm_tile_kernel<kOverwrite><<<dim3(tiles, 1, njobs), 256, smem_gemm, s>>>(jobs, k, pk0, 0);
       // step k on block column k2 (all rows below step k) and on block row k2 (right of it): first
       // the diagonal block of k2, whose inverse then runs on the second stream beside the rest of
       // the two strips
-      zgemm_tile_kernel<S, kSubtract><<<dim3(1, 1, njobs), 256, smem_gemm, s>>>(jobs, k, 1, 1, njobs, PackB(), 0, 0);
+      zgemm_tile_kernel<kSubtract><<<dim3(1, 1, njobs), 256, smem_gemm, s>>>(jobs, k, PackB(), 0, 0);
       if ((e = cudaEventRecord(la.panel, s)) != cudaSuccess) return e;
       if ((e = cudaStreamWaitEvent(la.s2, la.panel, 0)) != cudaSuccess) return e;
-      launch_diag_inverse<T>(false, jobs, njobs, k2, info, smem_diag, la.s2);
+      launch_diag_inverse<float2>(false, jobs, njobs, k2, info, smem_diag, la.s2);
       if ((e = cudaEventRecord(la.diag, la.s2)) != cudaSuccess) return e;
-      if (tiles > 1) zgemm_strips_kernel<S><<<dim3(2 * (tiles - 1), 1, njobs), 256, smem_gemm, s>>>(jobs, k, tiles - 1);
+      if (tiles > 1) zgemm_strips_kernel<<<dim3(2 * (tiles - 1), 1, njobs), 256, smem_gemm, s>>>(jobs, k, tiles - 1);
       if ((e = cudaStreamWaitEvent(s, la.diag, 0)) != cudaSuccess) return e;
       PackB pk1;  // W(k2) -> K half 1
       pk1.hi = tc.b_hi;
       pk1.lo = tc.b_lo;
       pk1.slot = tc.b_slot;
       pk1.k_off = 2 * kNb;
-      zgemm_tile_kernel<S, kOverwrite><<<dim3(tiles2, 1, njobs), 256, smem_gemm, s>>>(jobs, k2, tiles2, 1, njobs,
-                                                                                     pk1, 0);
+      zgemm_tile_kernel<kOverwrite><<<dim3(tiles2, 1, njobs), 256, smem_gemm, s>>>(jobs, k2, pk1, 0);
       const bool timed = timer && timer->used + 2 <= timer->cap;
       if (timed) cudaEventRecord(timer->ev[timer->used++], s);
       if ((e = launch_tc_pack(tc, jobs, njobs, k, 2, k2, max_N, s, false)) != cudaSuccess) return e;
@@ -830,7 +867,7 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
       if (next2) {
         if ((e = cudaEventRecord(la.panel, s)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(la.s2, la.panel, 0)) != cudaSuccess) return e;
-        launch_diag_inverse<T>(false, jobs, njobs, k2 + kNb, info, smem_diag, la.s2);
+        launch_diag_inverse<float2>(false, jobs, njobs, k2 + kNb, info, smem_diag, la.s2);
         if ((e = cudaEventRecord(la.diag, la.s2)) != cudaSuccess) return e;
       }
       if ((e = launch_tc_update(tc, jobs, njobs, k2, max_N, err, s, 2, next2 ? tc_num_sms() - free_sms : 0, 2)) !=
@@ -849,7 +886,7 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
       pk.hi = tc.b_hi;
       pk.lo = tc.b_lo;
       pk.slot = tc.b_slot;
-      zgemm_tile_kernel<S, kOverwrite><<<dim3(tiles, 1, njobs), 256, smem_gemm, s>>>(jobs, k, tiles, 1, njobs, pk, 0);
+      zgemm_tile_kernel<kOverwrite><<<dim3(tiles, 1, njobs), 256, smem_gemm, s>>>(jobs, k, pk, 0);
       const bool timed = timer && timer->used + 2 <= timer->cap;
       if (timed) cudaEventRecord(timer->ev[timer->used++], s);
       if ((e = launch_tc_pack(tc, jobs, njobs, k, 1, k, max_N, s, false)) != cudaSuccess) return e;
@@ -864,7 +901,7 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
           if ((e = launch_row_moves(fk, jobs, njobs, k + kNb, 0, split, max_N, la.s2, launches)) != cudaSuccess)
             return e;
         }
-        launch_diag_inverse<T>(panel, jobs, njobs, k + kNb, info, smem_diag, la.s2);
+        launch_diag_inverse<float2>(panel, jobs, njobs, k + kNb, info, smem_diag, la.s2);
         if ((e = cudaEventRecord(la.diag, la.s2)) != cudaSuccess) return e;
       }
       if ((e = launch_tc_update(tc, jobs, njobs, k, max_N, err, s, panel ? 4 : 2,
@@ -881,7 +918,7 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
         if ((e = launch_panel_select(fk, jobs, njobs, k + kNb, max_n, s, launches)) != cudaSuccess) return e;
         if ((e = launch_row_moves(fk, jobs, njobs, k + kNb, 0, max_N, max_N, s, launches)) != cudaSuccess) return e;
       }
-      launch_diag_inverse<T>(panel, jobs, njobs, k + kNb, info, smem_diag, s);
+      launch_diag_inverse<float2>(panel, jobs, njobs, k + kNb, info, smem_diag, s);
       if (launches) *launches += 1;
     }
   }
@@ -889,59 +926,101 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
   return cudaGetLastError();
 }
 
-template <typename T, typename S>
-cudaError_t eliminate_impl(const JobDev *jobs, int njobs, int max_n, int max_N, int *info, cudaStream_t s,
-                           long *launches, KernelTimer *timer, const TcMaps *tc, int *err, bool sparse_jobs,
-                           const Lookahead *la, bool panel) {
-  const FactorKind fk = sizeof(T) == sizeof(double2) ? kFactorFP64 : kFactorFP32;
+// FP32 factors.
+cudaError_t eliminate32(const JobDev *jobs, int njobs, int max_n, int max_N, int *info, cudaStream_t s,
+                        long *launches, KernelTimer *timer, const TcMaps *tc, int *err, const Lookahead *la,
+                        bool panel) {
   const int smem_diag = kNb * (kNb + 1) * (int)sizeof(double2);
-  const int smem_gemm = 4 * kKc * kTile * (int)sizeof(T);
+  const int smem_gemm = 4 * kKc * kTile * (int)sizeof(float2);
   cudaError_t e;
-  if ((e = ensure_smem(diag_inverse_kernel<T, 1>, smem_diag)) != cudaSuccess)
-    return e;
-  if ((e = ensure_smem(diag_inverse_kernel<T, 2>, smem_diag)) != cudaSuccess)
-    return e;
-  if ((e = ensure_smem(zgemm_tile_kernel<S, kOverwrite>, smem_gemm)) != cudaSuccess)
-    return e;
-  if ((e = ensure_smem(zgemm_tile_kernel<S, kSubtract>, smem_gemm)) != cudaSuccess)
-    return e;
-  if ((e = ensure_smem(zgemm_strips_kernel<S>, smem_gemm)) != cudaSuccess)
-    return e;
+  if ((e = ensure_smem(diag_inverse_kernel<float2, 1>, smem_diag)) != cudaSuccess) return e;
+  if ((e = ensure_smem(diag_inverse_kernel<float2, 2>, smem_diag)) != cudaSuccess) return e;
+  if ((e = ensure_smem(zgemm_tile_kernel<kOverwrite>, smem_gemm)) != cudaSuccess) return e;
+  if ((e = ensure_smem(zgemm_tile_kernel<kSubtract>, smem_gemm)) != cudaSuccess) return e;
+  if ((e = ensure_smem(zgemm_strips_kernel, smem_gemm)) != cudaSuccess) return e;
   // Look-ahead (tensor-core path): the update of step k first covers the tile holding the next
   // step's diagonal block; the next diagonal inverse then runs on the second stream while the other
   // tiles are updated on SMs left free for it (the inverses take one SM per job).
-  if (tc != nullptr && la != nullptr && la->s2 != nullptr && !sparse_jobs)
-    return eliminate_lookahead<T, S>(jobs, njobs, max_n, max_N, info, s, launches, timer, *tc, err, *la, smem_diag,
-                                     smem_gemm, panel);
+  if (tc != nullptr && la != nullptr && la->s2 != nullptr)
+    return eliminate_lookahead(jobs, njobs, max_n, max_N, info, s, launches, timer, *tc, err, *la, smem_diag,
+                               smem_gemm, panel);
   if (panel && (e = launch_pivot_init(jobs, njobs, s, launches)) != cudaSuccess) return e;
   for (int k = 0; k < max_n; k += kNb) {
     if (panel) {
-      if ((e = launch_panel_select(fk, jobs, njobs, k, max_n, s, launches)) != cudaSuccess) return e;
-      if ((e = launch_row_moves(fk, jobs, njobs, k, 0, max_N, max_N, s, launches)) != cudaSuccess) return e;
+      if ((e = launch_panel_select(kFactorFP32, jobs, njobs, k, max_n, s, launches)) != cudaSuccess) return e;
+      if ((e = launch_row_moves(kFactorFP32, jobs, njobs, k, 0, max_N, max_N, s, launches)) != cudaSuccess) return e;
     }
-    launch_diag_inverse<T>(panel, jobs, njobs, k, info, smem_diag, s);
+    launch_diag_inverse<float2>(panel, jobs, njobs, k, info, smem_diag, s);
     const int rest = max_N - k - 1;
     const int tiles = (rest + kTile - 1) / kTile;
     if (launches) *launches += 1;
     if (tiles > 0) {
-      zgemm_tile_kernel<S, kOverwrite><<<dim3(tiles, 1, njobs), 256, smem_gemm, s>>>(jobs, k, tiles, 1, njobs,
-                                                                                   PackB(), 0);
+      zgemm_tile_kernel<kOverwrite><<<dim3(tiles, 1, njobs), 256, smem_gemm, s>>>(jobs, k, PackB(), 0);
       const bool timed = timer && timer->used + 2 <= timer->cap;
       if (timed) cudaEventRecord(timer->ev[timer->used++], s);
       if (tc != nullptr) {
         if ((e = launch_tc_step(*tc, jobs, njobs, k, max_N, err, s)) != cudaSuccess) return e;
         if (launches) *launches += 1;  // pack + update
       } else {
-        if (sparse_jobs)
-          zgemm_tile_kernel<S, kSubtract><<<std::min(tiles * tiles * njobs, kSparseGrid), 256, smem_gemm, s>>>(
-              jobs, k, tiles, tiles, njobs, PackB(), 0);
-        else
-          zgemm_tile_kernel<S, kSubtract><<<dim3(tiles, tiles, njobs), 256, smem_gemm, s>>>(jobs, k, tiles, tiles,
-                                                                                           njobs, PackB(), 0);
+        zgemm_tile_kernel<kSubtract><<<dim3(tiles, tiles, njobs), 256, smem_gemm, s>>>(jobs, k, PackB(), 0);
       }
       if (timed) cudaEventRecord(timer->ev[timer->used++], s);
       if (launches) *launches += 2;
     }
+  }
+  if (panel && (e = launch_pivot_finish(jobs, njobs, s, launches)) != cudaSuccess) return e;
+  return cudaGetLastError();
+}
+
+void launch_update64(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, cudaStream_t s) {
+  using TL = dm::Tile<2, 2>;
+  const int rows = part == kFirstBlock ? kNb : max_N - k - 1;
+  const int tx = (rows + TL::kCols - 1) / TL::kCols, tr = (rows + TL::kRows - 1) / TL::kRows;
+  const int len = sparse ? 1 : dm::column_tiles((long)tx * tr * njobs);
+  const int ty = (tr + len - 1) / len;
+  const dim3 grid = sparse ? dim3(std::min(tx * ty * njobs, kSparseGrid)) : dim3(tx, ty, njobs);
+  zgemm64_update_kernel<<<grid, dm::kThreads, TL::kSmem, s>>>(jobs, k, tx, ty, njobs, part, len);
+}
+
+// FP64 factors.  With a second stream (and pivots inside the diagonal blocks) the update of step k
+// first covers the next diagonal block, whose inverse (a chain of 64 dependent pivot steps on one
+// SM per job) then runs on the second stream beside the rest of the update.
+cudaError_t eliminate64(const JobDev *jobs, int njobs, int max_n, int max_N, int *info, cudaStream_t s,
+                        long *launches, KernelTimer *timer, bool sparse, const Lookahead *la, bool panel) {
+  const int smem_diag = kNb * (kNb + 1) * (int)sizeof(double2);
+  cudaError_t e;
+  if ((e = ensure_smem(diag_inverse_kernel<double2, 1>, smem_diag)) != cudaSuccess) return e;
+  if ((e = ensure_smem(diag_inverse_kernel<double2, 2>, smem_diag)) != cudaSuccess) return e;
+  if ((e = ensure_smem(zgemm64_w_kernel<2>, dm::Tile<4, 2>::kSmem)) != cudaSuccess) return e;
+  if ((e = ensure_smem(zgemm64_update_kernel, dm::Tile<2, 2>::kSmem)) != cudaSuccess) return e;
+  const bool ahead = la != nullptr && la->s2 != nullptr && !sparse && !panel;
+  if (panel && (e = launch_pivot_init(jobs, njobs, s, launches)) != cudaSuccess) return e;
+  for (int k = 0; k < max_n; k += kNb) {
+    if (panel) {
+      if ((e = launch_panel_select(kFactorFP64, jobs, njobs, k, max_n, s, launches)) != cudaSuccess) return e;
+      if ((e = launch_row_moves(kFactorFP64, jobs, njobs, k, 0, max_N, max_N, s, launches)) != cudaSuccess) return e;
+    }
+    if (!ahead || k == 0) {
+      launch_diag_inverse<double2>(panel, jobs, njobs, k, info, smem_diag, s);
+      if (launches) *launches += 1;
+    }
+    const int rest = max_N - k - 1;
+    if (rest <= 0) continue;
+    const bool next = ahead && k + kNb < max_n;
+    zgemm64_w_kernel<2><<<dim3((rest + 31) / 32, 1, njobs), dm::kThreads, dm::Tile<4, 2>::kSmem, s>>>(jobs, k);
+    const bool timed = timer && timer->used + 2 <= timer->cap;
+    if (timed) cudaEventRecord(timer->ev[timer->used++], s);
+    if (next) {
+      launch_update64(jobs, njobs, k, max_N, kFirstBlock, false, s);
+      if ((e = cudaEventRecord(la->panel, s)) != cudaSuccess) return e;
+      if ((e = cudaStreamWaitEvent(la->s2, la->panel, 0)) != cudaSuccess) return e;
+      launch_diag_inverse<double2>(false, jobs, njobs, k + kNb, info, smem_diag, la->s2);
+      if ((e = cudaEventRecord(la->diag, la->s2)) != cudaSuccess) return e;
+    }
+    launch_update64(jobs, njobs, k, max_N, next ? kOtherTiles : kAllTiles, sparse, s);
+    if (timed) cudaEventRecord(timer->ev[timer->used++], s);
+    if (next && (e = cudaStreamWaitEvent(s, la->diag, 0)) != cudaSuccess) return e;
+    if (launches) *launches += next ? 4 : 2;
   }
   if (panel && (e = launch_pivot_finish(jobs, njobs, s, launches)) != cudaSuccess) return e;
   return cudaGetLastError();
@@ -1089,15 +1168,13 @@ cudaError_t launch_eliminate(FactorKind fk, const JobDev *jobs, int njobs, int m
                              cudaStream_t s, long *launches, KernelTimer *timer, const TcMaps *tc,
                              int *err, bool sparse_jobs, const Lookahead *la, bool panel) {
   if (fk == kFactorFP64)
-    return eliminate_impl<double2, double>(jobs, njobs, max_n, max_N, info, s, launches, timer, nullptr, err,
-                                           sparse_jobs, nullptr, panel);
+    return eliminate64(jobs, njobs, max_n, max_N, info, s, launches, timer, sparse_jobs, la, panel);
   if (tc) {
     cudaError_t e = tc_prepare();
     if (e == cudaSuccess) e = launch_tc_counters_reset(*tc, s);
     if (e != cudaSuccess) return e;
   }
-  return eliminate_impl<float2, float>(jobs, njobs, max_n, max_N, info, s, launches, timer, tc, err, sparse_jobs,
-                                       la, panel);
+  return eliminate32(jobs, njobs, max_n, max_N, info, s, launches, timer, tc, err, la, panel);
 }
 
 cudaError_t launch_finalize_direct(FactorKind fk, const JobDev *jobs, int njobs, int ns, int kkrsz, int *info,

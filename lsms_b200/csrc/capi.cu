@@ -1101,7 +1101,10 @@ int b200tau_create(b200tau_ctx **out, int device, int lmax, int n_spin_cant, int
   ctx->blk = (2 * ctx->kkrsz) * (2 * ctx->kkrsz);
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->la.s2, cudaStreamNonBlocking);
+  // the look-ahead's inverses take their SMs before the update's remaining tiles do
+  int least = 0, greatest = 0;
+  if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&ctx->la.s2, cudaStreamNonBlocking, greatest);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->la.panel, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->la.diag, cudaEventDisableTiming);
   AngularTables tab;
@@ -1709,7 +1712,7 @@ int b200tau_solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau
   ctx->launches = 0;
   CK(launch_kkr_build(ctx->d_jobs, 1, a.L, build_params(ctx, p), ctx->d_err, ctx->stream, &ctx->launches));
   CK(launch_eliminate(kFactorFP64, ctx->d_jobs, 1, J.n, J.N, ctx->d_info, ctx->stream, &ctx->launches, nullptr,
-                      nullptr, ctx->d_err, false, nullptr, panel));
+                      nullptr, ctx->d_err, false, &ctx->la, panel));
   CK(launch_inverse(ctx->d_jobs, 1, J.n, J.N, ctx->stream, &ctx->launches));
   CK(launch_tau_full(ctx->d_jobs, 1, a.L, a.N, tmat_view(ctx), ctx->stream, &ctx->launches));
   // reference site order (central site first): rows/cols [0, r) <-> [b, N), [r, N) <-> [0, b)

@@ -43,3 +43,73 @@ def test_mixed_odd_size(solver_factory, lattice, shells, n_reduced, pivoting):
         s.set_pivoting(T.PIVOT_AUTO)
     for i in range(2):
         assert _tau_err(prob, i, out[i]) <= TOL_MIXED
+
+
+def _dense(n, b, seed, shuffle=False):
+    """A well-conditioned complex matrix (condition number of a few tens at most) and a t0; with
+    `shuffle` its rows past the central block are permuted, so that pivots leave the diagonal blocks."""
+    rng = np.random.default_rng(seed)
+    m = np.eye(n) + 0.4 / np.sqrt(n) * (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n)))
+    if shuffle:
+        m[b:] = m[b + rng.permutation(n - b)]
+    t0 = rng.normal(size=(b, b)) + 1j * rng.normal(size=(b, b))
+    rhs = np.zeros((n, b), np.complex128)
+    rhs[:b] = t0
+    return m, t0, np.linalg.solve(m, rhs)[:b]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec,tol", [(T.PREC_FP64, 1e-12), (T.PREC_MIXED, TOL_MIXED)])
+@pytest.mark.parametrize("b", [1, 9, 16, 32])
+@pytest.mark.parametrize("rest", [0, 1, 15, 17, 63, 64, 65, 80, 129, 193, 447])
+def test_dense_edge_sizes(solver_factory, prec, tol, b, rest):
+    """n = b + rest around the 64-column steps, the 16- and 64-row tiles and the 8-wide fragments."""
+    m, t0, want = _dense(b + rest, b, 100 * b + rest)
+    got = solver_factory(3, 1, 1).solve_tau00_dense(m, t0, prec)
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec,tol", [(T.PREC_FP64, 1e-12), (T.PREC_MIXED, TOL_MIXED)])
+@pytest.mark.parametrize("rest", [70, 191, 321, 700])
+def test_dense_panel_pivoting(solver_factory, prec, tol, rest):
+    """Rows in random order: every step's pivots come from below its diagonal block, with the candidates
+    filtered once more than 256 rows are left."""
+    m, t0, want = _dense(16 + rest, 16, rest, shuffle=True)
+    s = solver_factory(3, 1, 1)
+    s.set_pivoting(T.PIVOT_PANEL)
+    try:
+        got = s.solve_tau00_dense(m, t0, prec)
+    finally:
+        s.set_pivoting(T.PIVOT_AUTO)
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lattice,shells,n_reduced", [("bcc", 1, 3), ("bcc", 3, 4), ("fcc", 3, 20)])
+def test_full_tau_and_adjoint_odd_sizes(solver_factory, lattice, shells, n_reduced):
+    """The inverse's tiles at sizes that are no multiple of 16: tau over the LIZ, and the gradients from
+    the dense inverse."""
+    from oracle import port
+    prob = _lmax_step_problem(lattice, shells, n_reduced, 8)
+    s = solver_factory(3, 1, 1)
+    s.load_problem(prob)
+    n, e = prob.nrmat_ns, prob.energies[0]
+    m = port.build_kkr(prob, 0)
+    off = np.concatenate([[0], np.cumsum((prob.liz_lmax + 1) ** 2)])
+    t = [prob.t_block(int(i), 0)[:k, :k] for i, k in zip(prob.liz_store_idx, np.diff(off))]
+    inv = np.linalg.inv(m)
+    want = np.concatenate([inv[:, off[j]:off[j + 1]] @ t[j] for j in range(len(t))], axis=1)
+    got = s.solve_tau_full(0, 0, 0, e, n)
+    assert np.abs(got - want).max() <= 1e-11 * np.abs(want).max()
+    rng = np.random.default_rng(2)
+    bar = rng.normal(size=(16, 16)) + 1j * rng.normal(size=(16, 16))
+    _, tbar, dlog = s.solve_vjp(T.make_jobs([(0, 0, 0, e)]), bar[None], [prob.num_liz])
+    g = np.concatenate([np.linalg.solve(t[j], (np.eye(n) - m)[off[j]:off[j + 1]]) for j in range(len(t))])
+    z, h, lam = g @ (inv[:, :16] @ t[0]), g @ inv, inv[:16].T @ bar
+    scale = max(np.abs(lam).max() * np.abs(z).max(), 1.0)
+    for j in range(len(t)):
+        r, k = slice(off[j], off[j + 1]), off[j + 1] - off[j]
+        wb = lam[r] @ z[r].T + (lam[r] if j == 0 else 0.0)
+        assert np.abs(tbar[0][j][:k, :k] - wb).max() <= 1e-10 * scale
+        assert np.abs(dlog[0][j][:k, :k] + h[r, r].T).max() <= 1e-10 * max(1.0, np.abs(h).max())
