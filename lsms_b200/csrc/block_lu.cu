@@ -48,10 +48,16 @@ using namespace cx;
 // row pv becomes A[pv][c] / d, column p becomes -A[r][p] / d, and A[pv][p] becomes 1/d, as the
 // in-place inverse needs, with no special cases in the update.
 // Layout: warp w holds columns 8w .. 8w + 7 and lane l rows l and l + 32, in registers (the step
-// loop is not unrolled: an unrolled body outgrows the instruction caches).  Per step the warp
-// holding column p finds the pivot (warp argmax) and publishes g; after the one block barrier of
-// the step, in every warp the lane holding row pv publishes u over the warp's columns (a per-warp
-// slot in shared memory, read only by that warp) and all lanes apply the update.
+// loop is not unrolled: an unrolled body outgrows the instruction caches).  A step's update writes each
+// column one place down, so the column to search next is always the first (a selection by index cost
+// 130 instructions of the chain) and after eight steps the columns are back in place.  A launch of one
+// block takes 45 us, some 1250 cycles a step (52 us with the columns in fixed places and the search after
+// the whole update; 59 us with the warps run ahead on one mbarrier per step instead of the block barrier).
+// What bounds the kernel is the chain from one pivot to the next, so in step p the warp that holds
+// column p + 1 updates that column first, searches it (warp argmax, with every lane's reciprocal of
+// its own candidate computed beside the reductions) and publishes step p + 1's g before it updates its
+// other columns; the one block barrier of the step follows.  In every warp the lane holding row pv
+// publishes u over the warp's columns (a per-warp slot in shared memory, read only by that warp).
 // ---------------------------------------------------------------------------------------------
 // Pivot search key of a row: |re| + |im| (non-negative doubles order as their bit patterns; NaN
 // counts as 0) with its 6 low mantissa bits replaced by 63 - row, so that the largest key is the
@@ -80,7 +86,7 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
   __shared__ double2 s_g[2][NB];              // the step's row factors g, by step parity
   __shared__ double2 s_row[kDiagWarps][8];    // per warp: u over the warp's columns
   __shared__ int s_pvp[2];
-  __shared__ int s_sing[2];
+  __shared__ int s_sing;
   __shared__ int s_pv[NB], s_inv[NB];
   T *__restrict__ Fk = static_cast<T *>(J.F) + (size_t)k + (size_t)k * J.ld;
   const int tid = threadIdx.x;
@@ -106,6 +112,7 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
     }
   }
   if (tid < NB) s_inv[tid] = tid;  // every entry in range whatever the pivots
+  if (tid == 0) s_sing = 0;
   __syncthreads();
   const int w = tid >> 5, l = tid & 31;
   double2 a[2][8];
@@ -118,80 +125,77 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
     }
   // rows already pivoted on (rows past kb count as used, so they are never chosen)
   bool used0 = l >= kb, used1 = l + 32 >= kb;
-  bool singular = false;
+  // The pivot of column p, whose rows of this lane are x0 and x1, and step p's g, published.
+  auto search = [&](double2 x0, double2 x1, int p) {
+    // the unused row of largest |re| + |im| as the largest 64-bit key (pivot_key), two warp
+    // max-reductions (high word, then the low word among the lanes holding the high max)
+    const unsigned long long k0 = used0 ? 0ull : pivot_key(cabs1(x0), l);
+    const unsigned long long k1 = used1 ? 0ull : pivot_key(cabs1(x1), l + 32);
+    const bool first = k0 > k1;
+    const unsigned long long kl = first ? k0 : k1;
+    // 1/d = conj(d) / |d|^2 of the lane's candidate (pivots of these blocks are far from the FP64
+    // range limits); 0 for a zero
+    const double2 xs = first ? x0 : x1;
+    const bool zero = xs.x == 0.0 && xs.y == 0.0;
+    const double rr = 1.0 / (zero ? 1.0 : xs.x * xs.x + xs.y * xs.y);
+    const double2 rl = make_double2(xs.x * rr, -xs.y * rr);
+    const unsigned hi = (unsigned)(kl >> 32);
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? (unsigned)kl : 0u);
+    // kb - p unused rows remain, so the key names one of them (a row < kb)
+    const int pv = min(63 - (int)(mlo & 63u), kb - 1);
+    double2 dinv;
+    dinv.x = __shfl_sync(0xffffffffu, rl.x, pv & 31);
+    dinv.y = __shfl_sync(0xffffffffu, rl.y, pv & 31);
+    double2 *g = s_g[p & 1];
+    g[l] = (l == pv) ? make_double2(1.0 - dinv.x, -dinv.y) : cmul(x0, dinv);
+    g[l + 32] = (l + 32 == pv) ? make_double2(1.0 - dinv.x, -dinv.y) : cmul(x1, dinv);
+    if (l == 0) {
+      s_pvp[p & 1] = pv;
+      s_pv[p] = pv;
+      if (dinv.x == 0.0 && dinv.y == 0.0) s_sing = 1;
+    }
+  };
+  if (w == 0) search(a[0][0], a[1][0], 0);
+  __syncthreads();
 #pragma unroll 1
   for (int p = 0; p < kb; ++p) {
-    const int par = p & 1;
-    if (w == (p >> 3)) {
-      // column p & 7 of this warp's registers (opaque copies: the compiler otherwise turns the
-      // selection into an indexed local-memory load)
-      double2 x0 = make_double2(0.0, 0.0), x1 = x0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        double2 t0 = a[0][j], t1 = a[1][j];
-        asm volatile("" : "+d"(t0.x), "+d"(t0.y), "+d"(t1.x), "+d"(t1.y));
-        if (j == (p & 7)) {
-          x0 = t0;
-          x1 = t1;
-        }
-      }
-      // the pivot: the unused row of largest |re| + |im| as the largest 64-bit key (pivot_key),
-      // two warp max-reductions (high word, then the low word among the lanes holding the high max)
-      const unsigned long long k0 = used0 ? 0ull : pivot_key(cabs1(x0), l);
-      const unsigned long long k1 = used1 ? 0ull : pivot_key(cabs1(x1), l + 32);
-      const unsigned long long kl = k0 > k1 ? k0 : k1;
-      const unsigned hi = (unsigned)(kl >> 32);
-      const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-      const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? (unsigned)kl : 0u);
-      // kb - p unused rows remain, so the key names one of them (a row < kb)
-      const int pv = min(63 - (int)(mlo & 63u), kb - 1);
-      const double2 xs = (pv >> 5) ? x1 : x0;
-      double2 d;
-      d.x = __shfl_sync(0xffffffffu, xs.x, pv & 31);
-      d.y = __shfl_sync(0xffffffffu, xs.y, pv & 31);
-      // 1/d = conj(d) / |d|^2 in every lane (pivots of these blocks are far from the FP64 range limits)
-      const bool zero = d.x == 0.0 && d.y == 0.0;
-      double2 dinv = make_double2(0.0, 0.0);
-      if (!zero) {
-        const double rr = 1.0 / (d.x * d.x + d.y * d.y);
-        dinv = make_double2(d.x * rr, -d.y * rr);
-      }
-      s_g[par][l] = (l == pv) ? make_double2(1.0 - dinv.x, -dinv.y) : cmul(x0, dinv);
-      s_g[par][l + 32] = (l + 32 == pv) ? make_double2(1.0 - dinv.x, -dinv.y) : cmul(x1, dinv);
-      if (l == 0) {
-        s_pvp[par] = pv;
-        s_sing[par] = zero ? 1 : 0;
-        s_pv[p] = pv;
-      }
-    }
-    __syncthreads();
-    const int pv = s_pvp[par];
-    if (s_sing[par]) singular = true;
+    // place j holds column 8w + ((p + j) & 7)
+    const int pv = s_pvp[p & 1];
+    const double2 g0 = s_g[p & 1][l], g1 = s_g[p & 1][l + 32];
     const int pl = pv & 31, pi = pv >> 5;
     if (l == pl) {  // publish u over this warp's columns, then mark row pv used
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) {
-        double2 v = pi ? a[1][jj] : a[0][jj];
-        if (8 * w + jj == p) v.x += 1.0;
-        s_row[w][jj] = v;
+      for (int j = 0; j < 8; ++j) {
+        double2 v = pi ? a[1][j] : a[0][j];
+        if (j == 0 && w == (p >> 3)) v.x += 1.0;
+        s_row[w][j] = v;
       }
       if (pi) used1 = true;
       else used0 = true;
     }
     __syncwarp();
-    const double2 g0 = s_g[par][l], g1 = s_g[par][l + 32];
+    auto update = [&](double2 x, double2 g, double2 u) {
+      x.x = fma(-g.x, u.x, x.x);
+      x.x = fma(g.y, u.y, x.x);
+      x.y = fma(-g.x, u.y, x.y);
+      x.y = fma(-g.y, u.x, x.y);
+      return x;
+    };
+    const double2 u1 = s_row[w][1], o0 = a[0][0], o1 = a[1][0];
+    a[0][0] = update(a[0][1], g0, u1);
+    a[1][0] = update(a[1][1], g1, u1);
+    if (p + 1 < kb && w == ((p + 1) >> 3)) search(a[0][0], a[1][0], p + 1);
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
-      const double2 u = s_row[w][jj];
-      a[0][jj].x = fma(-g0.x, u.x, a[0][jj].x);
-      a[0][jj].x = fma(g0.y, u.y, a[0][jj].x);
-      a[0][jj].y = fma(-g0.x, u.y, a[0][jj].y);
-      a[0][jj].y = fma(-g0.y, u.x, a[0][jj].y);
-      a[1][jj].x = fma(-g1.x, u.x, a[1][jj].x);
-      a[1][jj].x = fma(g1.y, u.y, a[1][jj].x);
-      a[1][jj].y = fma(-g1.x, u.y, a[1][jj].y);
-      a[1][jj].y = fma(-g1.y, u.x, a[1][jj].y);
+    for (int j = 2; j < 8; ++j) {
+      const double2 u = s_row[w][j];
+      a[0][j - 1] = update(a[0][j], g0, u);
+      a[1][j - 1] = update(a[1][j], g1, u);
     }
+    const double2 u0 = s_row[w][0];
+    a[0][7] = update(o0, g0, u0);
+    a[1][7] = update(o1, g1, u0);
+    __syncthreads();
   }
   __syncthreads();
   if (tid < kb) s_inv[s_pv[tid]] = tid;
@@ -200,7 +204,7 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int r = l + 32 * i, c = 8 * w + j;
+      const int r = l + 32 * i, c = 8 * w + ((j + kb) & 7);
       if (r < kb && c < kb) As[s_inv[r]][s_pv[c]] = a[i][j];
     }
   __syncthreads();
@@ -216,7 +220,7 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
       stc(Fk + r + (size_t)cc * J.ld, As[r][cc]);
     }
   }
-  if (singular && tid == 0) atomicCAS(&info[blockIdx.x], 0, k + 1);
+  if (s_sing && tid == 0) atomicCAS(&info[blockIdx.x], 0, k + 1);
 }
 
 template <typename T>
