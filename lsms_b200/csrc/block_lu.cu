@@ -232,12 +232,19 @@ void launch_diag_inverse(bool packed, const JobDev *jobs, int njobs, int k, int 
 // ---------------------------------------------------------------------------------------------
 // Complex GEMM tile on FP32 factors (SIMT), C (m x n) = A (m x K) B (K x n)  [kOverwrite, in place over B]
 //                                           C (m x n) -= A (m x K) B (K x n) [kSubtract]
-// 64 x 64 complex tile per CTA, 256 threads, 4 x 4 complex accumulators per thread; operands double-buffered through shared memory in K-chunks of 16.  Thread (tx, ty)
-// owns rows tx + 16 i and columns ty + 16 j so consecutive lanes touch consecutive rows of the
-// column-major matrix.
+// 64 x 64 complex tile per CTA, 256 threads, 4 x 4 complex accumulators per thread, each one packed
+// (re, im) pair: a complex multiply-add is two packed FMAs (fma.rn.f32x2, the same four products and
+// roundings as scalar FMAs), which leaves half the issue slots to the operand loads.  The whole
+// K <= 64 of both operands is requested by cp.async at once, in four K chunks of 16 that are
+// multiplied as they land, so a CTA waits out one memory round trip.  (31 jobs of N = 2160: the
+// elimination's small products 8.97 -> 8.29 ms in all, from scalar FMAs and a two-stage ring.)  Thread (tx, ty) owns rows
+// 2 tx, 2 tx + 1, 32 + 2 tx, 33 + 2 tx (16-byte shared-memory loads and stores) and columns
+// ty + 16 j.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTile = 64;
 constexpr int kKc = 16;
+constexpr int kTileBs = kNb + 2;  // B's columns in shared memory, padded to 16 bytes modulo 128
+constexpr int kTileSmem = (kNb * kTile + kTile * kTileBs) * (int)sizeof(float2);
 using dm::kOverwrite;
 using dm::kSubtract;
 
@@ -258,6 +265,26 @@ __device__ __forceinline__ float tf32_round(float x) {
   unsigned r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
   return __uint_as_float(r);
+}
+
+// Packed (x, y) pairs of FP32 in a 64-bit register, and d += a b elementwise.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+// 16 bytes to shared memory of which the first `bytes` (0, 8 or 16) are read and the rest are zeros.
+__device__ __forceinline__ void cp_async16_part(void *smem, const void *gmem, int bytes) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
 }
 
 template <int MODE>
@@ -291,75 +318,100 @@ __device__ __forceinline__ void zgemm_tile_body(const JobDev &J, int k, int bx, 
   n = min(n, kTile);
 
   extern __shared__ __align__(16) unsigned char zsm[];
-  T(*As)[kKc][kTile] = reinterpret_cast<T(*)[kKc][kTile]>(zsm);  // As[buf][kk][row]
-  T(*Bs)[kKc][kTile] = reinterpret_cast<T(*)[kKc][kTile]>(zsm + 2 * kKc * kTile * sizeof(T));
+  T(*As)[kTile] = reinterpret_cast<T(*)[kTile]>(zsm);                                    // As[kk][row]
+  T(*Bs)[kTileBs] = reinterpret_cast<T(*)[kTileBs]>(zsm + kNb * kTile * sizeof(T));  // Bs[col][kk]
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
-  const T zero = make_float2(0.f, 0.f);
+  const int nchunks = (K + kKc - 1) / kKc;
+  // rows of A start on an odd one (8 bytes off a 16-byte boundary) only after an odd last step
+  const bool aligned = (row0 & 1) == 0;
+#pragma unroll
+  for (int ch = 0; ch < kNb / kKc; ++ch) {
+    if (ch < nchunks) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int e = tid + q * 256;
+        const int r = (e & 31) * 2, kk = ch * kKc + (e >> 5);
+        const int left = kk < K ? max(0, min(2, m - r)) : 0;
+        const T *src = left > 0 ? Ab + r + (size_t)kk * ld : Ab;
+        if (aligned) {
+          cp_async16_part(&As[kk][r], src, 8 * left);
+        } else {
+          As[kk][r] = left > 0 ? src[0] : make_float2(0.f, 0.f);
+          As[kk][r + 1] = left > 1 ? src[1] : make_float2(0.f, 0.f);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int e = tid + q * 256;
+        const int kk = ch * kKc + (e & 7) * 2, c = e >> 3;
+        const int left = c < n ? max(0, min(2, K - kk)) : 0;
+        cp_async16_part(&Bs[c][kk], left > 0 ? Bb + kk + (size_t)c * ld : Bb, 8 * left);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  if (MODE == kSubtract) {  // C's lines on their way to L2 while the product runs
+    const int r = (tid & 3) * 16, c = tid >> 2;
+    if (r < m && c < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(Cb + r + (size_t)c * ld));
+  }
 
+  unsigned long long acc2[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc2[i][j] = 0ull;
+#pragma unroll
+  for (int ch = 0; ch < kNb / kKc; ++ch) {
+    if (ch >= nchunks) break;
+    if (ch == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
+    else if (ch == 1) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else if (ch == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int k2 = 0; k2 < kKc; k2 += 2) {
+      const int kk = ch * kKc + k2;
+      float4 b[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4 *>(&Bs[ty + 16 * j][kk]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 a01 = *reinterpret_cast<const float4 *>(&As[kk + h][2 * tx]);
+        const float4 a23 = *reinterpret_cast<const float4 *>(&As[kk + h][32 + 2 * tx]);
+        const float ar[4] = {a01.x, a01.z, a23.x, a23.z}, ai[4] = {a01.y, a01.w, a23.y, a23.w};
+        unsigned long long bp[4], bs[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float br = h ? b[j].z : b[j].x, bi = h ? b[j].w : b[j].y;
+          bp[j] = pack2(br, bi);
+          bs[j] = pack2(-bi, br);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const unsigned long long ax = pack2(ar[i], ar[i]), ay = pack2(ai[i], ai[i]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            fma2(acc2[i][j], ax, bp[j]);
+            fma2(acc2[i][j], ay, bs[j]);
+          }
+        }
+      }
+    }
+  }
   T acc[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = zero;
-
-  T ra[4], rb[4];
-  auto load_chunk = [&](int kc) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + q * 256;
-      const int ar = e & 63, ak = e >> 6;
-      const int kg = kc + ak;
-      ra[q] = (ar < m && kg < K) ? Ab[(size_t)ar + (size_t)kg * ld] : zero;
-      const int bk = e & 15, bc = e >> 4;
-      const int kg2 = kc + bk;
-      rb[q] = (bc < n && kg2 < K) ? Bb[(size_t)kg2 + (size_t)bc * ld] : zero;
-    }
-  };
-  auto store_chunk = [&](int buf) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + q * 256;
-      As[buf][e >> 6][e & 63] = ra[q];
-      Bs[buf][e & 15][e >> 4] = rb[q];
-    }
-  };
-
-  const int nchunks = (K + kKc - 1) / kKc;
-  load_chunk(0);
-  store_chunk(0);
-  __syncthreads();
-  for (int ch = 0; ch < nchunks; ++ch) {
-    const int buf = ch & 1;
-    if (ch + 1 < nchunks) load_chunk((ch + 1) * kKc);
-#pragma unroll
-    for (int kk = 0; kk < kKc; ++kk) {
-      T a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[buf][kk][tx + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[buf][kk][ty + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
-          acc[i][j].x = fma(-a[i].y, b[j].y, acc[i][j].x);
-          acc[i][j].y = fma(a[i].x, b[j].y, acc[i][j].y);
-          acc[i][j].y = fma(a[i].y, b[j].x, acc[i][j].y);
-        }
-    }
-    if (ch + 1 < nchunks) store_chunk(buf ^ 1);
-    __syncthreads();
-  }
-  // for kOverwrite every read of B = C happened before the last __syncthreads
+    for (int j = 0; j < 4; ++j) acc[i][j] = unpack2(acc2[i][j]);
+  // for kOverwrite every read of B = C (into shared memory) happened before the last __syncthreads
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int c = ty + 16 * j;
     if (c >= n) continue;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int r = tx + 16 * i;
+      const int r = 2 * tx + (i & 1) + 32 * (i >> 1);
       if (MODE == kOverwrite && pk.hi != nullptr) {
         // rows past kb pack as zero
         const int shift = pk.shift_k >= 0 ? min(kNb, J.n - pk.shift_k) : 0;
@@ -935,7 +987,7 @@ cudaError_t eliminate32(const JobDev *jobs, int njobs, int max_n, int max_N, int
                         long *launches, KernelTimer *timer, const TcMaps *tc, int *err, const Lookahead *la,
                         bool panel) {
   const int smem_diag = kNb * (kNb + 1) * (int)sizeof(double2);
-  const int smem_gemm = 4 * kKc * kTile * (int)sizeof(float2);
+  const int smem_gemm = kTileSmem;
   cudaError_t e;
   if ((e = ensure_smem(diag_inverse_kernel<float2, 1>, smem_diag)) != cudaSuccess) return e;
   if ((e = ensure_smem(diag_inverse_kernel<float2, 2>, smem_diag)) != cudaSuccess) return e;
