@@ -28,6 +28,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "cluster.cuh"
 #include "cplx.cuh"
 #include "dmma.cuh"
 #include "gj.cuh"
@@ -624,6 +625,10 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 // through a three-stage cp.async ring in shared memory (kResK columns of M and rows of X per
 // stage), so two stages of loads are in flight while one is multiplied.
 // BC = 16 or 32 is the padded column count (b <= BC).
+// A late refinement round has a few jobs left, 17 row blocks each at N = 2160: then a row block's K
+// range is split over up to the 8 CTAs of a cluster, whose partial sums are added through
+// distributed shared memory in rank order (a round on one job took 241 us with one CTA per row
+// block, the latency of its 270 stages, and takes 51 us split in eight).
 constexpr int kResK = 8;       // K per stage
 constexpr int kResStages = 3;
 
@@ -632,9 +637,16 @@ template <int BC>
 __host__ __device__ constexpr int residual_rows() {
   return kResThreads * 16 / BC;
 }
+constexpr int kResCluster = 8;  // CTAs per cluster, and the most that share a row block
+// Row blocks x split the launch aims at: one full wave of four CTAs per SM.
+constexpr int kResWave = 4 * 148;
+// The rows of a stage are padded by two elements: a fragment load's eight lanes of a 128-byte phase (two
+// rows or columns, four k) then hit eight different 16-byte banks, where unpadded rows put the four k
+// of a row on the same one.
+constexpr int kResPad = 2;
 template <int BC>
 __host__ __device__ constexpr int residual_smem_bytes() {
-  return kResStages * kResK * (residual_rows<BC>() + BC) * (int)sizeof(double2);
+  return kResStages * kResK * (residual_rows<BC>() + BC + 2 * kResPad) * (int)sizeof(double2);
 }
 
 // The jobs of a wave still refining: list[0] = their number, list[1..] their indices in order.
@@ -652,32 +664,32 @@ __global__ void active_list_kernel(const JobDev *__restrict__ jobs, int njobs, i
   if (lane == 0) list[0] = count;
 }
 
-// Without a list: grid (jobs, row blocks), converged jobs leave at once.  With `active` (from
-// active_list_kernel): a 1-D grid whose first count x rowblocks CTAs take (active job i % count,
-// row block i / count), so the jobs still refining spread evenly over the SMs; the rest leave.
+// Work item i is row block i / count of the i % count-th job: of the jobs listed in `active`
+// (active_list_kernel), so that the jobs still refining spread evenly over the SMs, or of all njobs.
+// With few items, `split` CTAs of a cluster share one item, each over its share of K.
 template <int BC>
-__global__ void __launch_bounds__(kResThreads, 4) residual_kernel(const JobDev *__restrict__ jobs,
-                                                                  const int *__restrict__ active, int rowblocks) {
+__global__ void __cluster_dims__(kResCluster, 1, 1) __launch_bounds__(kResThreads, 4)
+    residual_kernel(const JobDev *__restrict__ jobs, const int *__restrict__ active, int njobs, int rowblocks) {
   constexpr int ROWS = residual_rows<BC>();  // rows per CTA
   constexpr int RT = ROWS / 32;              // 8-row tiles per warp (four warps)
   constexpr int NB = BC / 8;                 // 8-column blocks
   static_assert(kResThreads == 128 && RT * 32 == ROWS && NB * 8 == BC && kResK % 4 == 0, "residual layout");
-  int jw = blockIdx.x, rb = blockIdx.y;
-  if (active != nullptr) {
-    const int cnt = active[0], i = blockIdx.x;
-    if (i >= cnt * rowblocks) return;
-    jw = active[1 + i % cnt];
-    rb = i / cnt;
-  }
-  const JobDev &J = jobs[jw];
-  if (converged(J) || J.inactive) return;
+  const int cnt = active != nullptr ? active[0] : njobs;
+  int split = kResCluster;  // the same in every CTA
+  while (split > 1 && cnt * rowblocks * split > kResWave) split >>= 1;
+  const int item = blockIdx.x / split, slice = blockIdx.x % split;
+  if ((int)(blockIdx.x / kResCluster) * (kResCluster / split) >= cnt * rowblocks) return;  // (the whole cluster)
+  const bool valid = item < cnt * rowblocks;
+  const int ji = valid ? item % cnt : 0, rb = valid ? item / cnt : 0;
+  const JobDev &J = jobs[active != nullptr ? active[1 + ji] : ji];
   const int N = J.N, ld = J.ld, b = J.b;
   const int row0 = rb * ROWS;
-  if (row0 >= N) return;
+  const bool live = valid && !converged(J) && !J.inactive && row0 < N;
+  if (split == 1 && !live) return;
   extern __shared__ __align__(16) unsigned char rsm[];
-  double2(*Ms)[kResK][ROWS] = reinterpret_cast<double2(*)[kResK][ROWS]>(rsm);
-  double2(*Xs)[kResK][BC] =
-      reinterpret_cast<double2(*)[kResK][BC]>(rsm + sizeof(double2) * kResStages * kResK * ROWS);
+  double2(*Ms)[kResK][ROWS + kResPad] = reinterpret_cast<double2(*)[kResK][ROWS + kResPad]>(rsm);
+  double2(*Xs)[kResK][BC + kResPad] = reinterpret_cast<double2(*)[kResK][BC + kResPad]>(
+      rsm + sizeof(double2) * kResStages * kResK * (ROWS + kResPad));
   const int tid = threadIdx.x;
   const int lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int wrow = (tid >> 5) * (8 * RT);  // the warp's first row within the CTA's rows
@@ -706,17 +718,19 @@ __global__ void __launch_bounds__(kResThreads, 4) residual_kernel(const JobDev *
   for (int r = 0; r < RT; ++r)
 #pragma unroll
     for (int j = 0; j < NB; ++j) ar[r][j][0] = ar[r][j][1] = ai[r][j][0] = ai[r][j][1] = 0.0;
-  const int nst = (N + kResK - 1) / kResK;
+  // this CTA's stages [q0, q0 + nst) of the K range
+  const int stages = (N + kResK - 1) / kResK, per = (stages + split - 1) / split;
+  const int q0 = slice * per, nst = live ? max(0, min(per, stages - q0)) : 0;
 #pragma unroll
   for (int q = 0; q < kResStages - 1; ++q) {
-    if (q < nst) stage(q * kResK, q);
+    if (q < nst) stage((q0 + q) * kResK, q);
     else asm volatile("cp.async.commit_group;" ::: "memory");
   }
   for (int q = 0; q < nst; ++q) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kResStages - 2) : "memory");
     __syncthreads();  // stage q landed for every thread; stage q - 1 is no longer read
     const int nq = q + kResStages - 1;
-    if (nq < nst) stage(nq * kResK, nq % kResStages);
+    if (nq < nst) stage((q0 + nq) * kResK, nq % kResStages);
     else asm volatile("cp.async.commit_group;" ::: "memory");
     const int st = q % kResStages;
 #pragma unroll
@@ -740,21 +754,48 @@ __global__ void __launch_bounds__(kResThreads, 4) residual_kernel(const JobDev *
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   // with panel pivoting the factors are those of P M: row gr of R goes to its physical row
   const int *__restrict__ rowpos = J.piv != nullptr ? J.piv + ld : nullptr;
-#pragma unroll
-  for (int r = 0; r < RT; ++r) {
-    const int gr = row0 + wrow + 8 * r + g;
-    if (gr >= N) continue;
+  // entry e = (r * NB + j) * 2 + i of this thread
+  auto put = [&](int e, double2 v) {
+    const int gr = row0 + wrow + 8 * (e / (2 * NB)) + g, c = 8 * ((e / 2) % NB) + 2 * t + (e & 1);
+    if (gr >= N || c >= b) return;
     const int dst = rowpos != nullptr ? rowpos[gr] : gr;
+    const double2 bv = (gr >= J.n) ? J.t0[(gr - J.n) + (size_t)c * J.t0_ld] : zero;
+    J.R[(size_t)dst + (size_t)c * ld] = make_double2(bv.x - v.x, bv.y - v.y);
+  };
+  constexpr int E = RT * NB * 2;
+  if (split == 1) {
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) put((r * NB + j) * 2 + i, make_double2(ar[r][j][i], ai[r][j][i]));
+    return;
+  }
+  // partial sums to shared memory; CTA `slice` of the item adds up its share of the entries
+  static_assert(E * kResThreads * (int)sizeof(double2) <= residual_smem_bytes<BC>(), "partial sums fit the ring");
+  double2 *part = reinterpret_cast<double2 *>(rsm);
+  __syncthreads();  // the ring is no longer read
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
 #pragma unroll
     for (int j = 0; j < NB; ++j)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int c = 8 * j + 2 * t + i;
-        if (c >= b) continue;
-        const double2 bv = (gr >= J.n) ? J.t0[(gr - J.n) + (size_t)c * J.t0_ld] : zero;
-        J.R[(size_t)dst + (size_t)c * ld] = make_double2(bv.x - ar[r][j][i], bv.y - ai[r][j][i]);
+      for (int i = 0; i < 2; ++i)
+        part[((r * NB + j) * 2 + i) * kResThreads + tid] = make_double2(ar[r][j][i], ai[r][j][i]);
+  cl::cluster_sync();
+  if (live) {
+    const int first = cl::cluster_rank() - slice;
+    for (int e = slice * (E / split); e < (slice + 1) * (E / split); ++e) {
+      double2 v = zero;
+      for (int c = 0; c < split; ++c) {
+        const double2 p = cl::ld_remote(cl::remote_u32(part + e * kResThreads + tid, first + c));
+        v = make_double2(v.x + p.x, v.y + p.y);
       }
+      put(e, v);
+    }
   }
+  cl::cluster_sync();  // no CTA leaves while another reads its partial sums
 }
 
 // Y[n:N] = S^-1 rhs with rhs = R[n:N] (mode 1) or t0 (mode 0, which also zeroes Y[0:n]).
@@ -1258,12 +1299,11 @@ cudaError_t launch_residual(const JobDev *jobs, int njobs, int max_N, int *activ
   const cudaError_t e = ensure_smem(residual_kernel<BC>, sm);
   if (e != cudaSuccess) return e;
   const int rowblocks = (max_N + residual_rows<BC>() - 1) / residual_rows<BC>();
-  if (active) {
-    active_list_kernel<<<1, 32, 0, s>>>(jobs, njobs, active);
-    residual_kernel<BC><<<njobs * rowblocks, kResThreads, sm, s>>>(jobs, active, rowblocks);
-  } else {
-    residual_kernel<BC><<<dim3(njobs, rowblocks), kResThreads, sm, s>>>(jobs, nullptr, rowblocks);
-  }
+  if (active) active_list_kernel<<<1, 32, 0, s>>>(jobs, njobs, active);
+  // room for every item alone, or for the split of the few items that are split
+  int grid = std::max(njobs * rowblocks, std::min(njobs * rowblocks * kResCluster, kResWave));
+  grid = (grid + kResCluster - 1) / kResCluster * kResCluster;
+  residual_kernel<BC><<<grid, kResThreads, sm, s>>>(jobs, active, njobs, rowblocks);
   return cudaGetLastError();
 }
 
