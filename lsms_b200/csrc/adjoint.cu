@@ -141,8 +141,6 @@ __global__ void __launch_bounds__(256) schur_inverse_kernel(const JobDev *__rest
   const JobDev &J = jobs[blockIdx.x];
   const int b = J.b, n = J.n, ld = J.ld;
   __shared__ double2 A[kMaxB][2 * kMaxB + 1];
-  __shared__ int s_piv;
-  __shared__ double2 s_dinv;
   const double2 *S = static_cast<const double2 *>(J.F) + (size_t)n + (size_t)n * ld;
   for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
     const int c = e / b, r = e - c * b;
@@ -150,7 +148,7 @@ __global__ void __launch_bounds__(256) schur_inverse_kernel(const JobDev *__rest
     A[r][b + c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
   }
   __syncthreads();
-  gj_solve_smem(A, b, &s_piv, &s_dinv);  // a singular S was already reported by the forward solve
+  gj_solve_smem(A, b);  // a singular S was already reported by the forward solve
   for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
     const int c = e / b, r = e - c * b;
     J.Y[(size_t)r + (size_t)c * ld] = A[r][b + c];

@@ -60,14 +60,6 @@ using namespace cx;
 // other columns; the one block barrier of the step follows.  In every warp the lane holding row pv
 // publishes u over the warp's columns (a per-warp slot in shared memory, read only by that warp).
 // ---------------------------------------------------------------------------------------------
-// Pivot search key of a row: |re| + |im| (non-negative doubles order as their bit patterns; NaN
-// counts as 0) with its 6 low mantissa bits replaced by 63 - row, so that the largest key is the
-// largest value, ties - and values within 2^-46 relative of each other - going to the lowest row.
-__device__ __forceinline__ unsigned long long pivot_key(double v, int row) {
-  v = (v == v) ? v : 0.0;
-  return ((unsigned long long)__double_as_longlong(v) & ~63ull) | (unsigned long long)(63 - row);
-}
-
 constexpr int kDiagThreads = 256;
 constexpr int kDiagWarps = kDiagThreads / 32;
 static_assert(kDiagWarps * 8 == kNb && kNb == 64, "diagonal inverse layout: 8 columns per warp, 2 rows per lane");
@@ -128,8 +120,7 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
   bool used0 = l >= kb, used1 = l + 32 >= kb;
   // The pivot of column p, whose rows of this lane are x0 and x1, and step p's g, published.
   auto search = [&](double2 x0, double2 x1, int p) {
-    // the unused row of largest |re| + |im| as the largest 64-bit key (pivot_key), two warp
-    // max-reductions (high word, then the low word among the lanes holding the high max)
+    // the unused row of largest |re| + |im|, as the largest 64-bit key
     const unsigned long long k0 = used0 ? 0ull : pivot_key(cabs1(x0), l);
     const unsigned long long k1 = used1 ? 0ull : pivot_key(cabs1(x1), l + 32);
     const bool first = k0 > k1;
@@ -140,11 +131,8 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
     const bool zero = xs.x == 0.0 && xs.y == 0.0;
     const double rr = 1.0 / (zero ? 1.0 : xs.x * xs.x + xs.y * xs.y);
     const double2 rl = make_double2(xs.x * rr, -xs.y * rr);
-    const unsigned hi = (unsigned)(kl >> 32);
-    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? (unsigned)kl : 0u);
     // kb - p unused rows remain, so the key names one of them (a row < kb)
-    const int pv = min(63 - (int)(mlo & 63u), kb - 1);
+    const int pv = min(pivot_row(kl), kb - 1);
     double2 dinv;
     dinv.x = __shfl_sync(0xffffffffu, rl.x, pv & 31);
     dinv.y = __shfl_sync(0xffffffffu, rl.y, pv & 31);
@@ -176,26 +164,19 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
       else used0 = true;
     }
     __syncwarp();
-    auto update = [&](double2 x, double2 g, double2 u) {
-      x.x = fma(-g.x, u.x, x.x);
-      x.x = fma(g.y, u.y, x.x);
-      x.y = fma(-g.x, u.y, x.y);
-      x.y = fma(-g.y, u.x, x.y);
-      return x;
-    };
     const double2 u1 = s_row[w][1], o0 = a[0][0], o1 = a[1][0];
-    a[0][0] = update(a[0][1], g0, u1);
-    a[1][0] = update(a[1][1], g1, u1);
+    a[0][0] = cfnma(a[0][1], g0, u1);
+    a[1][0] = cfnma(a[1][1], g1, u1);
     if (p + 1 < kb && w == ((p + 1) >> 3)) search(a[0][0], a[1][0], p + 1);
 #pragma unroll
     for (int j = 2; j < 8; ++j) {
       const double2 u = s_row[w][j];
-      a[0][j - 1] = update(a[0][j], g0, u);
-      a[1][j - 1] = update(a[1][j], g1, u);
+      a[0][j - 1] = cfnma(a[0][j], g0, u);
+      a[1][j - 1] = cfnma(a[1][j], g1, u);
     }
     const double2 u0 = s_row[w][0];
-    a[0][7] = update(o0, g0, u0);
-    a[1][7] = update(o1, g1, u0);
+    a[0][7] = cfnma(o0, g0, u0);
+    a[1][7] = cfnma(o1, g1, u0);
     __syncthreads();
   }
   __syncthreads();
@@ -575,8 +556,6 @@ __global__ void __launch_bounds__(256) finalize_direct_kernel(const JobDev *__re
   const JobDev &J = jobs[blockIdx.x];
   const int b = J.b;
   __shared__ double2 A[kMaxB][2 * kMaxB + 1];
-  __shared__ int s_piv;
-  __shared__ double2 s_dinv;
   const T *Sb = static_cast<const T *>(J.F) + (size_t)J.n + (size_t)J.n * J.ld;
   for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
     const int c = e / b, r = e - c * b;
@@ -584,7 +563,7 @@ __global__ void __launch_bounds__(256) finalize_direct_kernel(const JobDev *__re
     A[r][b + c] = J.t0[r + (size_t)c * J.t0_ld];
   }
   __syncthreads();
-  if (gj_solve_smem(A, b, &s_piv, &s_dinv) && threadIdx.x == 0) atomicCAS(&info[blockIdx.x], 0, -1);
+  if (gj_solve_smem(A, b) && threadIdx.x == 0) atomicCAS(&info[blockIdx.x], 0, -1);
   write_out(J, A, ns, kkrsz);
 }
 
@@ -806,8 +785,6 @@ __global__ void __launch_bounds__(256) schur_solve_kernel(const JobDev *__restri
   if ((mode == 1 && converged(J)) || J.inactive) return;
   const int b = J.b, n = J.n, ld = J.ld;
   __shared__ double2 A[kMaxB][2 * kMaxB + 1];
-  __shared__ int s_piv;
-  __shared__ double2 s_dinv;
   const T *Sb = static_cast<const T *>(J.F) + (size_t)n + (size_t)n * ld;
   for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
     const int c = e / b, r = e - c * b;
@@ -820,7 +797,7 @@ __global__ void __launch_bounds__(256) schur_solve_kernel(const JobDev *__restri
       J.Y[(size_t)r + (size_t)c * ld] = make_double2(0.0, 0.0);
     }
   __syncthreads();
-  if (gj_solve_smem(A, b, &s_piv, &s_dinv) && threadIdx.x == 0) atomicCAS(&info[blockIdx.x], 0, -1);
+  if (gj_solve_smem(A, b) && threadIdx.x == 0) atomicCAS(&info[blockIdx.x], 0, -1);
   for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
     const int c = e / b, r = e - c * b;
     J.Y[(size_t)(n + r) + (size_t)c * ld] = A[r][b + c];
