@@ -777,7 +777,7 @@ __global__ void __cluster_dims__(kResCluster, 1, 1) __launch_bounds__(kResThread
   cl::cluster_sync();  // no CTA leaves while another reads its partial sums
 }
 
-// Y[n:N] = S^-1 rhs with rhs = R[n:N] (mode 1) or t0 (mode 0, which also zeroes Y[0:n]).
+// Y[n:N] = S^-1 rhs with rhs = R[n:N] (mode 1) or t0 (mode 0, whose backward sweep takes Y[0:n] as 0).
 template <typename T>
 __global__ void __launch_bounds__(256) schur_solve_kernel(const JobDev *__restrict__ jobs, int mode,
                                                           int *info) {
@@ -791,11 +791,6 @@ __global__ void __launch_bounds__(256) schur_solve_kernel(const JobDev *__restri
     A[r][c] = ldc(Sb + r + (size_t)c * ld);
     A[r][b + c] = mode == 0 ? J.t0[r + (size_t)c * J.t0_ld] : J.R[(size_t)(n + r) + (size_t)c * ld];
   }
-  if (mode == 0)
-    for (int e = threadIdx.x; e < n * b; e += blockDim.x) {
-      const int r = e % n, c = e / n;
-      J.Y[(size_t)r + (size_t)c * ld] = make_double2(0.0, 0.0);
-    }
   __syncthreads();
   if (gj_solve_smem(A, b) && threadIdx.x == 0) atomicCAS(&info[blockIdx.x], 0, -1);
   for (int e = threadIdx.x; e < b * b; e += blockDim.x) {

@@ -131,11 +131,11 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
       : "memory");
 }
 
-// Grid (cs, njobs) of `threads`-thread CTAs in clusters of (cs, 1, 1): one cluster per job.
+// `grid` (x a multiple of cs) of `threads`-thread CTAs in clusters of (cs, 1, 1).
 template <typename Kern, typename... Args>
-cudaError_t launch_cluster(Kern kern, int cs, int njobs, int threads, int smem, cudaStream_t s, Args... args) {
+cudaError_t launch_cluster_grid(Kern kern, int cs, dim3 grid, int threads, int smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cs, njobs, 1);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -147,6 +147,11 @@ cudaError_t launch_cluster(Kern kern, int cs, int njobs, int threads, int smem, 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+// Grid (cs, njobs): one cluster per job.
+template <typename Kern, typename... Args>
+cudaError_t launch_cluster(Kern kern, int cs, int njobs, int threads, int smem, cudaStream_t s, Args... args) {
+  return launch_cluster_grid(kern, cs, dim3(cs, njobs), threads, smem, s, args...);
 }
 
 }  // namespace cl

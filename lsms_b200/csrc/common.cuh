@@ -276,6 +276,10 @@ cudaError_t launch_refine_end(const JobDev *jobs, int njobs, int ns, int kkrsz, 
 // X (+)= Y).  `fp32_arith` selects FP32 arithmetic on FP32 factors.  max_N bounds the jobs' N.
 cudaError_t launch_sweep(FactorKind fk, const JobDev *jobs, int njobs, int b, int max_N, bool forward, int mode,
                          bool fp32_arith, const CUtensorMap *fmap, cudaStream_t s, int active_hint = 0);
+// The sweeps in FP64 arithmetic (sweep64.cu), for FP64 or FP32 factors; `want` of the jobs are expected
+// to work (the others leave at once), which sizes the clusters.
+cudaError_t launch_sweep64(FactorKind fk, const JobDev *jobs, int njobs, int b, bool forward, int mode, int want,
+                           cudaStream_t s);
 // The dataflow sweeps for FP32 factors in FP32 arithmetic with b <= 16 (sweep_flow.cu), operand
 // units loaded through `fmap` (TcMaps::tFu over the jobs' factor slots).  Sets *launched when it
 // took the launch; false (and cudaSuccess) without a map or when the shape does not fit its

@@ -12,7 +12,7 @@
 // rank t % cs, so every tile has one writer.  The operand panels (A21_k or W_k rows of a tile,
 // 64 rows x 32 columns per unit) are constant during a sweep, so each CTA streams its units
 // through a two-stage cp.async ring in shared memory, fetching the next unit while it multiplies
-// the current one; the arithmetic is FP64 FMA.  One cluster barrier (release / acquire) per block
+// the current one; the arithmetic is FP32 FMA (for FP64 arithmetic see sweep64.cu).  One cluster barrier (release / acquire) per block
 // step orders the tile updates; cross-CTA reads of R and Y go through L2 (__ldcg).
 // In the forward sweep the owner of the next diagonal block updates that tile first and computes
 // Y_(k+1) = D_(k+1) R_(k+1) while the other CTAs finish step k, so the small D multiply is off the
@@ -36,10 +36,10 @@ using namespace cl;
 constexpr int kUnitCols = 32;  // operand columns per pipeline unit
 constexpr int kMaxCluster = 8;
 
+using T = float2;  // factor storage
+using V = float2;  // arithmetic: the correction solve in single precision on FP32 factors, as in LAPACK's zcgesv
+
 // Shared-memory layout of the sweep kernels.
-// T: factor storage type; V: arithmetic type of the sweep (double2, or float2 for a correction
-// solve in single precision on FP32 factors, as in LAPACK's zcgesv).
-template <typename T, typename V>
 struct SweepSmem {
   static constexpr int kUnitBytes = kUnitCols * 64 * (int)sizeof(T);
   static constexpr int kLs = 0;                                     // 2 units
@@ -127,7 +127,7 @@ struct BackwardUnits {
 };
 
 // acc[j] += sum_kk Lu[kk][r] * Ys[y0 + kk][cg + 4 j] over one unit of ncol columns.
-template <typename T, typename V, int NJ>
+template <int NJ>
 __device__ __forceinline__ void unit_product(V (&acc)[NJ], const T *__restrict__ Lu,
                                              const V (*__restrict__ Ys)[kMaxB], int y0, int ncol, int r, int cg) {
 #pragma unroll 8
@@ -139,7 +139,6 @@ __device__ __forceinline__ void unit_product(V (&acc)[NJ], const T *__restrict__
 }
 
 // Columns [b, bc) of a 64 x kMaxB staging block read as zero.
-template <typename V>
 __device__ __forceinline__ void zero_pad_columns(V (*Ys)[kMaxB], int b, int bc) {
   for (int e = threadIdx.x; e < 64 * (bc - b); e += blockDim.x) Ys[e % 64][b + e / 64] = vzero<V>();
 }
@@ -147,10 +146,10 @@ __device__ __forceinline__ void zero_pad_columns(V (*Ys)[kMaxB], int b, int bc) 
 // Grid (cs, njobs), cluster (cs, 1, 1), 256 threads.  Refinement rounds only: the initial solve
 // has B = 0 above the central block, so its forward sweep is the identity.  BC is 16 or 32,
 // the padded column count of the right-hand side (b <= BC).
-template <typename T, typename V, int BC>
+template <int BC>
 __global__ void __launch_bounds__(256) forward_sweep_kernel(const JobDev *__restrict__ jobs) {
   constexpr int NJ = BC / 4;
-  using L = SweepSmem<T, V>;
+  using L = SweepSmem;
   const JobDev &J = jobs[blockIdx.y];
   // uniform over the cluster: the flag changes only between launches
   if (converged(J.conv) || J.n == 0 || J.inactive) return;
@@ -172,7 +171,7 @@ __global__ void __launch_bounds__(256) forward_sweep_kernel(const JobDev *__rest
     V acc[NJ];
 #pragma unroll
     for (int j = 0; j < NJ; ++j) acc[j] = vzero<V>();
-    unit_product<T, V, NJ>(acc, Ds, Rs, 0, kb, r, cg);
+    unit_product<NJ>(acc, Ds, Rs, 0, kb, r, cg);
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
       const int c = cg + 4 * j;
@@ -224,7 +223,7 @@ __global__ void __launch_bounds__(256) forward_sweep_kernel(const JobDev *__rest
       do {
         cp_async_wait<1>();
         __syncthreads();  // this unit has landed for every thread; Ys is complete
-        unit_product<T, V, NJ>(acc, Ls + stage * kUnitElems, Ys, it.h * kUnitCols, it.ncol(), r, cg);
+        unit_product<NJ>(acc, Ls + stage * kUnitElems, Ys, it.h * kUnitCols, it.ncol(), r, cg);
         __syncthreads();  // every thread is done with the stage before it is refilled
         if (!pf.done()) {
           stage_block(Ls + stage * kUnitElems, F, ld, pf.t * 64, pf.k + pf.h * kUnitCols, pf.ncol());
@@ -260,10 +259,10 @@ __global__ void __launch_bounds__(256) forward_sweep_kernel(const JobDev *__rest
 
 // Grid (cs, njobs), cluster (cs, 1, 1), 256 threads.  mode 0 sets X = Y, mode 1 adds X += Y
 // (and skips converged jobs).
-template <typename T, typename V, int BC>
+template <int BC>
 __global__ void __launch_bounds__(256) backward_sweep_kernel(const JobDev *__restrict__ jobs, int mode) {
   constexpr int NJ = BC / 4;
-  using L = SweepSmem<T, V>;
+  using L = SweepSmem;
   const JobDev &J = jobs[blockIdx.y];
   if ((mode == 1 && converged(J.conv)) || J.inactive) return;
   const int rank = cluster_rank(), cs = cluster_size();
@@ -311,7 +310,7 @@ __global__ void __launch_bounds__(256) backward_sweep_kernel(const JobDev *__res
       do {
         cp_async_wait<1>();
         __syncthreads();
-        unit_product<T, V, NJ>(acc, Ls + stage * kUnitElems, Ys, it.h * kUnitCols, it.ncol(), r, cg);
+        unit_product<NJ>(acc, Ls + stage * kUnitElems, Ys, it.h * kUnitCols, it.ncol(), r, cg);
         __syncthreads();
         if (!pf.done()) {
           stage_block(Ls + stage * kUnitElems, F, ld, pf.t * 64, pf.k + pf.h * kUnitCols, pf.ncol());
@@ -321,7 +320,8 @@ __global__ void __launch_bounds__(256) backward_sweep_kernel(const JobDev *__res
         stage ^= 1;
         it.next();
       } while (!it.done() && it.k == k && it.t == t && it.h != 0);
-      // Y[tile] -= W[tile, k:k+kb] Y_k for the rows above the block
+      // Y[tile] -= W[tile, k:k+kb] Y_k for the rows above the block (the initial solve, mode 0, has
+      // Y = 0 there before the central block, which is every tile's first)
       const int gr = t * 64 + r;
       if (gr < k) {
 #pragma unroll
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(256) backward_sweep_kernel(const JobDev *__res
           const int c = cg + 4 * j;
           if (c >= b) continue;
           double2 *dst = J.Y + (size_t)gr + (size_t)c * ld;
-          *dst = to_d(csub(to_v<V>(__ldcg(dst)), acc[j]));
+          *dst = to_d(csub(mode == 0 && k == n ? vzero<V>() : to_v<V>(__ldcg(dst)), acc[j]));
         }
       }
     }
@@ -387,46 +387,35 @@ int cluster_for(K *kern, int smem, int njobs) {
   return 1;
 }
 
-template <typename T, typename V, int BC>
+template <int BC>
 cudaError_t sweep_impl(const JobDev *jobs, int njobs, bool forward, int mode, cudaStream_t s, int want) {
   cudaError_t e;
   if (forward) {
-    const int smem = SweepSmem<T, V>::kForward;
-    if ((e = ensure_smem(forward_sweep_kernel<T, V, BC>, smem)) != cudaSuccess)
+    const int smem = SweepSmem::kForward;
+    if ((e = ensure_smem(forward_sweep_kernel<BC>, smem)) != cudaSuccess)
       return e;
-    const int cs = cluster_for(forward_sweep_kernel<T, V, BC>, smem, want);
-    return launch_cluster(forward_sweep_kernel<T, V, BC>, cs, njobs, 256, smem, s, jobs);
+    const int cs = cluster_for(forward_sweep_kernel<BC>, smem, want);
+    return launch_cluster(forward_sweep_kernel<BC>, cs, njobs, 256, smem, s, jobs);
   }
-  const int smem = SweepSmem<T, V>::kBackward;
-  if ((e = ensure_smem(backward_sweep_kernel<T, V, BC>, smem)) != cudaSuccess)
+  const int smem = SweepSmem::kBackward;
+  if ((e = ensure_smem(backward_sweep_kernel<BC>, smem)) != cudaSuccess)
     return e;
-  const int cs = cluster_for(backward_sweep_kernel<T, V, BC>, smem, want);
-  return launch_cluster(backward_sweep_kernel<T, V, BC>, cs, njobs, 256, smem, s, jobs, mode);
-}
-
-template <typename T, typename V>
-cudaError_t sweep_b(const JobDev *jobs, int njobs, int b, bool forward, int mode, cudaStream_t s,
-                    int active_hint = 0) {
-  const int want = active_hint > 0 && active_hint < njobs ? active_hint : njobs;
-  return b <= 16 ? sweep_impl<T, V, 16>(jobs, njobs, forward, mode, s, want)
-                 : sweep_impl<T, V, 32>(jobs, njobs, forward, mode, s, want);
+  const int cs = cluster_for(backward_sweep_kernel<BC>, smem, want);
+  return launch_cluster(backward_sweep_kernel<BC>, cs, njobs, 256, smem, s, jobs, mode);
 }
 
 }  // namespace
-
 
 cudaError_t launch_sweep(FactorKind fk, const JobDev *jobs, int njobs, int b, int max_N, bool forward, int mode,
                          bool fp32_arith, const CUtensorMap *fmap, cudaStream_t s, int active_hint) {
   if (njobs <= 0) return cudaSuccess;
   if (b < 1 || b > kMaxB || (forward && mode != 1)) return cudaErrorInvalidValue;
-  if (fk == kFactorFP64) return sweep_b<double2, double2>(jobs, njobs, b, forward, mode, s, active_hint);
-  if (fp32_arith) {
-    bool done = false;
-    const cudaError_t e = launch_flow_sweep(jobs, njobs, b, max_N, forward, mode, fmap, s, &done, active_hint);
-    if (e != cudaSuccess || done) return e;
-    return sweep_b<float2, float2>(jobs, njobs, b, forward, mode, s, active_hint);
-  }
-  return sweep_b<float2, double2>(jobs, njobs, b, forward, mode, s, active_hint);
+  const int want = active_hint > 0 && active_hint < njobs ? active_hint : njobs;
+  if (fk == kFactorFP64 || !fp32_arith) return launch_sweep64(fk, jobs, njobs, b, forward, mode, want, s);
+  bool done = false;
+  const cudaError_t e = launch_flow_sweep(jobs, njobs, b, max_N, forward, mode, fmap, s, &done, active_hint);
+  if (e != cudaSuccess || done) return e;
+  return b <= 16 ? sweep_impl<16>(jobs, njobs, forward, mode, s, want) : sweep_impl<32>(jobs, njobs, forward, mode, s, want);
 }
 
 }  // namespace b200

@@ -711,14 +711,14 @@ __global__ void __launch_bounds__(kBlock, 1)
 
   flow_setup(S, ns, cs);
   if (tid < kThreads) {
-    // own tiles of Y (rows < n) in FP32
+    // own tiles of Y (rows < n) in FP32; 0 in the initial solve (mode 0)
     for (int i = 0; q + i * cs < Tn; ++i) {
       const int t = q + i * cs;
       float2 v[kPerThread];  // a tile's loads in flight together, then its stores
 #pragma unroll
       for (int j = 0; j < kPerThread; ++j) {
         const int e = tid + j * kThreads, c = e >> 6, gr = 64 * t + (e & 63);
-        v[j] = (c < b && gr < n) ? to_v<float2>(__ldcg(Yb + (size_t)gr + (size_t)c * ld)) : make_float2(0.f, 0.f);
+        v[j] = (mode == 1 && c < b && gr < n) ? to_v<float2>(__ldcg(Yb + (size_t)gr + (size_t)c * ld)) : make_float2(0.f, 0.f);
       }
 #pragma unroll
       for (int j = 0; j < kPerThread; ++j) S.tiles[i * kTileElems + tid + j * kThreads] = v[j];

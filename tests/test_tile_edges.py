@@ -113,3 +113,28 @@ def test_full_tau_and_adjoint_odd_sizes(solver_factory, lattice, shells, n_reduc
         wb = lam[r] @ z[r].T + (lam[r] if j == 0 else 0.0)
         assert np.abs(tbar[0][j][:k, :k] - wb).max() <= 1e-10 * scale
         assert np.abs(dlog[0][j][:k, :k] + h[r, r].T).max() <= 1e-10 * max(1.0, np.abs(h).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sweep", [T.SWEEP_FP32, T.SWEEP_FP64])
+@pytest.mark.parametrize("cant", [1, 2])
+@pytest.mark.parametrize("njobs", [1, 2, 7, 33])
+def test_batch_sizes(solver_factory, njobs, cant, sweep):
+    """Cluster sizes of the sweeps and the residual's split of K follow the number of jobs: each job of a
+    batch against the oracle, FP64 and mixed."""
+    from oracle import port
+    prob = W.make_problem("bcc", 5.42, 2, 3, W.semicircle_contour(-0.2, 0.7, njobs), 5, n_species=None,
+                          n_spin_cant=cant, n_spin_pola=cant)
+    s = solver_factory(3, cant, cant)
+    s.load_problem(prob)
+    jobs = T.make_jobs([(0, i, 0, e) for i, e in enumerate(prob.energies)])
+    s.set_mixed_sweep(sweep)
+    try:
+        out = {prec: s.solve_jobs(jobs, prec) for prec in (T.PREC_FP64, T.PREC_MIXED)}
+    finally:
+        s.set_mixed_sweep(T.SWEEP_FP32)
+    for i in range(0, njobs, max(1, njobs // 4)):
+        # two backward-stable FP64 solves differ by a few times cond(M) 2^-53 (cond up to 1e4 here)
+        bound = max(1e-12, 8 * np.linalg.cond(port.build_kkr(prob, i)) * 2.0 ** -53)
+        assert _tau_err(prob, i, out[T.PREC_FP64][i]) <= bound
+        assert _tau_err(prob, i, out[T.PREC_MIXED][i]) <= TOL_MIXED
