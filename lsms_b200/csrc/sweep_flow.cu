@@ -546,21 +546,21 @@ struct Deferred {
   }
 };
 
-// Grid (cs, njobs), cluster (cs, 1, 1), 320 threads: 8 compute warps, the producer warp and the
-// MMA warp.
+// Grid (cs, njobs, slices of kCols columns), cluster (cs, 1, 1), 320 threads: 8 compute warps, the
+// producer warp and the MMA warp.
 // Refinement rounds only (the initial solve has B = 0 above the central block).  own_max:
 // resident tiles per CTA (ceil(tiles / cs)).
 __global__ void __launch_bounds__(kBlock, 1)
-    forward_flow_kernel(const JobDev *__restrict__ jobs, int own_max, const __grid_constant__ CUtensorMap fmap,
-                        int col0) {
+    forward_flow_kernel(const JobDev *__restrict__ jobs, int own_max, const __grid_constant__ CUtensorMap fmap) {
   const JobDev &J = jobs[blockIdx.y];
+  const int col0 = kCols * blockIdx.z;
   // uniform over the cluster: the flag changes only between launches
-  if (converged(J.conv) || J.n == 0 || J.inactive) return;
+  if (converged(J.conv) || J.n == 0 || J.inactive || col0 >= J.b) return;
   const int q = cluster_rank(), cs = cluster_size(), csm = cs - 1, lcs = __ffs(cs) - 1;
   const FlowLayout L = flow_layout(cs, own_max, true);
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   const FlowSmem S(aligned_smem(sm_raw), L);
-  // this launch's right-hand-side columns: [col0, col0 + b) of R and Y
+  // this cluster's right-hand-side columns: [col0, col0 + b) of R and Y
   const int n = J.n, N = J.N, ld = J.ld, b = min(kCols, J.b - col0), ns = L.ns, nsm = ns - 1, lns = __ffs(ns) - 1;
   double2 *const Rb = J.R + (size_t)col0 * ld;
   double2 *const Yb = J.Y + (size_t)col0 * ld;
@@ -686,18 +686,19 @@ __global__ void __launch_bounds__(kBlock, 1)
   flow_teardown(S, tmem);
 }
 
-// Grid (cs, njobs), cluster (cs, 1, 1), 320 threads.  mode 0 sets X = Y, mode 1 adds X += Y
+// Grid and cluster as above, 320 threads.  mode 0 sets X = Y, mode 1 adds X += Y
 // (and skips converged jobs).
 __global__ void __launch_bounds__(kBlock, 1)
     backward_flow_kernel(const JobDev *__restrict__ jobs, int own_max, int mode,
-                         const __grid_constant__ CUtensorMap fmap, int col0) {
+                         const __grid_constant__ CUtensorMap fmap) {
   const JobDev &J = jobs[blockIdx.y];
-  if ((mode == 1 && converged(J.conv)) || J.inactive) return;
+  const int col0 = kCols * blockIdx.z;
+  if ((mode == 1 && converged(J.conv)) || J.inactive || col0 >= J.b) return;
   const int q = cluster_rank(), cs = cluster_size(), csm = cs - 1, lcs = __ffs(cs) - 1;
   const FlowLayout L = flow_layout(cs, own_max, false);
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   const FlowSmem S(aligned_smem(sm_raw), L);
-  // bc: rows of the central block; b: this launch's right-hand-side columns [col0, col0 + b) of Y, X
+  // bc: rows of the central block; b: this cluster's right-hand-side columns [col0, col0 + b) of Y, X
   const int n = J.n, ld = J.ld, bc = J.b, b = min(kCols, J.b - col0), ns = L.ns, nsm = ns - 1,
             lns = __ffs(ns) - 1;
   const double2 *const Yb = J.Y + (size_t)col0 * ld;
@@ -886,7 +887,10 @@ cudaError_t launch_flow_sweep(const JobDev *jobs, int njobs, int b, int max_N, b
   const int T = (max_N + 63) / 64;
   const void *kern = forward ? reinterpret_cast<const void *>(forward_flow_kernel)
                              : reinterpret_cast<const void *>(backward_flow_kernel);
-  const int want = active_hint > 0 && active_hint < njobs ? active_hint : njobs;
+  // the sweeps are column-separable: more than kCols right-hand-side columns are slices with clusters
+  // of their own (the factor units stream once per slice)
+  const int slices = (b + kCols - 1) / kCols;
+  const int want = slices * (active_hint > 0 && active_hint < njobs ? active_hint : njobs);
   int cs = 0, fallback = 0;
   for (int c = 8; c >= 1; c >>= 1) {
     const FlowLayout L = flow_layout(c, (T + c - 1) / c, forward);
@@ -904,14 +908,9 @@ cudaError_t launch_flow_sweep(const JobDev *jobs, int njobs, int b, int max_N, b
   const FlowLayout L = flow_layout(cs, (T + cs - 1) / cs, forward);
   cudaError_t e = ensure_smem(kern, L.total);
   if (e != cudaSuccess) return e;
-  // the sweeps are column-separable: more than kCols right-hand-side columns take one launch per
-  // kCols of them (the factor units stream once per launch)
-  for (int col0 = 0; col0 < b && e == cudaSuccess; col0 += kCols) {
-    if (forward)
-      e = launch_cluster(forward_flow_kernel, cs, njobs, kBlock, L.total, s, jobs, L.own, *fmap, col0);
-    else
-      e = launch_cluster(backward_flow_kernel, cs, njobs, kBlock, L.total, s, jobs, L.own, mode, *fmap, col0);
-  }
+  const dim3 grid(cs, njobs, slices);
+  e = forward ? launch_cluster_grid(forward_flow_kernel, cs, grid, kBlock, L.total, s, jobs, L.own, *fmap)
+              : launch_cluster_grid(backward_flow_kernel, cs, grid, kBlock, L.total, s, jobs, L.own, mode, *fmap);
   if (e == cudaSuccess) *launched = true;
   return e;
 }
