@@ -119,6 +119,10 @@ struct JobDev {
                          // 64 x 64 diagonal blocks only
 };
 
+// Structure of a stored t block (launch_tdiag_flags): exactly diagonal, or every spin block exactly
+// diagonal (0: neither).
+constexpr unsigned char kTdiagFull = 1, kTdiagSpin = 2;
+
 struct BuildParams {
   const AngularTables *tables;  // device
   const double2 *tmat;          // device tmatStore, column-major (tmat_ld x nstore)
@@ -128,7 +132,7 @@ struct BuildParams {
   int ns;                       // n_spin_cant
   int npola;                    // n_spin_pola
   int f_kind;                   // 0: no F copy (F aliases M), 1: FP64 copy, 2: FP32 copy
-  const unsigned char *tdiag;   // [(store * group + iie) * 2 + ispin]: t block exactly diagonal
+  const unsigned char *tdiag;   // [(store * group + iie) * 2 + ispin]: kTdiag* of the t block
   int group;                    // energies in the uploaded tmatStore group
   int g_mode;                   // 1: write the structure constants G (no t factor, zero diagonal
                                 // blocks) into M instead of M = 1 - t G (adjoint)
@@ -217,9 +221,9 @@ inline cudaError_t ensure_smem(K *kernel, int bytes) {
 // kernels enqueued.
 cudaError_t launch_kkr_build(const JobDev *jobs, int njobs, int max_L, const BuildParams &p,
                              int *err_flags, cudaStream_t s, long *launches);
-// flags[(store * group + iie) * 2 + ispin] = 1 when that b x b t block of the device tmatStore
-// (column-major, leading dimension ld per store column) has no non-zero off-diagonal element;
-// spin 1 is written as 0 unless the store is collinear spin-polarised (`colpol`).
+// flags[(store * group + iie) * 2 + ispin] = the structure (kTdiag*) of that b x b t block of the device
+// tmatStore (column-major, leading dimension ld per store column); spin 1 is written as 0 unless the
+// store is collinear spin-polarised (`colpol`).
 cudaError_t launch_tdiag_flags(const double2 *tmat, long ld, int nstore, int group, int b, int kkrsz, bool colpol,
                                unsigned char *flags, cudaStream_t s);
 // Block elimination of F over the first n columns (all jobs of the wave).

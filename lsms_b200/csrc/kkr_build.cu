@@ -300,25 +300,30 @@ __global__ void __launch_bounds__(kThreads)
     // M block = -t_i * diag_s(G): rows (s_r, r'), columns (s_c, c') (setgij.f:29-38)
     const double2 *__restrict__ tb =
         p.tmat + (long)J.store[i] * p.tmat_ld + (long)J.iie * p.blk + jsm;
-    const bool tdiag = p.tdiag != nullptr && p.tdiag[((long)J.store[i] * p.group + J.iie) * 2 + J.ispin] != 0;
-    // With a diagonal t (spherical scatterer) or for G itself each G element gives its M
-    // elements directly; otherwise G is staged for the t G product.
-    const bool direct = tdiag || p.g_mode;
+    // With a t that is diagonal in L (a spherical scatterer: each spin block of a non-collinear t is
+    // diagonal) or for G itself each G element gives its M elements directly (16 non-collinear jobs of
+    // N = 4320: 1.36 ms, 5.75 ms through the product); otherwise G is staged for the t G product.
+    const int tdiag = p.tdiag != nullptr ? p.tdiag[((long)J.store[i] * p.group + J.iie) * 2 + J.ispin] : 0;
+    const bool direct = tdiag != 0 || p.g_mode;
+    const bool spin_mix = tdiag == kTdiagSpin && !p.g_mode;  // (else the off-diagonal spin blocks are zero)
     // G(lm2, lm1) = pi4 i^(l2-l1) sum_l3 cgnt(l3/2, lm1, lm2) D(l3, m2-m1) (:148-176); lanes run
     // along lm2 (rows) so that the direct stores are column segments.  When kki divides 32 a
     // lane's row lm2 is the same for all its elements, so the diagonal t values are loaded once.
     const bool lane_row = (32 % kki) == 0;
-    double2 tdg0 = make_double2(0.0, 0.0), tdg1 = tdg0;  // spin 0, 1
-    if (direct && !p.g_mode && lane_row) {
-      const int t0 = lane % kki, t1 = kkrsz + lane % kki;
-      tdg0 = __ldg(tb + t0 + (long)t0 * bstore);
-      if (ns > 1) tdg1 = __ldg(tb + t1 + (long)t1 * bstore);
-    }
+    double2 tdg[2][2] = {};  // -t of the lane's row, [row spin][column spin]; 1 on the diagonal for G itself
+    if (direct && lane_row)
+#pragma unroll
+      for (int sr = 0; sr < 2; ++sr)
+#pragma unroll
+        for (int sc = 0; sc < 2; ++sc) {
+          if (sr >= ns || sc >= ns || (sr != sc && !spin_mix) || p.g_mode) continue;
+          const double2 tv = __ldg(tb + sr * kkrsz + lane % kki + (long)(sc * kkrsz + lane % kki) * bstore);
+          tdg[sr][sc] = make_double2(-tv.x, -tv.y);
+        }
     const double2 *Dw = sm.D[warp];
-    if (direct && ns == 1 && kki == 16 && kkj == 16 && T.lmax == 3) {
+    if (direct && kki == 16 && kkj == 16 && T.lmax == 3) {
       // -t_rr G for lmax-3 blocks from the per-lane gather records: the same sums, products and
       // roundings as the general loop below (the folded signs are exact)
-      const double2 tneg = make_double2(-tdg0.x, -tdg0.y);
       const int lm2 = lane & 15;
 #pragma unroll 2
       for (int it = 0; it < 8; ++it) {
@@ -338,8 +343,16 @@ __global__ void __launch_bounds__(kThreads)
         acc.x *= T.pi4;
         acc.y *= T.pi4;
         const double2 g = (d >> 24) ? make_double2(-acc.y, acc.x) : acc;
-        const double2 v = p.g_mode ? g : cfma(tneg, g, make_double2(0.0, 0.0));
-        put((size_t)(row0 + lm2) + (size_t)(col0 + lm1) * ld, v);
+#pragma unroll
+        for (int sr = 0; sr < 2; ++sr)
+#pragma unroll
+          for (int sc = 0; sc < 2; ++sc) {
+            if (sr >= ns || sc >= ns) continue;
+            double2 v = make_double2(0.0, 0.0);
+            if (sr == sc && p.g_mode) v = g;
+            else if (sr == sc || spin_mix) v = cfma(tdg[sr][sc], g, make_double2(0.0, 0.0));
+            put((size_t)(row0 + sr * 16 + lm2) + (size_t)(col0 + sc * 16 + lm1) * ld, v);
+          }
       }
       continue;
     }
@@ -368,21 +381,24 @@ __global__ void __launch_bounds__(kThreads)
         sm.G[warp][lm2 * kMaxKK + lm1] = g;
         continue;
       }
-      for (int sr = 0; sr < ns; ++sr) {
-        double2 v = g;
-        if (!p.g_mode) {  // -t_rr G, rounded as the general path's one nonzero term
-          double2 tv = sr == 0 ? tdg0 : tdg1;
-          if (!lane_row) {
-            const int trow = sr * kkrsz + lm2;
-            tv = __ldg(tb + trow + (long)trow * bstore);
+#pragma unroll
+      for (int sr = 0; sr < 2; ++sr)
+#pragma unroll
+        for (int sc = 0; sc < 2; ++sc) {
+          if (sr >= ns || sc >= ns) continue;
+          double2 v = make_double2(0.0, 0.0);
+          if (p.g_mode) {
+            if (sr == sc) v = g;
+          } else if (sr == sc || spin_mix) {  // -t_rr G, rounded as the general path's one nonzero term
+            double2 tv = tdg[sr][sc];
+            if (!lane_row) {
+              tv = __ldg(tb + sr * kkrsz + lm2 + (long)(sc * kkrsz + lm2) * bstore);
+              tv = make_double2(-tv.x, -tv.y);
+            }
+            v = cfma(tv, g, v);
           }
-          const double2 pr2 = cfma(tv, g, make_double2(0.0, 0.0));
-          v = make_double2(-pr2.x, -pr2.y);
+          put((size_t)(row0 + sr * kki + lm2) + (size_t)(col0 + sc * kkj + lm1) * ld, v);
         }
-        for (int sc = 0; sc < ns; ++sc)
-          put((size_t)(row0 + sr * kki + lm2) + (size_t)(col0 + sc * kkj + lm1) * ld,
-              sc == sr ? v : make_double2(0.0, 0.0));
-      }
     }
     __syncwarp();
     if (direct) continue;
@@ -411,7 +427,8 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// One warp per (store, energy, spin) t block: is every off-diagonal element exactly zero?
+// One warp per (store, energy, spin) t block: kTdiagFull when every off-diagonal element is exactly
+// zero, kTdiagSpin when every element off the diagonals of the spin blocks is, else 0.
 __global__ void tdiag_flags_kernel(const double2 *__restrict__ tmat, long ld, int nstore, int group, int b,
                                    int kkrsz, int colpol, unsigned char *__restrict__ flags) {
   const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -424,14 +441,17 @@ __global__ void tdiag_flags_kernel(const double2 *__restrict__ tmat, long ld, in
   }
   const long blk = (long)(2 * kkrsz) * (2 * kkrsz);
   const double2 *t = tmat + (long)st * ld + (long)ie * blk + (colpol ? (long)kkrsz * kkrsz * sp : 0);
-  bool off = false;
+  bool off = false, off_l = false;
   for (int e = lane; e < b * b; e += 32) {
     const int c = e / b, r = e - c * b;
     const double2 v = t[e];
-    off |= r != c && (v.x != 0.0 || v.y != 0.0);
+    const bool nz = v.x != 0.0 || v.y != 0.0;
+    off |= r != c && nz;
+    off_l |= r % kkrsz != c % kkrsz && nz;
   }
   off = __any_sync(0xffffffffu, off);
-  if (lane == 0) flags[f] = off ? 0 : 1;
+  off_l = __any_sync(0xffffffffu, off_l);
+  if (lane == 0) flags[f] = !off ? kTdiagFull : !off_l ? kTdiagSpin : 0;
 }
 
 }  // namespace

@@ -138,3 +138,24 @@ def test_batch_sizes(solver_factory, njobs, cant, sweep):
         bound = max(1e-12, 8 * np.linalg.cond(port.build_kkr(prob, i)) * 2.0 ** -53)
         assert _tau_err(prob, i, out[T.PREC_FP64][i]) <= bound
         assert _tau_err(prob, i, out[T.PREC_MIXED][i]) <= TOL_MIXED
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("outer", [3, 2, 1])
+@pytest.mark.parametrize("coupled", [False, True])
+def test_build_non_collinear_t(solver_factory, outer, coupled):
+    """M of a non-collinear t whose spin blocks are diagonal (one product per element), and of one with
+    elements off those diagonals, equal lmax and lmax steps."""
+    from oracle import port
+    L = W.lattice_shells("bcc", 5.42, 1).shape[1]
+    lmax = np.full(L, 3, np.int32)
+    lmax[L // 2:] = outer
+    prob = W.make_problem("bcc", 5.42, 1, 3, [0.4 + 0.2j], 3, n_species=None, n_spin_cant=2, n_spin_pola=2, liz_lmax=lmax)
+    if coupled:
+        rng = np.random.default_rng(1)
+        prob.tmat_store[2:5, 0, :1024] += 0.01 * (rng.normal(size=(3, 1024)) + 1j * rng.normal(size=(3, 1024)))
+    s = solver_factory(3, 2, 2)
+    s.load_problem(prob)
+    got = s.build_kkr(0, 0, 0, prob.energies[0], prob.nrmat_ns)
+    want = port.build_kkr(prob, 0)
+    assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
