@@ -103,16 +103,16 @@ __global__ void __launch_bounds__(kSelThreads) panel_select_kernel(const JobDev 
   const int n = J.n, ld = J.ld;
   int *__restrict__ piv = J.piv;
   const unsigned *__restrict__ mags = reinterpret_cast<const unsigned *>(piv + pivot_mags_offset(ld));
-  extern __shared__ __align__(16) unsigned char sel_smem[];
-  float2(*A)[kPivCands] = reinterpret_cast<float2(*)[kPivCands]>(sel_smem);  // A[col][cand]
+  __shared__ float2 s_col[2][kPivCands];  // the step's column, by step parity
+  __shared__ float2 s_row[kNb];           // the pivot row's columns, in the threads' places
+  __shared__ unsigned long long s_best[2][kPivCands / 32];
+  __shared__ int s_dst[2 * kNb], s_src[2 * kNb], s_cnt;
   __shared__ int s_cand[kPivCands];
   __shared__ int s_out[kNb];
   __shared__ int s_hist[256];
   __shared__ int s_warp[32];
   __shared__ unsigned s_prefix;
   __shared__ int s_remain;
-  __shared__ float s_wv[2][kPivCands / 32];
-  __shared__ int s_wi[2][kPivCands / 32];
   const int tid = threadIdx.x;
 
   // --- candidates: the diagonal block's rows, then the largest rows below it ---
@@ -179,105 +179,104 @@ __global__ void __launch_bounds__(kSelThreads) panel_select_kernel(const JobDev 
     __syncthreads();
   } else {
     const T *__restrict__ F = static_cast<const T *>(J.F);
+    // Thread (candidate r, column group g) holds its 16 columns in registers.  A step writes the columns
+    // of the group that holds the step's column one place down, so that group's column to rank is
+    // always in place 0; the others stay put.  (A launch takes 128 us; 173 us with the rows in shared
+    // memory and one thread finding the row moves.)
     const int r = tid & (kPivCands - 1), g = tid / kPivCands, c0 = g * kGroupCols;
     const int cand = r < R ? s_cand[r] : -1;
-    for (int j = c0; j < c0 + kGroupCols; ++j)
-      A[j][r] = (cand >= 0 && j < kb) ? to_f2(F[(size_t)cand + (size_t)(k + j) * ld]) : make_float2(0.f, 0.f);
-    __syncthreads();
+    float2 a[kGroupCols];
+#pragma unroll
+    for (int j = 0; j < kGroupCols; ++j)
+      a[j] = (cand >= 0 && c0 + j < kb) ? to_f2(F[(size_t)cand + (size_t)(k + c0 + j) * ld]) : make_float2(0.f, 0.f);
     bool taken = false;
     for (int p = 0; p < kb; ++p) {
-      const int par = p & 1, gp = p / kGroupCols;
-      if (g == gp) {  // the threads holding column p rank their rows: warp arg-max, ties low
-        float v = -1.f;
-        if (cand >= 0 && !taken) {
-          v = cabs1f(A[p][r]);
-          if (!(v == v)) v = 0.f;  // a NaN ranks as zero, so a row in range is still chosen
-        }
-        int idx = r;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-          if (ov > v || (ov == v && oi < idx)) {
-            v = ov;
-            idx = oi;
-          }
-        }
-        if ((tid & 31) == 0) {
-          s_wv[par][r >> 5] = v;
-          s_wi[par][r >> 5] = idx;
-        }
+      const int par = p & 1;
+      const bool mine = g == p / kGroupCols;  // (uniform over a warp)
+      if (mine) {  // rank the rows: the largest |re| + |im| (its bits order as integers), ties low
+        float v = cabs1f(a[0]);
+        if (!(v == v)) v = 0.f;  // a NaN ranks as zero, so a row in range is still chosen
+        const bool on = cand >= 0 && !taken;
+        const unsigned hi = on ? __float_as_uint(v) + 1u : 0u;
+        const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned lo = __reduce_max_sync(0xffffffffu, hi == mhi ? (unsigned)(kPivCands - 1 - r) : 0u);
+        if ((tid & 31) == 0) s_best[par][r >> 5] = ((unsigned long long)mhi << 32) | lo;
+        s_col[par][r] = a[0];
       }
       __syncthreads();
-      float bv = s_wv[par][0];
-      int bi = s_wi[par][0];
+      unsigned long long best = s_best[par][0];
 #pragma unroll
-      for (int w = 1; w < kPivCands / 32; ++w) {
-        const float ov = s_wv[par][w];
-        const int oi = s_wi[par][w];
-        if (ov > bv || (ov == bv && oi < bi)) {
-          bv = ov;
-          bi = oi;
-        }
+      for (int w = 1; w < kPivCands / 32; ++w) best = s_best[par][w] > best ? s_best[par][w] : best;
+      // R > kb > p candidates remain untaken, each ranked above the taken ones: bi is one of them
+      const int bi = kPivCands - 1 - (int)(unsigned)best;
+      if (r == bi) {
+        taken = true;
+#pragma unroll
+        for (int j = 0; j < kGroupCols; ++j) s_row[c0 + j] = a[j];
       }
-      // R > kb > p candidates remain untaken, each ranked >= 0: bi is one of them
-      if (r == bi) taken = true;
       if (tid == 0) s_out[p] = s_cand[bi];
-      const int jlo = max(p + 1, c0), jhi = min(kb, c0 + kGroupCols);
-      if (cand >= 0 && !taken && jlo < jhi) {
-        const float2 d = A[p][bi];
-        const float dd = d.x * d.x + d.y * d.y;
-        float2 f = make_float2(0.f, 0.f);
-        if (dd > 0.f) {
-          const float2 a = A[p][r];
-          f = make_float2((a.x * d.x + a.y * d.y) / dd, (a.y * d.x - a.x * d.y) / dd);
-        }
-        for (int j = jlo; j < jhi; ++j) {
-          const float2 pj = A[j][bi];
-          float2 x = A[j][r];
-          x.x -= f.x * pj.x - f.y * pj.y;
-          x.y -= f.x * pj.y + f.y * pj.x;
-          A[j][r] = x;
-        }
-      }
+      const float2 d = s_col[par][bi], x0 = s_col[par][r];
+      const float dd = d.x * d.x + d.y * d.y;
+      float2 f = make_float2(0.f, 0.f);
+      if (dd > 0.f && !taken) f = make_float2((x0.x * d.x + x0.y * d.y) / dd, (x0.y * d.x - x0.x * d.y) / dd);
       __syncthreads();
+      auto sub = [&](float2 x, float2 pj) {
+        x.x -= f.x * pj.x - f.y * pj.y;
+        x.y -= f.x * pj.y + f.y * pj.x;
+        return x;
+      };
+      if (mine) {
+#pragma unroll
+        for (int j = 1; j < kGroupCols; ++j) a[j - 1] = sub(a[j], s_row[c0 + j]);
+        a[kGroupCols - 1] = make_float2(0.f, 0.f);  // (the step's own column is not needed again)
+      } else if (p < c0) {
+#pragma unroll
+        for (int j = 0; j < kGroupCols; ++j) a[j] = sub(a[j], s_row[c0 + j]);
+      }
     }
+    __syncthreads();
   }
-  if (tid != 0) return;
   // the moves that bring the pivot rows to k..k+kb-1 (pivot order) and the displaced rows to the
   // vacated positions; a permutation of at most 2 kb positions, also applied to perm
+  if (tid == 0) {
+    // kb distinct rows in [k, n) by construction; anything else leaves the rows in place
+    bool ok = true;
+    unsigned long long in_s = 0ull;
+    for (int p = 0; p < kb; ++p) {
+      ok = ok && s_out[p] >= k && s_out[p] < n;
+      if (s_out[p] - k < kb) in_s |= 1ull << (s_out[p] - k);
+    }
+    int cnt = 0;
+    for (int i = 0; i < kb; ++i)
+      if (s_out[i] != k + i) {
+        s_dst[cnt] = k + i;
+        s_src[cnt] = s_out[i];
+        ++cnt;
+      }
+    int vj = 0;
+    for (int i = 0; i < kb; ++i)
+      if (!((in_s >> i) & 1ull)) {
+        while (vj < kb && s_out[vj] < k + kb) ++vj;  // the next vacated position, in pivot order
+        if (vj == kb) break;  // (as many vacated positions as displaced rows: not reached)
+        s_dst[cnt] = s_out[vj];
+        s_src[cnt] = k + i;
+        ++cnt;
+        ++vj;
+      }
+    s_cnt = ok ? cnt : 0;
+  }
+  __syncthreads();
+  const int cnt = s_cnt;
   int *mv = piv + pivot_moves_offset(ld);
-  int *dst = mv + 1, *src = mv + 1 + 2 * kNb;
-  // kb distinct rows in [k, n) by construction; anything else leaves the rows in place
-  for (int p = 0; p < kb; ++p)
-    if (s_out[p] < k || s_out[p] >= n) {
-      mv[0] = 0;
-      return;
-    }
-  int cnt = 0;
-  unsigned long long in_s = 0ull;
-  for (int p = 0; p < kb; ++p)
-    if (s_out[p] - k < kb) in_s |= 1ull << (s_out[p] - k);
-  for (int i = 0; i < kb; ++i)
-    if (s_out[i] != k + i) {
-      dst[cnt] = k + i;
-      src[cnt] = s_out[i];
-      ++cnt;
-    }
-  int vj = 0;
-  for (int i = 0; i < kb; ++i)
-    if (!((in_s >> i) & 1ull)) {
-      while (vj < kb && s_out[vj] < k + kb) ++vj;  // the next vacated position, in pivot order
-      if (vj == kb) break;  // (as many vacated positions as displaced rows: not reached)
-      dst[cnt] = s_out[vj];
-      src[cnt] = k + i;
-      ++cnt;
-      ++vj;
-    }
-  mv[0] = cnt;
-  int old[2 * kNb];
-  for (int c = 0; c < cnt; ++c) old[c] = piv[src[c]];
-  for (int c = 0; c < cnt; ++c) piv[dst[c]] = old[c];
+  if (tid == 0) mv[0] = cnt;
+  int old = 0;
+  if (tid < cnt) {
+    mv[1 + tid] = s_dst[tid];
+    mv[1 + 2 * kNb + tid] = s_src[tid];
+    old = piv[s_src[tid]];
+  }
+  __syncthreads();
+  if (tid < cnt) piv[s_dst[tid]] = old;
 }
 
 // The step's row moves applied to columns [c0, c1) of F: one warp per column reads every moved
@@ -332,14 +331,11 @@ template <typename T>
 cudaError_t select_impl(const JobDev *jobs, int njobs, int k, int max_n, cudaStream_t s, long *launches) {
   if (max_n - k <= 0) return cudaSuccess;
   const int m = max_n - k - kNb;  // rows below the diagonal block, at most
-  const int smem = kNb * kPivCands * (int)sizeof(float2);
-  cudaError_t e = ensure_smem(panel_select_kernel<T>, smem);
-  if (e != cudaSuccess) return e;
   if (m > kPivCands - kNb) {  // magnitudes are ranked only when the candidates must be filtered
     panel_mags_kernel<T><<<dim3((m + 255) / 256, njobs), 256, 0, s>>>(jobs, k);
     if (launches) *launches += 1;
   }
-  panel_select_kernel<T><<<njobs, kSelThreads, smem, s>>>(jobs, k);
+  panel_select_kernel<T><<<njobs, kSelThreads, 0, s>>>(jobs, k);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }
