@@ -21,6 +21,7 @@
 #include "cplx.cuh"
 #include "dmma.cuh"
 #include "gj.cuh"
+#include "split8.cuh"
 
 namespace b200 {
 namespace {
@@ -30,13 +31,7 @@ using namespace cx;
 using dm::kOverwrite;
 using dm::kSubtract;
 
-struct GemmView {
-  const double2 *A;
-  const double2 *B;
-  double2 *C;
-  int lda, ldb, ldc;
-  int m, n, K;
-};
+using GemmView = s8::View;
 
 // C (m x n) = A B  [kOverwrite, C may alias B: one row of tiles, so a CTA reads all of its columns of
 // B before it writes them]
@@ -175,6 +170,20 @@ cudaError_t gemm_launch(const JobDev *jobs, int njobs, int k, int max_m, int max
   if (max_m <= 0 || max_n <= 0) return cudaSuccess;
   if (launches) *launches += 1;
   return gemm_launch_tile<Op, MODE == kOverwrite ? 4 : 2, 2, MODE>(jobs, njobs, k, max_m, max_n, s);
+}
+
+// A pass's update at step k: on the integer tensor cores where it is large enough.
+template <class Op>
+cudaError_t subtract_launch(const JobDev *jobs, int njobs, int k, int max_m, int max_n, const SplitBufs *split, int pass,
+                            int *err, cudaStream_t s, long *launches) {
+  if (!split || !split_pays(max_m, max_n, njobs))
+    return gemm_launch<Op, kSubtract>(jobs, njobs, k, max_m, max_n, s, launches);
+  const Op op;
+  const cudaError_t e = s8::launch_split_pack(*split, jobs, njobs, k, max_m, max_n, s, op);
+  if (e != cudaSuccess) return e;
+  if (launches) *launches += 3;
+  return s8::launch_split_update(*split, jobs, njobs, k, max_m, max_n, false,
+                                 split->counters + pass * split->steps + k / kNb, err, s, op);
 }
 
 // One CTA per (LIZ position p, job): with G in M's storage, X refined and V = M^-1,
@@ -319,14 +328,17 @@ cudaError_t launch_tau_full(const JobDev *jobs, int njobs, int max_L, int max_N,
   return cudaGetLastError();
 }
 
-cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, cudaStream_t s, long *launches) {
+cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, const SplitBufs *split, int *err,
+                           cudaStream_t s, long *launches) {
   if (njobs <= 0) return cudaSuccess;
   cudaError_t e;
+  if (split && (e = cudaMemsetAsync(split->counters + split->steps, 0, 2 * sizeof(int) * split->steps, s)) != cudaSuccess)
+    return e;
   identity_kernel<<<dim3(max_N, njobs), 256, 0, s>>>(jobs);
   if (launches) *launches += 1;
   for (int k = 0; k < max_n; k += kNb) {
     if ((e = gemm_launch<OpInvDiag, kOverwrite>(jobs, njobs, k, kNb, k + kNb, s, launches)) != cudaSuccess) return e;
-    if ((e = gemm_launch<OpInvLower, kSubtract>(jobs, njobs, k, max_N - k - 1, k + kNb, s, launches)) != cudaSuccess)
+    if ((e = subtract_launch<OpInvLower>(jobs, njobs, k, max_N - k - 1, k + kNb, split, 1, err, s, launches)) != cudaSuccess)
       return e;
   }
   schur_inverse_kernel<<<njobs, 256, 0, s>>>(jobs);
@@ -334,7 +346,7 @@ cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, 
   if ((e = gemm_launch<OpSchurApply, kOverwrite>(jobs, njobs, 0, kMaxB, max_N, s, launches)) != cudaSuccess) return e;
   if ((e = gemm_launch<OpInvUpper, kSubtract>(jobs, njobs, -1, max_n, max_N, s, launches)) != cudaSuccess) return e;
   for (int k = ((max_n - 1) / kNb) * kNb; k >= 0 && max_n > 0; k -= kNb)
-    if ((e = gemm_launch<OpInvUpper, kSubtract>(jobs, njobs, k, k, max_N, s, launches)) != cudaSuccess) return e;
+    if ((e = subtract_launch<OpInvUpper>(jobs, njobs, k, k, max_N, split, 2, err, s, launches)) != cudaSuccess) return e;
   return cudaGetLastError();
 }
 

@@ -32,6 +32,7 @@
 #include "cplx.cuh"
 #include "dmma.cuh"
 #include "gj.cuh"
+#include "split8.cuh"
 
 namespace b200 {
 namespace {
@@ -457,6 +458,22 @@ __device__ __forceinline__ void update64_column(const JobDev &J, int k, int bx, 
 // Which tiles of the trailing block an update launch covers: all, the ones of its first 64 x 64
 // (the next step's diagonal block), or the others.
 enum { kAllTiles = 0, kFirstBlock = 1, kOtherTiles = 2 };
+
+// Step k's update as the integer tensor cores take it (split8.cuh).
+struct OpTrailing {
+  __device__ bool operator()(const JobDev &J, int k, s8::View &g) const {
+    if (k >= J.n || J.inactive) return false;
+    const int kb = min(kNb, J.n - k), e = k + kb;
+    double2 *F = static_cast<double2 *>(J.F);
+    g.A = F + (size_t)e + (size_t)k * J.ld;
+    g.B = F + (size_t)k + (size_t)e * J.ld;
+    g.C = F + (size_t)e + (size_t)e * J.ld;
+    g.lda = g.ldb = g.ldc = J.ld;
+    g.m = g.n = J.N - e;
+    g.K = kb;
+    return g.m > 0;
+  }
+};
 
 // W = D A12 overwrites its own operand, so a CTA takes all kb rows of its columns.
 template <int WN>
@@ -1055,7 +1072,8 @@ void launch_update64(const JobDev *jobs, int njobs, int k, int max_N, int part, 
 // first covers the next diagonal block, whose inverse (a chain of 64 dependent pivot steps on one
 // SM per job) then runs on the second stream beside the rest of the update.
 cudaError_t eliminate64(const JobDev *jobs, int njobs, int max_n, int max_N, int *info, cudaStream_t s,
-                        long *launches, KernelTimer *timer, bool sparse, const Lookahead *la, bool panel) {
+                        long *launches, KernelTimer *timer, bool sparse, const Lookahead *la, bool panel,
+                        const SplitBufs *split, int *err) {
   const int smem_diag = kNb * (kNb + 1) * (int)sizeof(double2);
   cudaError_t e;
   if ((e = ensure_smem(diag_inverse_kernel<double2, 1>, smem_diag)) != cudaSuccess) return e;
@@ -1063,6 +1081,8 @@ cudaError_t eliminate64(const JobDev *jobs, int njobs, int max_n, int max_N, int
   if ((e = ensure_smem(zgemm64_w_kernel<2>, dm::Tile<4, 2>::kSmem)) != cudaSuccess) return e;
   if ((e = ensure_smem(zgemm64_update_kernel, dm::Tile<2, 2>::kSmem)) != cudaSuccess) return e;
   const bool ahead = la != nullptr && la->s2 != nullptr && !sparse && !panel;
+  if (sparse) split = nullptr;
+  if (split && (e = cudaMemsetAsync(split->counters, 0, sizeof(int) * split->steps, s)) != cudaSuccess) return e;
   if (panel && (e = launch_pivot_init(jobs, njobs, s, launches)) != cudaSuccess) return e;
   for (int k = 0; k < max_n; k += kNb) {
     if (panel) {
@@ -1086,7 +1106,16 @@ cudaError_t eliminate64(const JobDev *jobs, int njobs, int max_n, int max_N, int
       launch_diag_inverse<double2>(false, jobs, njobs, k + kNb, info, smem_diag, la->s2);
       if ((e = cudaEventRecord(la->diag, la->s2)) != cudaSuccess) return e;
     }
-    launch_update64(jobs, njobs, k, max_N, next ? kOtherTiles : kAllTiles, sparse, s);
+    if (split && split_pays(rest, rest, njobs)) {
+      const OpTrailing op;
+      if ((e = s8::launch_split_pack(*split, jobs, njobs, k, rest, rest, s, op)) != cudaSuccess) return e;
+      if ((e = s8::launch_split_update(*split, jobs, njobs, k, rest, rest, next, split->counters + k / kNb, err, s, op)) !=
+          cudaSuccess)
+        return e;
+      if (launches) *launches += 2;
+    } else {
+      launch_update64(jobs, njobs, k, max_N, next ? kOtherTiles : kAllTiles, sparse, s);
+    }
     if (timed) cudaEventRecord(timer->ev[timer->used++], s);
     if (next && (e = cudaStreamWaitEvent(s, la->diag, 0)) != cudaSuccess) return e;
     if (launches) *launches += next ? 4 : 2;
@@ -1235,9 +1264,9 @@ cudaError_t launch_copy_to_factor(FactorKind fk, const double2 *M, void *F, int 
 
 cudaError_t launch_eliminate(FactorKind fk, const JobDev *jobs, int njobs, int max_n, int max_N, int *info,
                              cudaStream_t s, long *launches, KernelTimer *timer, const TcMaps *tc,
-                             int *err, bool sparse_jobs, const Lookahead *la, bool panel) {
+                             int *err, bool sparse_jobs, const Lookahead *la, bool panel, const SplitBufs *split) {
   if (fk == kFactorFP64)
-    return eliminate64(jobs, njobs, max_n, max_N, info, s, launches, timer, sparse_jobs, la, panel);
+    return eliminate64(jobs, njobs, max_n, max_N, info, s, launches, timer, sparse_jobs, la, panel, split, err);
   if (tc) {
     cudaError_t e = tc_prepare();
     if (e == cudaSuccess) e = launch_tc_counters_reset(*tc, s);

@@ -146,6 +146,10 @@ struct b200tau_ctx {
   TcMaps tc;
   float *d_pack = nullptr;
   int tc_ld = 0, tc_slots = 0;
+  // FP64 updates on the integer tensor cores: operand digit planes + TMA descriptors
+  SplitBufs split;
+  unsigned char *d_split = nullptr;
+  int split_ld = 0, split_slots = 0;
   // the mixed path's FP64 re-solve as graphs with a conditional body (fallback_graph)
   cudaStream_t cap_stream = nullptr;
   std::vector<FallbackGraph> fb;  // most recently used last
@@ -469,6 +473,56 @@ int ensure_tc(b200tau_ctx *ctx, int ld, int slots) {
   return B200TAU_OK;
 }
 
+// The digit planes of the FP64 update, for `slots` jobs of leading dimension up to ld.
+int ensure_split(b200tau_ctx *ctx, int ld, int slots) {
+  if (ctx->d_split && ld <= ctx->split_ld && slots <= ctx->split_slots) return B200TAU_OK;
+  CK(cudaStreamSynchronize(ctx->stream));
+  cudaFree(ctx->d_split);
+  ctx->d_split = nullptr;
+  ld = std::max(ld, ctx->split_ld);
+  slots = std::max(slots, ctx->split_slots);
+  SplitBufs &t = ctx->split;
+  t.ld = ld;
+  t.steps = ld / kNb + 1;
+  t.a_slot = (size_t)2 * ld * kSplitDigits * kSplitRowBytes;
+  t.b_slot = (size_t)ld * kSplitDigits * kSplitRowBytes;
+  CK(cudaMalloc(&ctx->d_split, split_slot_bytes(ld) * slots + sizeof(int) * kSplitCounters * t.steps));
+  t.a = reinterpret_cast<signed char *>(ctx->d_split);
+  t.b = t.a + t.a_slot * slots;
+  t.a_scale = reinterpret_cast<double *>(t.b + t.b_slot * slots);
+  t.b_scale = t.a_scale + (size_t)ld * slots;
+  t.balance = reinterpret_cast<int *>(t.b_scale + (size_t)ld * slots);
+  t.counters = t.balance + (size_t)kNb * slots;
+  void *fn = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  CK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
+  if (!fn || q != cudaDriverEntryPointSuccess) return fail(ctx, B200TAU_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+  EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(fn);
+  const cuuint32_t estr[3] = {1, 1, 1};
+  for (int i = 0; i < 2; ++i) {
+    const cuuint64_t rows = (cuuint64_t)(i == 0 ? 2 : 1) * ld * kSplitDigits;
+    const cuuint64_t dims[3] = {(cuuint64_t)kSplitRowBytes, rows, (cuuint64_t)slots};
+    const cuuint64_t strides[2] = {(cuuint64_t)kSplitRowBytes, rows * kSplitRowBytes};
+    const cuuint32_t box[3] = {(cuuint32_t)kSplitRowBytes, (cuuint32_t)(i == 0 ? 128 : 32), 1};
+    const CUresult r = enc(i == 0 ? &t.tA : &t.tB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, i == 0 ? t.a : t.b, dims, strides,
+                           box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(ctx, B200TAU_ERR_CUDA, "cuTensorMapEncodeTiled (digits) failed (%d)", (int)r);
+  }
+  ctx->split_ld = ld;
+  ctx->split_slots = slots;
+  return B200TAU_OK;
+}
+
+// The digit planes for a wave of FP64 factors, or null where no update is large enough for them.
+int split_for(b200tau_ctx *ctx, FactorKind fk, int maxN, int ld, int nw, const SplitBufs **out) {
+  *out = nullptr;
+  if (fk != kFactorFP64 || !split_pays(maxN, maxN, nw)) return B200TAU_OK;
+  const int rc = ensure_split(ctx, ld, std::max(nw, ctx->slots));
+  if (rc == B200TAU_OK) *out = &ctx->split;
+  return rc;
+}
+
 // Tensor map over the FP32 factor slots of the current wave (floats; column c of slot z starts at
 // z * f_bytes + c * 2 ld * 4 bytes), the destination of the tensor-core update's TMA reduce-add.
 int encode_factor_map(b200tau_ctx *ctx, int ld, int slots) {
@@ -741,10 +795,11 @@ int run_pipeline(b200tau_ctx *ctx, const std::vector<JobDev> &h, int nw, int max
     if ((rc = encode_factor_map(ctx, ld, ctx->slots))) return rc;
     tc = &ctx->tc;
   }
-  int rc = phase_begin(ctx);
-  if (rc) return rc;
+  const SplitBufs *split = nullptr;
+  int rc = split_for(ctx, p.fk, maxN, ld, nw, &split);
+  if (rc || (rc = phase_begin(ctx))) return rc;
   CK(launch_eliminate(p.fk, ctx->d_jobs, nw, maxn, maxN, ctx->d_info, ctx->stream, &ctx->launches,
-                      ctx->profiling ? &ctx->timer : nullptr, tc, ctx->d_err, false, &ctx->la, panel));
+                      ctx->profiling ? &ctx->timer : nullptr, tc, ctx->d_err, false, &ctx->la, panel, split));
   if ((rc = phase_end(ctx, 1)) || (rc = phase_begin(ctx))) return rc;
   if (p.steps > 0) {
     if ((rc = run_refinement(ctx, h, nw, maxn, maxN, b, ns, kkrsz, p, tc ? &tc->tFu : nullptr, panel))) return rc;
@@ -763,7 +818,7 @@ int run_pipeline(b200tau_ctx *ctx, const std::vector<JobDev> &h, int nw, int max
 // refinement's later rounds size their sweep clusters for a quarter of the wave's jobs.  The FP64
 // re-solve of unconverged mixed jobs stays a separate graph (fallback_graph).
 int wave_graph(b200tau_ctx *ctx, int nw, int maxL, int maxn, int maxN, int ld, const Plan &p, bool panel,
-               const TcMaps *tc, WaveGraph **out) {
+               const TcMaps *tc, const SplitBufs *split, WaveGraph **out) {
   const bool fp32_sweep = p.fk == kFactorFP32 && ctx->mixed_sweep == B200TAU_SWEEP_FP32;
   const std::vector<long long> key = {
       nw, maxL, maxn, maxN, ld, ctx->b, ctx->ns, ctx->kkrsz, (long long)p.fk, p.steps, p.f_separate ? 1 : 0,
@@ -771,7 +826,8 @@ int wave_graph(b200tau_ctx *ctx, int nw, int maxL, int maxn, int maxN, int ld, c
       ctx->tmat_ld, ctx->group_size, ctx->table_polls, (long long)(uintptr_t)ctx->d_jobs,
       (long long)(uintptr_t)ctx->d_info, (long long)(uintptr_t)ctx->d_active, (long long)(uintptr_t)ctx->d_err,
       (long long)(uintptr_t)ctx->d_tmat, (long long)(uintptr_t)ctx->d_tdiag, (long long)(uintptr_t)ctx->d_F,
-      (long long)(uintptr_t)ctx->d_pack, ctx->tc_ld, ctx->tc_slots, ctx->la.min_n, ctx->la.pair_min_rest};
+      (long long)(uintptr_t)ctx->d_pack, ctx->tc_ld, ctx->tc_slots, ctx->la.min_n, ctx->la.pair_min_rest,
+      (long long)(uintptr_t)(split ? ctx->d_split : nullptr), ctx->split_ld};
   for (size_t i = 0; i < ctx->wg.size(); ++i)
     if (ctx->wg[i].key == key) {
       const WaveGraph g = ctx->wg[i];  // most recently used last
@@ -790,7 +846,7 @@ int wave_graph(b200tau_ctx *ctx, int nw, int maxL, int maxn, int maxN, int ld, c
     e = launch_kkr_build(ctx->d_jobs, nw, maxL, build_params(ctx, p), ctx->d_err, cs, &n);
     if (e == cudaSuccess)
       e = launch_eliminate(p.fk, ctx->d_jobs, nw, maxn, maxN, ctx->d_info, cs, &n, nullptr, tc, ctx->d_err, false,
-                           &ctx->la, panel);
+                           &ctx->la, panel, split);
     if (p.steps > 0) {
       const CUtensorMap *fmap = tc ? &tc->tFu : nullptr;
       if (e == cudaSuccess)
@@ -902,7 +958,10 @@ int run_wave(b200tau_ctx *ctx, const b200tau_job *jobs, const int *idx, int nw, 
     gp.f_kind = 0;
     gp.g_mode = 1;
     CK(launch_kkr_build(ctx->d_jobs, nw, maxL, gp, ctx->d_err, ctx->stream, &ctx->launches));
-    CK(launch_inverse(ctx->d_jobs, nw, maxn, maxN, ctx->stream, &ctx->launches));
+    const SplitBufs *split = nullptr;
+    int rc = split_for(ctx, kFactorFP64, maxN, ld, nw, &split);
+    if (rc) return rc;
+    CK(launch_inverse(ctx->d_jobs, nw, maxn, maxN, split, ctx->d_err, ctx->stream, &ctx->launches));
     CK(launch_vjp_assemble(ctx->d_jobs, nw, maxL, ctx->kkrsz, ctx->ns, ctx->stream, &ctx->launches));
     return B200TAU_OK;
   }
@@ -916,7 +975,9 @@ int run_wave(b200tau_ctx *ctx, const b200tau_job *jobs, const int *idx, int nw, 
       tc = &ctx->tc;
     }
     WaveGraph *g = nullptr;
-    if ((rc = wave_graph(ctx, nw, maxL, maxn, maxN, ld, p, panel, tc, &g))) return rc;
+    const SplitBufs *split = nullptr;
+    if ((rc = split_for(ctx, p.fk, maxN, ld, nw, &split))) return rc;
+    if ((rc = wave_graph(ctx, nw, maxL, maxn, maxN, ld, p, panel, tc, split, &g))) return rc;
     CK(cudaGraphLaunch(g->exec, ctx->stream));
     ctx->launches += g->launches;
     if (p.fk != kFactorFP32 || !ctx->fallback_on || p.steps == 0) return B200TAU_OK;
@@ -940,7 +1001,9 @@ int run_wave(b200tau_ctx *ctx, const b200tau_job *jobs, const int *idx, int nw, 
   gp.f_kind = 0;
   gp.g_mode = 1;
   CK(launch_kkr_build(ctx->d_jobs, nw, maxL, gp, ctx->d_err, ctx->stream, &ctx->launches));
-  CK(launch_inverse(ctx->d_jobs, nw, maxn, maxN, ctx->stream, &ctx->launches));
+  const SplitBufs *split = nullptr;
+  if ((rc = split_for(ctx, kFactorFP64, maxN, ld, nw, &split))) return rc;
+  CK(launch_inverse(ctx->d_jobs, nw, maxn, maxN, split, ctx->d_err, ctx->stream, &ctx->launches));
   CK(launch_vjp_assemble(ctx->d_jobs, nw, maxL, ctx->kkrsz, ctx->ns, ctx->stream, &ctx->launches));
   return B200TAU_OK;
 }
@@ -1013,7 +1076,10 @@ int solve_impl(b200tau_ctx *ctx, const b200tau_job *jobs, int njobs, int prec, d
   const int maxN = ctx->atoms[jobs[order[0]].atom].N;
   const int ld = round_up(maxN, 64);
   // mixed with the FP64 re-solve enabled also holds an FP64 copy of M per slot
-  const size_t extra = (p.fk == kFactorFP32 && ctx->fallback_on) ? (size_t)ld * ld * sizeof(double2) : 0;
+  // and FP64 the digit planes of its updates
+  const size_t extra = p.fk == kFactorFP64  ? split_slot_bytes(ld)
+                       : ctx->fallback_on ? (size_t)ld * ld * sizeof(double2)
+                                          : 0;
   const int slots = choose_slots(ctx, ld, njobs, p, extra);
   if ((rc = ensure_workspace(ctx, ld, slots, p))) return rc;
   if ((rc = ensure_jobs(ctx, slots))) return rc;
@@ -1146,6 +1212,7 @@ void b200tau_destroy(b200tau_ctx *ctx) {
   cudaFree(ctx->d_t0);
   cudaFree(ctx->d_tdiag);
   cudaFree(ctx->d_pack);
+  cudaFree(ctx->d_split);
   cudaFree(ctx->d_V);
   cudaFree(ctx->d_adj);
   cudaFree(ctx->d_ffb);
@@ -1626,7 +1693,7 @@ int b200tau_solve_vjp(b200tau_ctx *ctx, const b200tau_job *jobs, int njobs, cons
   // the factors kept by a forward FP64 solve of these jobs (b200tau_set_keep_factors), used once
   const bool reuse = kept_matches(ctx, jobs, njobs) && ctx->kept_ld == ld && ctx->kept_order == order;
   ctx->kept_valid = false;
-  const int slots = reuse ? njobs : choose_slots(ctx, ld, njobs, p, v_need * sizeof(double2));
+  const int slots = reuse ? njobs : choose_slots(ctx, ld, njobs, p, v_need * sizeof(double2) + split_slot_bytes(ld));
   if ((rc = ensure_workspace(ctx, ld, slots, p))) return rc;
   if ((rc = ensure_jobs(ctx, slots))) return rc;
   if ((rc = ensure_v(ctx, ld, slots))) return rc;
@@ -1687,6 +1754,8 @@ int b200tau_solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau
   if ((rc = ensure_v(ctx, ld, 1))) return rc;
   const bool panel = use_panel(ctx, a.N, kFactorFP64);
   if (panel && (rc = ensure_piv(ctx, ld, 1))) return rc;
+  const SplitBufs *split = nullptr;
+  if ((rc = split_for(ctx, kFactorFP64, a.N, ld, 1, &split))) return rc;
   JobDev J;
   std::memset(&J, 0, sizeof(J));
   J.energy = make_double2(job->energy[0], job->energy[1]);
@@ -1712,8 +1781,8 @@ int b200tau_solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau
   ctx->launches = 0;
   CK(launch_kkr_build(ctx->d_jobs, 1, a.L, build_params(ctx, p), ctx->d_err, ctx->stream, &ctx->launches));
   CK(launch_eliminate(kFactorFP64, ctx->d_jobs, 1, J.n, J.N, ctx->d_info, ctx->stream, &ctx->launches, nullptr,
-                      nullptr, ctx->d_err, false, &ctx->la, panel));
-  CK(launch_inverse(ctx->d_jobs, 1, J.n, J.N, ctx->stream, &ctx->launches));
+                      nullptr, ctx->d_err, false, &ctx->la, panel, split));
+  CK(launch_inverse(ctx->d_jobs, 1, J.n, J.N, split, ctx->d_err, ctx->stream, &ctx->launches));
   CK(launch_tau_full(ctx->d_jobs, 1, a.L, a.N, tmat_view(ctx), ctx->stream, &ctx->launches));
   // reference site order (central site first): rows/cols [0, r) <-> [b, N), [r, N) <-> [0, b)
   const int r = a.N - a.b, b = a.b;

@@ -192,6 +192,34 @@ cudaError_t launch_tc_pack(const TcMaps &maps, const JobDev *jobs, int njobs, in
 cudaError_t launch_tc_update(const TcMaps &maps, const JobDev *jobs, int njobs, int k, int max_N, int *err,
                              cudaStream_t s, int part, int max_grid, int nblk = 1);
 cudaError_t launch_tc_counters_reset(const TcMaps &maps, cudaStream_t s);
+// Operand digit planes of the FP64 update on the integer tensor cores (split8.cuh).  Per wave slot:
+// A kSplitDigits planes of 2 ld rows, B kSplitDigits planes of ld rows, kSplitRowBytes each, and the
+// power-of-two scales of ld rows and ld columns, and of the kNb inner indices.
+constexpr int kSplitDigits = 8;
+constexpr int kSplitRowBytes = 2 * kNb;
+struct SplitBufs {
+  CUtensorMap tA, tB;  // {kSplitRowBytes, rows of all planes, slots}, boxes of 128 and 32 rows
+  signed char *a = nullptr, *b = nullptr;
+  size_t a_slot = 0, b_slot = 0;
+  double *a_scale = nullptr, *b_scale = nullptr;
+  int *balance = nullptr;  // kNb exponents per slot (balance_kernel)
+  int ld = 0;
+  int *counters = nullptr;  // work counters: kSplitCounters per step, zeroed before their launches
+  int steps = 0;
+};
+constexpr int kSplitCounters = 3;  // elimination, inverse lower pass, inverse upper pass
+constexpr size_t split_slot_bytes(int ld) {
+  return (size_t)ld * (3 * kSplitDigits * kSplitRowBytes + 2 * sizeof(double)) + kNb * sizeof(int);
+}
+// The integer tensor cores take an FP64 update of at least kSplitMin rows and columns and kSplitElems
+// elements of C over the wave: the packs and the fill of the pipeline cost some 35 us a launch, which the
+// faster products (30 against 50 to 60 TF/s) save from about 5 M elements on (a 64-column step; 31 jobs:
+// 400 x 400; one job of N = 2160 stays on the FP64 tensor cores).
+constexpr int kSplitMin = 256;
+constexpr long kSplitElems = 5L << 20;
+constexpr bool split_pays(int m, int n, int njobs) {
+  return m >= kSplitMin && n >= kSplitMin && (long)m * n * njobs >= kSplitElems;
+}
 // A second stream and two events for the elimination's look-ahead (all null: none).
 struct Lookahead {
   cudaStream_t s2 = nullptr;
@@ -229,12 +257,13 @@ cudaError_t launch_tdiag_flags(const double2 *tmat, long ld, int nstore, int gro
 // Block elimination of F over the first n columns (all jobs of the wave).
 // With FP32 factors and `tc` non-null the trailing update runs on the tensor cores (tc_update.cu).
 // `sparse_jobs`: most records are inactive (the FP64 re-solve), so the trailing update runs on a
-// small looping grid instead of one CTA per tile.  `panel`: the records carry pivot buffers and
+// small looping grid instead of one CTA per tile.  `split` (FP64): large updates run on the integer
+// tensor cores.  `panel`: the records carry pivot buffers and
 // every step picks its rows by panel pivoting (pivot.cu).
 cudaError_t launch_eliminate(FactorKind fk, const JobDev *jobs, int njobs, int max_n, int max_N,
                              int *info, cudaStream_t s, long *launches, KernelTimer *timer,
                              const TcMaps *tc, int *err, bool sparse_jobs = false,
-                             const Lookahead *la = nullptr, bool panel = false);
+                             const Lookahead *la = nullptr, bool panel = false, const SplitBufs *split = nullptr);
 // Panel pivoting (pivot.cu), for the records with a pivot buffer: the identity permutation; the
 // selection that picks step k's kb rows from [k, n) and writes the step's row moves; those moves
 // applied to columns [c0, c1) of F; and the final row positions for the residual.
@@ -309,7 +338,8 @@ cudaError_t launch_tau_full(const JobDev *jobs, int njobs, int max_L, int max_N,
                             long *launches);
 // Adjoint (adjoint.cu), FP64 factors: V = M^-1 from the block factors in F, then per LIZ site the
 // tau00 cotangent pull-back and d ln det M / d t (needs G in M, X refined, V).
-cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, cudaStream_t s, long *launches);
+cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, const SplitBufs *split, int *err,
+                           cudaStream_t s, long *launches);
 cudaError_t launch_vjp_assemble(const JobDev *jobs, int njobs, int max_L, int kkrsz, int ns, cudaStream_t s,
                                 long *launches);
 

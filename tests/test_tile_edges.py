@@ -159,3 +159,45 @@ def test_build_non_collinear_t(solver_factory, outer, coupled):
     got = s.build_kkr(0, 0, 0, prob.energies[0], prob.nrmat_ns)
     want = port.build_kkr(prob, 0)
     assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_reduced", [0, 3, 10])
+def test_updates_by_digit_products(solver_factory, n_reduced):
+    """32 jobs of N = 816 and less: the steps with enough elements run on the integer tensor cores, their
+    row panels, column tiles and the first block that the look-ahead takes out ending anywhere.  Against
+    the oracle, and against each job alone, which stays on the FP64 tensor cores; the gradients likewise
+    (the inverse's two passes)."""
+    from oracle import port
+    njobs = 32
+    L = W.lattice_shells("bcc", 5.42, 4).shape[1]
+    lmax = np.full(L, 3, np.int32)
+    lmax[L - n_reduced:] = 2
+    prob = W.make_problem("bcc", 5.42, 4, 3, W.semicircle_contour(-0.2, 0.7, njobs), 13, n_species=2, liz_lmax=lmax)
+    s = solver_factory(3, 1, 1)
+    s.load_problem(prob)
+    specs = [(0, i, 0, e) for i, e in enumerate(prob.energies)]
+    out = s.solve_jobs(T.make_jobs(specs), T.PREC_FP64)
+    rng = np.random.default_rng(2)
+    bar = rng.normal(size=(njobs, 16, 16)) + 1j * rng.normal(size=(njobs, 16, 16))
+    _, tb, ld = s.solve_vjp(T.make_jobs(specs), bar, [prob.num_liz] * njobs)
+    for i in (0, 15, 31):
+        # two backward-stable FP64 solves differ by a few times cond(M) 2^-53
+        bound = max(1e-12, 8 * np.linalg.cond(port.build_kkr(prob, i)) * 2.0 ** -53)
+        assert _tau_err(prob, i, out[i]) <= bound
+        alone = s.solve_jobs(T.make_jobs(specs[i:i + 1]), T.PREC_FP64)
+        assert _tau_err(prob, i, alone[0]) <= bound
+        # the gradients too go through one refined solve
+        _, tb1, ld1 = s.solve_vjp(T.make_jobs(specs[i:i + 1]), bar[i:i + 1], [prob.num_liz])
+        assert np.abs(tb[i] - tb1[0]).max() <= 10 * bound * np.abs(tb1[0]).max()
+        # d ln det M comes from the unrefined inverse, whose error is that of the block LU (pivots inside
+        # the diagonal blocks).  Against -((G M^-1)_jj)^T with t_j (G M^-1)_jj = (M^-1 - 1)_jj: the digits
+        # may not add to the error of the FP64 products, but for the spread of two such roundings.
+        inv = np.linalg.inv(port.build_kkr(prob, i))
+        off = np.concatenate([[0], np.cumsum((lmax + 1) ** 2)])
+        err = [0.0, 0.0]
+        for j in range(prob.num_liz):
+            k = off[j + 1] - off[j]
+            t = prob.t_block(int(prob.liz_store_idx[j]), i)[:k, :k]
+            want = -np.linalg.solve(t, inv[off[j]:off[j + 1], off[j]:off[j + 1]] - np.eye(k)).T
+            err = [max(e, np.abs(d[j][:k, :k] - want).max()) for e, d in zip(err, (ld[i], ld1[0]))]
+        assert err[0] <= 8 * err[1] + 10 * bound * np.abs(ld1[0]).max()
