@@ -236,12 +236,17 @@ Plan plan_for(const b200tau_ctx *ctx, int prec) {
   return p;
 }
 
+// N x b vectors per slot: X, R, Y, and the history of the accelerated refinement.
+size_t vec_elems_for(const Plan &p, int ld) {
+  return (size_t)(3 + (p.fk == kFactorFP32 ? kHistory : 0)) * ld * kMaxB;
+}
+
 size_t f_elem_bytes(const Plan &p) { return p.fk == kFactorFP32 ? sizeof(float2) : sizeof(double2); }
 
 int ensure_workspace(b200tau_ctx *ctx, int ld, int slots, const Plan &p) {
   const size_t m_need = (size_t)ld * ld;
   const size_t f_need = p.f_separate ? m_need * f_elem_bytes(p) : 0;
-  const size_t v_need = (size_t)3 * ld * kMaxB;
+  const size_t v_need = vec_elems_for(p, ld);
   const bool ok = ctx->d_M && m_need <= ctx->m_elems && f_need <= ctx->f_bytes &&
                   v_need <= ctx->vec_elems && slots <= ctx->slots;
   if (ok) return B200TAU_OK;
@@ -302,7 +307,7 @@ int choose_slots(b200tau_ctx *ctx, int ld, int njobs, const Plan &p, size_t extr
   // memory already held by the context's workspace counts as available to it
   freeb += ctx->m_elems * ctx->slots * sizeof(double2) + ctx->f_bytes * ctx->slots;
   const size_t per = (size_t)ld * ld * (sizeof(double2) + (p.f_separate ? f_elem_bytes(p) : 0)) +
-                     (size_t)3 * ld * kMaxB * sizeof(double2) + extra_per_slot;
+                     vec_elems_for(p, ld) * sizeof(double2) + extra_per_slot;
   const size_t budget = freeb / 2;
   int s = (int)std::max<size_t>(1, budget / std::max<size_t>(per, 1));
   s = std::min(s, ctx->max_slots);
@@ -317,6 +322,7 @@ void fill_slot(b200tau_ctx *ctx, JobDev &J, int slot, int ld, const Plan &p) {
   J.X = v;
   J.R = v + (size_t)ld * kMaxB;
   J.Y = v + (size_t)2 * ld * kMaxB;
+  J.hist = p.fk == kFactorFP32 ? v + (size_t)3 * ld * kMaxB : nullptr;
   J.ld = ld;
   J.conv = ctx->d_conv + slot;
   J.cnorm = ctx->d_cnorm + slot;
@@ -747,10 +753,12 @@ int run_refinement(b200tau_ctx *ctx, const std::vector<JobDev> &h, int nw, int m
   refresh_active_hint(ctx);
   CK(launch_refine_begin(p.fk, ctx->d_jobs, nw, maxn, maxN, b, ctx->d_info, ctx->stream, &ctx->launches,
                          fp32_sweep, fmap));
+  const bool accelerate = p.fk == kFactorFP32 && p.steps > 2;
+  if (accelerate) CK(launch_accelerate(ctx->d_jobs, nw, b, 0, ctx->stream, &ctx->launches));
   for (int it = 0; it < p.steps; ++it) {
     const int hint = it >= kHintAfterRounds ? ctx->active_hint : 0;
     CK(launch_refine_round(p.fk, ctx->d_jobs, nw, maxn, maxN, b, true, ctx->d_info, ctx->stream, &ctx->launches,
-                           fp32_sweep, fmap, hint, ctx->d_active));
+                           fp32_sweep, fmap, hint, ctx->d_active, accelerate ? it + 1 : 0));
     if (it + 1 == kHintAfterRounds && p.steps > kHintAfterRounds && !ctx->hint_pending) {
       if (ctx->h_hint_cap < nw) {  // (no copy into the old buffer is pending)
         if (ctx->h_hint) cudaFreeHost(ctx->h_hint);
@@ -854,9 +862,13 @@ int wave_graph(b200tau_ctx *ctx, int nw, int maxL, int maxn, int maxN, int ld, c
       // rounds after kHintAfterRounds size their sweep clusters for a quarter of the wave (most jobs
       // have converged by then; if more are left their clusters run in two waves, which costs about
       // what the smaller clusters would)
-      for (int it = 0; it < p.steps && e == cudaSuccess; ++it)
+      const bool accelerate = p.fk == kFactorFP32 && p.steps > 2;
+      if (accelerate && e == cudaSuccess) e = launch_accelerate(ctx->d_jobs, nw, ctx->b, 0, cs, &n);
+      for (int it = 0; it < p.steps && e == cudaSuccess; ++it) {
         e = launch_refine_round(p.fk, ctx->d_jobs, nw, maxn, maxN, ctx->b, true, ctx->d_info, cs, &n, fp32_sweep,
-                                fmap, it >= kHintAfterRounds ? std::max(1, (nw + 3) / 4) : 0, ctx->d_active);
+                                fmap, it >= kHintAfterRounds ? std::max(1, (nw + 3) / 4) : 0, ctx->d_active,
+                                accelerate ? it + 1 : 0);
+      }
       if (e == cudaSuccess) e = launch_refine_end(ctx->d_jobs, nw, ctx->ns, ctx->kkrsz, cs, &n);
     } else if (e == cudaSuccess) {
       e = launch_finalize_direct(p.fk, ctx->d_jobs, nw, ctx->ns, ctx->kkrsz, ctx->d_info, cs, &n);

@@ -32,6 +32,9 @@ constexpr int kTcTileCols = 256;
 // A refining job stops once its estimated remaining error on tau00 is below this fraction of
 // max|tau00|: 100x below the mixed path's 1e-10 accuracy target.
 constexpr double kRefineTol = 1e-12;
+// N x b vectors that the accelerated refinement of FP32 factors keeps: the iterate before the round, and
+// the corrected iterates and corrections of two earlier rounds (accelerate_kernel, block_lu.cu).
+constexpr int kHistory = 5;
 // JobDev::conv values (0: still refining)
 constexpr int kConverged = 1;
 constexpr int kDiverged = 2;  // the corrections stopped shrinking (numerical)
@@ -115,6 +118,7 @@ struct JobDev {
   double2 *tbar;         // L blocks of b x b, LIZ site order: d<taubar, tau00>/d t_site
   double2 *dlogdet;      // L blocks of b x b: d ln det M / d t_site (may be null)
   int *err;              // the context's device error word (kErr* bits), or null
+  double2 *hist;         // kHistory N x b vectors of the accelerated refinement (MIXED), or null
   int *piv;              // panel pivoting's buffer (pivot_ints(ld) ints), null: pivots inside the
                          // 64 x 64 diagonal blocks only
 };
@@ -302,7 +306,9 @@ cudaError_t launch_refine_begin(FactorKind fk, const JobDev *jobs, int njobs, in
 // there and spreads its CTAs over them alone.
 cudaError_t launch_refine_round(FactorKind fk, const JobDev *jobs, int njobs, int max_n, int max_N, int b,
                                 bool check, int *info, cudaStream_t s, long *launches, bool fp32_sweep = false,
-                                const CUtensorMap *fmap = nullptr, int active_hint = 0, int *active = nullptr);
+                                const CUtensorMap *fmap = nullptr, int active_hint = 0, int *active = nullptr, int accelerate = 0);
+// The accelerated step of a round (MIXED records with history): round 0 is the initial solve.
+cudaError_t launch_accelerate(const JobDev *jobs, int njobs, int b, int round, cudaStream_t s, long *launches);
 cudaError_t launch_refine_end(const JobDev *jobs, int njobs, int ns, int kkrsz, cudaStream_t s, long *launches);
 // One block sweep of the correction solve for all jobs, one thread-block cluster per job
 // (sweep.cu): forward (R -> Y over the D_k, A21_k factors) or backward (Y over the W_k factors,
