@@ -191,12 +191,15 @@ cudaError_t subtract_launch(const JobDev *jobs, int njobs, int k, int max_m, int
 //   tbar_site = Lambda Z^T (+ Lambda for the central site),  dlogdet_site = -H^T,
 // written as b x b blocks in the t-matrix store layout (row s kkrsz + lm for the site's lm < kk,
 // zero elsewhere).  bp = ns kk <= kMaxB.
-constexpr int kAk = 32;  // K chunk of the contraction
-constexpr int kVjpSmem =
-    (int)sizeof(double2) * (kMaxB * (kAk + 1) + 2 * kAk * (kMaxB + 1)) > (int)sizeof(double2) * 3 * kMaxB * (kMaxB + 1)
-        ? (int)sizeof(double2) * (kMaxB * (kAk + 1) + 2 * kAk * (kMaxB + 1))
-        : (int)sizeof(double2) * 3 * kMaxB * (kMaxB + 1);
+//
+// The two contractions run on the FP64 tensor cores: warps 0 - 3 take Z, 4 - 7 H, each every fourth K
+// step of 4, with the MMA fragments loaded straight from global memory (a G fragment is eight rows of
+// four columns, an X or V fragment four rows of eight columns: whole 32-byte sectors); the four partial
+// results are added in shared memory in warp order.  NB = 2 or 4 blocks of eight a side (bp, b <= 8 NB).
+// 16 jobs of 87 sites (N = 1392) take 402 us; the DFMA form took 1180 us.
+constexpr int kVjpSmem = (int)sizeof(double2) * 3 * kMaxB * (kMaxB + 1);
 
+template <int NB>
 __global__ void __launch_bounds__(256) vjp_assemble_kernel(const JobDev *__restrict__ jobs, int kkrsz, int ns) {
   const JobDev &J = jobs[blockIdx.y];
   const int p = blockIdx.x;
@@ -205,53 +208,60 @@ __global__ void __launch_bounds__(256) vjp_assemble_kernel(const JobDev *__restr
   const int site = J.perm[p];
   const int kk = bp / ns;
   const int N = J.N, n = J.n, b = J.b, ld = J.ld;
-  // K-chunk staging (G rows of the site, X, V columns of the site), then Z, H and Lambda in the
-  // same shared memory (vjp_smem_bytes)
   extern __shared__ __align__(16) unsigned char vsm[];
-  double2(*Gs)[kAk + 1] = reinterpret_cast<double2(*)[kAk + 1]>(vsm);
-  double2(*Xs)[kMaxB + 1] = reinterpret_cast<double2(*)[kMaxB + 1]>(vsm + sizeof(double2) * kMaxB * (kAk + 1));
-  double2(*Vs)[kMaxB + 1] = Xs + kAk;
   double2(*Zs)[kMaxB + 1] = reinterpret_cast<double2(*)[kMaxB + 1]>(vsm);
   double2(*Hs)[kMaxB + 1] = Zs + kMaxB;
   double2(*Ls)[kMaxB + 1] = Hs + kMaxB;  // Lambda
-  const int tid = threadIdx.x;
-  // each thread owns up to 4 entries of Z (bp x b) and of H (bp x bp): entry e = tid + 256 q
-  double2 zacc[4], hacc[4];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  {
+    const bool z = warp < 4;  // Z = G X, else H = G V[:, p]
+    const double2 *__restrict__ Gp = J.M + off + g;
+    const double2 *__restrict__ Bp = z ? J.X : J.V + (size_t)off * ld;
+    const int nc = z ? b : bp;
+    const double2 zero = make_double2(0.0, 0.0);
+    double re[NB][NB][2], im[NB][NB][2];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) zacc[q] = hacc[q] = make_double2(0.0, 0.0);
-  for (int kc = 0; kc < N; kc += kAk) {
-    for (int e = tid; e < bp * kAk; e += 256) {
-      const int i = e % bp, kq = e / bp;
-      Gs[i][kq] = kc + kq < N ? J.M[(size_t)(off + i) + (size_t)(kc + kq) * ld] : make_double2(0.0, 0.0);
-    }
-    for (int e = tid; e < kAk * b; e += 256) {
-      const int kq = e % kAk, c = e / kAk;
-      Xs[kq][c] = kc + kq < N ? J.X[(size_t)(kc + kq) + (size_t)c * ld] : make_double2(0.0, 0.0);
-    }
-    for (int e = tid; e < kAk * bp; e += 256) {
-      const int kq = e % kAk, c = e / kAk;
-      Vs[kq][c] = kc + kq < N ? J.V[(size_t)(kc + kq) + (size_t)(off + c) * ld] : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
+    for (int i = 0; i < NB; ++i)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + 256 * q;
-      if (e < bp * b) {
-        const int i = e % bp, c = e / bp;
-        for (int kq = 0; kq < kAk; ++kq) zacc[q] = cfma(Gs[i][kq], Xs[kq][c], zacc[q]);
-      }
-      if (e < bp * bp) {
-        const int i = e % bp, c = e / bp;
-        for (int kq = 0; kq < kAk; ++kq) hacc[q] = cfma(Gs[i][kq], Vs[kq][c], hacc[q]);
-      }
-    }
-    __syncthreads();
-  }
+      for (int j = 0; j < NB; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+#pragma unroll 2
+    for (int k0 = 4 * (warp & 3); k0 < N; k0 += 16) {
+      const int k = k0 + t;
+      double2 a[NB], x[NB];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {  // (the last barrier of the K loop freed the staging memory)
-    const int e = tid + 256 * q;
-    if (e < bp * b) Zs[e % bp][e / bp] = zacc[q];
-    if (e < bp * bp) Hs[e % bp][e / bp] = hacc[q];
+      for (int i = 0; i < NB; ++i) a[i] = k < N && 8 * i + g < bp ? Gp[8 * i + (size_t)k * ld] : zero;
+#pragma unroll
+      for (int j = 0; j < NB; ++j) x[j] = k < N && 8 * j + g < nc ? Bp[k + (size_t)(8 * j + g) * ld] : zero;
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          dm::mma_884(re[i][j][0], re[i][j][1], a[i].x, x[j].x);
+          dm::mma_884(im[i][j][0], im[i][j][1], a[i].x, x[j].y);
+        }
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          dm::mma_884(re[i][j][0], re[i][j][1], -a[i].y, x[j].y);
+          dm::mma_884(im[i][j][0], im[i][j][1], a[i].y, x[j].x);
+        }
+    }
+    double2(*D)[kMaxB + 1] = z ? Zs : Hs;
+    for (int w = 0; w < 4; ++w) {
+      if ((warp & 3) == w)
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+#pragma unroll
+          for (int j = 0; j < NB; ++j)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              double2 &d = D[8 * i + g][8 * j + 2 * t + q];
+              d = w == 0 ? make_double2(re[i][j][q], im[i][j][q])
+                         : make_double2(d.x + re[i][j][q], d.y + im[i][j][q]);
+            }
+      __syncthreads();
+    }
   }
   // Lambda[i][c] = sum_r V[n + r][off + i] taubar[r][c]
   for (int e = tid; e < bp * b; e += 256) {
@@ -353,9 +363,12 @@ cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, 
 cudaError_t launch_vjp_assemble(const JobDev *jobs, int njobs, int max_L, int kkrsz, int ns, cudaStream_t s,
                                 long *launches) {
   if (njobs <= 0) return cudaSuccess;
-  cudaError_t e = ensure_smem(vjp_assemble_kernel, kVjpSmem);
+  const int nb = ns * kkrsz <= 16 ? 2 : 4;
+  const cudaError_t e = nb == 2 ? ensure_smem(vjp_assemble_kernel<2>, kVjpSmem) : ensure_smem(vjp_assemble_kernel<4>, kVjpSmem);
   if (e != cudaSuccess) return e;
-  vjp_assemble_kernel<<<dim3(max_L, njobs), 256, kVjpSmem, s>>>(jobs, kkrsz, ns);
+  const dim3 grid(max_L, njobs);
+  if (nb == 2) vjp_assemble_kernel<2><<<grid, 256, kVjpSmem, s>>>(jobs, kkrsz, ns);
+  else vjp_assemble_kernel<4><<<grid, 256, kVjpSmem, s>>>(jobs, kkrsz, ns);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }
