@@ -443,14 +443,15 @@ __global__ void __launch_bounds__(256, 2) zgemm_strips_kernel(const JobDev *__re
 // step k's W = D A12 (kOverwrite) and A22 -= A21 W (kSubtract).
 // ---------------------------------------------------------------------------------------------
 // A column of `len` tiles of step k's trailing block from tile (bx, by) down.
+template <int W>
 __device__ __forceinline__ void update64_column(const JobDev &J, int k, int bx, int by, int len, double2 *sm) {
-  constexpr int R = dm::Tile<2, 2>::kRows, C = dm::Tile<2, 2>::kCols;
+  constexpr int R = dm::Tile<W, W>::kRows, C = dm::Tile<W, W>::kCols;
   const int N = J.N, ld = J.ld;
   const int kb = min(kNb, J.n - k);
   double2 *F = static_cast<double2 *>(J.F);
   const int col0 = k + kb + bx * C, row0 = k + kb + by * R;
   if (col0 >= N || row0 >= N) return;
-  dm::zgemm_column<2, 2, kSubtract>(F + (size_t)row0 + (size_t)k * ld, ld, F + (size_t)k + (size_t)col0 * ld, ld,
+  dm::zgemm_column<W, W, kSubtract>(F + (size_t)row0 + (size_t)k * ld, ld, F + (size_t)k + (size_t)col0 * ld, ld,
                                       F + (size_t)row0 + (size_t)col0 * ld, ld, min(len * R, N - row0),
                                       min(C, N - col0), kb, sm);
 }
@@ -490,14 +491,16 @@ __global__ void __launch_bounds__(dm::kThreads, 2) zgemm64_w_kernel(const JobDev
                                       min(dm::Tile<4, WN>::kCols, J.N - col0), kb, zsm64);
 }
 
-// 32 x 32 tiles in columns of `len`: tx columns of tiles, ty rows of columns.  Four CTAs of four warps
+// Tiles of 16 W x 16 W in columns of `len`: tx columns of tiles, ty rows of columns.  W = 2, or 1 for the
+// next diagonal block of a few jobs (a tile keeps its SM's FP64 pipe for 2.2 us with W = 2).  Four CTAs of four warps
 // on an SM: 31 jobs of N = 2160 took 32.3 ms of updates with 64 x 64 tiles at two CTAs, 28.4 with
 // 64 x 32 at three, 27.9 with these at four (48.2 -> 30.0 ms for the whole elimination, from DFMA tiles
 // without look-ahead).
+template <int W>
 __global__ void __launch_bounds__(dm::kThreads, 4) zgemm64_update_kernel(const JobDev *__restrict__ jobs, int k, int tx,
                                                                          int ty, int nj, int part, int len) {
   extern __shared__ __align__(16) double2 zsm64[];
-  using TL = dm::Tile<2, 2>;
+  using TL = dm::Tile<W, W>;
   if (gridDim.z == (unsigned)nj) {
     const JobDev &J = jobs[blockIdx.z];
     const int bx = blockIdx.x;
@@ -509,7 +512,7 @@ __global__ void __launch_bounds__(dm::kThreads, 4) zgemm64_update_kernel(const J
       l -= skip;
       if (l <= 0) return;
     }
-    update64_column(J, k, bx, by, l, zsm64);
+    update64_column<W>(J, k, bx, by, l, zsm64);
     return;
   }
   // a 1-D grid smaller than the tiles (the FP64 re-solve of a mixed wave, where most jobs are
@@ -519,7 +522,7 @@ __global__ void __launch_bounds__(dm::kThreads, 4) zgemm64_update_kernel(const J
     const JobDev &J = jobs[z];
     if (J.inactive || k >= J.n) continue;
     for (int v = blockIdx.x; v < tx * ty; v += gridDim.x)
-      update64_column(J, k, v % tx, (v / tx) * len, len, zsm64);
+      update64_column<W>(J, k, v % tx, (v / tx) * len, len, zsm64);
   }
 }
 
@@ -1058,14 +1061,20 @@ cudaError_t eliminate32(const JobDev *jobs, int njobs, int max_n, int max_N, int
   return cudaGetLastError();
 }
 
-void launch_update64(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, cudaStream_t s) {
-  using TL = dm::Tile<2, 2>;
+template <int W>
+void launch_update64_tiles(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, cudaStream_t s) {
+  using TL = dm::Tile<W, W>;
   const int rows = part == kFirstBlock ? kNb : max_N - k - 1;
   const int tx = (rows + TL::kCols - 1) / TL::kCols, tr = (rows + TL::kRows - 1) / TL::kRows;
   const int len = sparse ? 1 : dm::column_tiles((long)tx * tr * njobs);
   const int ty = (tr + len - 1) / len;
   const dim3 grid = sparse ? dim3(std::min(tx * ty * njobs, kSparseGrid)) : dim3(tx, ty, njobs);
-  zgemm64_update_kernel<<<grid, dm::kThreads, TL::kSmem, s>>>(jobs, k, tx, ty, njobs, part, len);
+  zgemm64_update_kernel<W><<<grid, dm::kThreads, TL::kSmem, s>>>(jobs, k, tx, ty, njobs, part, len);
+}
+
+void launch_update64(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, cudaStream_t s) {
+  if (part == kFirstBlock && 16 * njobs <= 4 * 148) launch_update64_tiles<1>(jobs, njobs, k, max_N, part, sparse, s);
+  else launch_update64_tiles<2>(jobs, njobs, k, max_N, part, sparse, s);
 }
 
 // FP64 factors.  With a second stream (and pivots inside the diagonal blocks) the update of step k
@@ -1079,7 +1088,9 @@ cudaError_t eliminate64(const JobDev *jobs, int njobs, int max_n, int max_N, int
   if ((e = ensure_smem(diag_inverse_kernel<double2, 1>, smem_diag)) != cudaSuccess) return e;
   if ((e = ensure_smem(diag_inverse_kernel<double2, 2>, smem_diag)) != cudaSuccess) return e;
   if ((e = ensure_smem(zgemm64_w_kernel<2>, dm::Tile<4, 2>::kSmem)) != cudaSuccess) return e;
-  if ((e = ensure_smem(zgemm64_update_kernel, dm::Tile<2, 2>::kSmem)) != cudaSuccess) return e;
+  if ((e = ensure_smem(zgemm64_update_kernel<1>, dm::Tile<1, 1>::kSmem)) != cudaSuccess) return e;
+  if ((e = ensure_smem(zgemm64_update_kernel<2>, dm::Tile<2, 2>::kSmem)) != cudaSuccess) return e;
+  if ((e = ensure_smem(zgemm64_w_kernel<1>, dm::Tile<4, 1>::kSmem)) != cudaSuccess) return e;
   const bool ahead = la != nullptr && la->s2 != nullptr && !sparse && !panel;
   if (sparse) split = nullptr;
   if (split && (e = cudaMemsetAsync(split->counters, 0, sizeof(int) * split->steps, s)) != cudaSuccess) return e;
@@ -1096,7 +1107,11 @@ cudaError_t eliminate64(const JobDev *jobs, int njobs, int max_n, int max_N, int
     const int rest = max_N - k - 1;
     if (rest <= 0) continue;
     const bool next = ahead && k + kNb < max_n;
-    zgemm64_w_kernel<2><<<dim3((rest + 31) / 32, 1, njobs), dm::kThreads, dm::Tile<4, 2>::kSmem, s>>>(jobs, k);
+    // 16 columns a CTA where that is at most a CTA an SM (half the time of a 32-column tile: 9 -> 7.9 us)
+    if ((rest + 15) / 16 * njobs <= 148)
+      zgemm64_w_kernel<1><<<dim3((rest + 15) / 16, 1, njobs), dm::kThreads, dm::Tile<4, 1>::kSmem, s>>>(jobs, k);
+    else
+      zgemm64_w_kernel<2><<<dim3((rest + 31) / 32, 1, njobs), dm::kThreads, dm::Tile<4, 2>::kSmem, s>>>(jobs, k);
     const bool timed = timer && timer->used + 2 <= timer->cap;
     if (timed) cudaEventRecord(timer->ev[timer->used++], s);
     if (next) {
