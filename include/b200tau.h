@@ -175,6 +175,8 @@ int b200tau_solve_dense_noalloc(const double *m, int n, int ldm, const double *t
  * group's first energy) and each site's block has the site's own size (the reference places
  * kkrsz_ns x kkrsz_ns blocks at multiples of kkrsz_ns). */
 int b200tau_solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau_full, int n);
+/* The same, row-major. */
+int b200tau_solve_tau_full_rows(b200tau_ctx *ctx, const b200tau_job *job, double *tau_full, int n);
 
 /* Build only: the KKR matrix M = 1 - t G for one job in the reference's site
  * order (central site first), written to host memory (n x n, ld = n) where

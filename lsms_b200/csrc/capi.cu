@@ -1747,7 +1747,7 @@ int b200tau_solve_vjp(b200tau_ctx *ctx, const b200tau_job *jobs, int njobs, cons
   return check_err_flags(ctx);
 }
 
-int b200tau_solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau_full, int n) {
+static int solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau_full, int n, bool rows) {
   if (!ctx) return B200TAU_ERR_ARG;
   ctx->kept_valid = false;
   if (!job || !tau_full) return fail(ctx, B200TAU_ERR_ARG, "solve_tau_full: bad arguments");
@@ -1795,22 +1795,8 @@ int b200tau_solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau
   CK(launch_eliminate(kFactorFP64, ctx->d_jobs, 1, J.n, J.N, ctx->d_info, ctx->stream, &ctx->launches, nullptr,
                       nullptr, ctx->d_err, false, &ctx->la, panel, split));
   CK(launch_inverse(ctx->d_jobs, 1, J.n, J.N, split, ctx->d_err, ctx->stream, &ctx->launches));
-  CK(launch_tau_full(ctx->d_jobs, 1, a.L, a.N, tmat_view(ctx), ctx->stream, &ctx->launches));
-  // reference site order (central site first): rows/cols [0, r) <-> [b, N), [r, N) <-> [0, b)
-  const int r = a.N - a.b, b = a.b;
-  const size_t es = sizeof(double2);
-  double2 *hm = reinterpret_cast<double2 *>(tau_full);
-  const double2 *W = J.M;
-  if (r > 0) {
-    CK(cudaMemcpy2DAsync(hm + b + (size_t)b * n, n * es, W, ld * es, r * es, r, cudaMemcpyDeviceToHost,
-                         ctx->stream));
-    CK(cudaMemcpy2DAsync(hm + b, n * es, W + (size_t)r * ld, ld * es, r * es, b, cudaMemcpyDeviceToHost,
-                         ctx->stream));
-    CK(cudaMemcpy2DAsync(hm + (size_t)b * n, n * es, W + r, ld * es, b * es, r, cudaMemcpyDeviceToHost,
-                         ctx->stream));
-  }
-  CK(cudaMemcpy2DAsync(hm, n * es, W + r + (size_t)r * ld, ld * es, b * es, b, cudaMemcpyDeviceToHost,
-                       ctx->stream));
+  CK(launch_tau_full(ctx->d_jobs, 1, a.L, a.N, tmat_view(ctx), rows, ctx->stream, &ctx->launches));
+  CK(cudaMemcpyAsync(tau_full, J.M, sizeof(double2) * n * n, cudaMemcpyDeviceToHost, ctx->stream));
   int info = 0;
   CK(cudaMemcpyAsync(&info, ctx->d_info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1818,6 +1804,14 @@ int b200tau_solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau
   if ((rc = check_host_err(ctx))) return rc;
   if (info) return fail(ctx, B200TAU_ERR_SINGULAR, "solve_tau_full: singular pivot (info %d)", info);
   return B200TAU_OK;
+}
+
+int b200tau_solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau_full, int n) {
+  return solve_tau_full(ctx, job, tau_full, n, false);
+}
+
+int b200tau_solve_tau_full_rows(b200tau_ctx *ctx, const b200tau_job *job, double *tau_full, int n) {
+  return solve_tau_full(ctx, job, tau_full, n, true);
 }
 
 int b200tau_build_kkr(b200tau_ctx *ctx, const b200tau_job *job, double *m_out, int n) {

@@ -340,8 +340,8 @@ struct TmatView {
 };
 // Full tau = M^-1 T into M's storage (positions order), from V = M^-1 (or (P M)^-1 with panel
 // pivoting) and the sites' t-matrices; the contract of the reference's solveTauFullzgetrf.
-cudaError_t launch_tau_full(const JobDev *jobs, int njobs, int max_L, int max_N, const TmatView &tv, cudaStream_t s,
-                            long *launches);
+cudaError_t launch_tau_full(const JobDev *jobs, int njobs, int max_L, int max_N, const TmatView &tv, bool rows,
+                            cudaStream_t s, long *launches);
 // Adjoint (adjoint.cu), FP64 factors: V = M^-1 from the block factors in F, then per LIZ site the
 // tau00 cotangent pull-back and d ln det M / d t (needs G in M, X refined, V).
 cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, const SplitBufs *split, int *err,

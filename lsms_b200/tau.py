@@ -53,7 +53,7 @@ EXPORTS = (
     "b200tau_profile_read", "b200tau_set_mixed_engine", "b200tau_solve_dense_noalloc",
     "b200tau_profile_phases", "b200tau_set_mixed_sweep", "b200tau_solve_vjp",
     "b200tau_last_fallback_count", "b200tau_set_mixed_fallback", "b200tau_set_build_wait",
-    "b200tau_set_pivoting", "b200tau_solve_tau_full", "b200tau_set_graphs",
+    "b200tau_set_pivoting", "b200tau_solve_tau_full", "b200tau_solve_tau_full_rows", "b200tau_set_graphs",
     "b200tau_set_keep_factors", "b200tau_set_paired_steps",
     "b200tau_autotune_paired_steps",
 )
@@ -114,6 +114,7 @@ def load_library():
     lib.b200tau_set_build_wait.argtypes = [P, L]
     lib.b200tau_set_pivoting.argtypes = [P, I]
     lib.b200tau_solve_tau_full.argtypes = [P, P, P, I]
+    lib.b200tau_solve_tau_full_rows.argtypes = [P, P, P, I]
     lib.b200tau_set_graphs.argtypes = [P, I]
     lib.b200tau_set_paired_steps.argtypes = [P, I]
     lib.b200tau_autotune_paired_steps.argtypes = [P, P, I, P, I, I, P, P]
@@ -366,9 +367,9 @@ class TauSolver:
         """Full tau = M^-1 T (numpy [row, col], reference site order): solveTauFullzgetrf's
         contract (linearSolvers_CPU.cpp:125-144), as the Kubo current matrix uses it."""
         jobs = make_jobs([(atom, iie, ispin, energy)])
-        out = np.zeros((n * n,), np.complex128)
-        self._check(self.lib.b200tau_solve_tau_full(self.ctx, ctypes.cast(jobs, ctypes.c_void_p), _ptr(out), n))
-        return out.reshape(n, n).T.copy()
+        out = np.zeros((n, n), np.complex128)
+        self._check(self.lib.b200tau_solve_tau_full_rows(self.ctx, ctypes.cast(jobs, ctypes.c_void_p), _ptr(out), n))
+        return out
 
     def build_kkr(self, atom: int, iie: int, ispin: int, energy: complex, n: int) -> np.ndarray:
         """The device-built KKR matrix in the reference's site order (numpy [row, col])."""
