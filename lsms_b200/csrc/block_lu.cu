@@ -45,163 +45,186 @@ using namespace cx;
 // Rows are never interchanged: step p pivots on the not-yet-used row pv with the largest
 // |A[pv][p]|, and the permutation is applied when the block is written back (for the in-place
 // result P, A^-1[i][pv_k] = P[pv_i][k]).
-// One Gauss-Jordan step as a single rank-1 update of the whole block, A[r][c] -= g_r u_c, with
-//   u = row pv, except u_p = d + 1 (d = A[pv][p]);   g_r = A[r][p] / d (r != pv),  g_pv = 1 - 1/d:
-// row pv becomes A[pv][c] / d, column p becomes -A[r][p] / d, and A[pv][p] becomes 1/d, as the
-// in-place inverse needs, with no special cases in the update.
-// Layout: warp w holds columns 8w .. 8w + 7 and lane l rows l and l + 32, in registers (the step
-// loop is not unrolled: an unrolled body outgrows the instruction caches).  A step's update writes each
-// column one place down, so the column to search next is always the first (a selection by index cost
-// 130 instructions of the chain) and after eight steps the columns are back in place.  A launch of one
-// block takes 45 us, some 1250 cycles a step (52 us with the columns in fixed places and the search after
-// the whole update; 59 us with the warps run ahead on one mbarrier per step instead of the block barrier).
-// What bounds the kernel is the chain from one pivot to the next, so in step p the warp that holds
-// column p + 1 updates that column first, searches it (warp argmax, with every lane's reciprocal of
-// its own candidate computed beside the reductions) and publishes step p + 1's g before it updates its
-// other columns; the one block barrier of the step follows.  In every warp the lane holding row pv
-// publishes u over the warp's columns (a per-warp slot in shared memory, read only by that warp).
+// One step subtracts g u^T from every column but p, u = row pv, g_r = A[r][p] / d (d = A[pv][p]) and
+// g_pv = 1 - 1/d, which leaves row pv divided by d; column p becomes -g_r, and 1/d in row pv.
+//
+// What bounds the kernel is the chain from one pivot to the next, so the block is taken in panels of
+// eight columns.  One warp does a panel's eight steps in registers (lane l rows l and l + 32, columns
+// rotating through the places so that the next one to search is always the first), where a step needs
+// no barrier and no shared memory: the pivot is a warp argmax on 64-bit keys, beside which every lane
+// computes the reciprocal of its own candidate, and row pv is shuffled out of its lane.  The panel's
+// result X holds the columns e_pv of the eight steps' product, so every other column then takes
+// C += X U, U = the panel's pivot rows, with those rows of C cleared first: 8 x 8 x 8 products on the FP64
+// tensor cores.  All eight warps update the next panel; the other columns are updated by six warps, one
+// block of eight columns each, while the next panel's steps run (the warp that would share the
+// scheduler of the panel's stays idle).
+// A full block takes 47.5 k cycles, 742 a step, against 75.7 k with every step over all 64 columns, where the
+// eight warps wait for row pv to pass through shared memory (300 cycles of a step) and for a barrier; panels
+// of four columns take 54.0 k.  One mixed solve of N = 2160: 5.25 -> 4.85 ms; one of N = 240: 0.43 -> 0.38 ms.
 // ---------------------------------------------------------------------------------------------
 constexpr int kDiagThreads = 256;
-constexpr int kDiagWarps = kDiagThreads / 32;
-static_assert(kDiagWarps * 8 == kNb && kNb == 64, "diagonal inverse layout: 8 columns per warp, 2 rows per lane");
+static_assert(kDiagThreads == 256 && kNb == 64, "diagonal inverse layout: 2 rows per lane, 8 panels, 8 row tiles");
 
-// PER_SM = blocks per SM the register budget allows: 1 (the update's chains unconstrained, for the
-// elimination that keeps one SM per job free for the inverses) or 2 (two per SM, for the
-// elimination with panel pivoting, which leaves fewer SMs to them).
+// 1 / d = conj(d) / |d|^2 (pivots of these blocks are far from the FP64 range limits); 0 for a zero.
+// 1 / |d|^2 by two Newton steps from the hardware's 20-bit approximation (2^-20, 2^-40, 2^-80 before
+// rounding), without the branches of a division, which kept the compiler from filling the chain's
+// latencies with the rest of the update (180 cycles a step).
+__device__ __forceinline__ double2 reciprocal(double2 d) {
+  const double q = d.x == 0.0 && d.y == 0.0 ? 1.0 : d.x * d.x + d.y * d.y;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(q));
+  r = fma(r, fma(-q, r, 1.0), r);
+  r = fma(r, fma(-q, r, 1.0), r);
+  return make_double2(d.x * r, -d.y * r);
+}
+
+// PER_SM = blocks per SM the register budget allows: 1 (for the elimination that keeps one SM per job
+// free for the inverses) or 2 (for the elimination with panel pivoting, which leaves fewer SMs to them).
 template <typename T, int PER_SM>
 __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(const JobDev *__restrict__ jobs, int k,
                                                                             int *info) {
-  constexpr int NB = kNb;
+  constexpr int NB = kNb, kStride = NB + 1, kMb = NB / 8;
   const JobDev &J = jobs[blockIdx.x];
   if (k >= J.n || J.inactive) return;
   const int kb = min(NB, J.n - k);
+  const int np = (kb + 7) / 8, kbp = 8 * np;  // panels; rows and columns kb .. kbp - 1 are the identity's
   extern __shared__ __align__(16) double2 dyn_smem[];
-  double2(*As)[NB + 1] = reinterpret_cast<double2(*)[NB + 1]>(dyn_smem);  // staging As[row][col]
-  __shared__ double2 s_g[2][NB];              // the step's row factors g, by step parity
-  __shared__ double2 s_row[kDiagWarps][8];    // per warp: u over the warp's columns
-  __shared__ int s_pvp[2];
+  double2(*As)[kStride] = reinterpret_cast<double2(*)[kStride]>(dyn_smem);  // As[column][row]
+  // Us[column][step]: 8 steps of a column in 192 bytes, so that a fragment's eight lanes (two columns,
+  // four steps) hit eight 16-byte banks
+  __shared__ double2 Us[NB][12];
   __shared__ int s_sing;
   __shared__ int s_pv[NB], s_inv[NB];
   T *__restrict__ Fk = static_cast<T *>(J.F) + (size_t)k + (size_t)k * J.ld;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   constexpr int kPer = NB * NB / kDiagThreads;  // entries per thread of a full block
-  if (kb == NB) {
+  {
     // all of a thread's loads in flight at once (a loop over them waits out one DRAM round trip
     // per entry)
     double2 v[kPer];
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const int e = tid + i * kDiagThreads;
-      v[i] = ldc(Fk + (e % NB) + (size_t)(e / NB) * J.ld);
+      const int e = tid + i * kDiagThreads, r = e % NB, c = e / NB;
+      v[i] = r < kb && c < kb ? ldc(Fk + r + (size_t)c * J.ld) : make_double2(r == c ? 1.0 : 0.0, 0.0);
     }
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       const int e = tid + i * kDiagThreads;
-      As[e % NB][e / NB] = v[i];
-    }
-  } else {
-    for (int e = tid; e < kb * kb; e += kDiagThreads) {
-      const int cc = e / kb, r = e - cc * kb;
-      As[r][cc] = ldc(Fk + r + (size_t)cc * J.ld);
+      As[e / NB][e % NB] = v[i];
     }
   }
-  if (tid < NB) s_inv[tid] = tid;  // every entry in range whatever the pivots
+  if (tid < NB) s_pv[tid] = s_inv[tid] = tid;  // every entry in range whatever the pivots
   if (tid == 0) s_sing = 0;
   __syncthreads();
-  const int w = tid >> 5, l = tid & 31;
-  double2 a[2][8];
+  bool used0 = l >= kbp, used1 = l + 32 >= kbp;  // rows already pivoted on (warp 0)
+  // C += X U for the 8 x 8 block (mb, nb) of A, X = the finished panel q
+  auto update = [&](int mb, int nb, int q) {
+    const int r = 8 * mb + (l >> 2);
+    double2 *c0 = &As[8 * nb + 2 * (l & 3)][r], *c1 = c0 + kStride;
+    double re[2], im[2];
+    re[0] = c0->x, im[0] = c0->y, re[1] = c1->x, im[1] = c1->y;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int r = l + 32 * i, c = 8 * w + j;
-      a[i][j] = (r < kb && c < kb) ? As[r][c] : make_double2(0.0, 0.0);
+    for (int ks = 0; ks < 2; ++ks) {
+      const double2 x = As[8 * q + 4 * ks + (l & 3)][r], u = Us[8 * nb + (l >> 2)][4 * ks + (l & 3)];
+      dm::mma_884(re[0], re[1], x.x, u.x);
+      dm::mma_884(im[0], im[1], x.x, u.y);
+      dm::mma_884(re[0], re[1], -x.y, u.y);
+      dm::mma_884(im[0], im[1], x.y, u.x);
     }
-  // rows already pivoted on (rows past kb count as used, so they are never chosen)
-  bool used0 = l >= kb, used1 = l + 32 >= kb;
-  // The pivot of column p, whose rows of this lane are x0 and x1, and step p's g, published.
-  auto search = [&](double2 x0, double2 x1, int p) {
-    // the unused row of largest |re| + |im|, as the largest 64-bit key
-    const unsigned long long k0 = used0 ? 0ull : pivot_key(cabs1(x0), l);
-    const unsigned long long k1 = used1 ? 0ull : pivot_key(cabs1(x1), l + 32);
-    const bool first = k0 > k1;
-    const unsigned long long kl = first ? k0 : k1;
-    // 1/d = conj(d) / |d|^2 of the lane's candidate (pivots of these blocks are far from the FP64
-    // range limits); 0 for a zero
-    const double2 xs = first ? x0 : x1;
-    const bool zero = xs.x == 0.0 && xs.y == 0.0;
-    const double rr = 1.0 / (zero ? 1.0 : xs.x * xs.x + xs.y * xs.y);
-    const double2 rl = make_double2(xs.x * rr, -xs.y * rr);
-    // kb - p unused rows remain, so the key names one of them (a row < kb)
-    const int pv = min(pivot_row(kl), kb - 1);
-    double2 dinv;
-    dinv.x = __shfl_sync(0xffffffffu, rl.x, pv & 31);
-    dinv.y = __shfl_sync(0xffffffffu, rl.y, pv & 31);
-    double2 *g = s_g[p & 1];
-    g[l] = (l == pv) ? make_double2(1.0 - dinv.x, -dinv.y) : cmul(x0, dinv);
-    g[l + 32] = (l + 32 == pv) ? make_double2(1.0 - dinv.x, -dinv.y) : cmul(x1, dinv);
-    if (l == 0) {
-      s_pvp[p & 1] = pv;
-      s_pv[p] = pv;
-      if (dinv.x == 0.0 && dinv.y == 0.0) s_sing = 1;
-    }
+    *c0 = make_double2(re[0], im[0]);
+    *c1 = make_double2(re[1], im[1]);
   };
-  if (w == 0) search(a[0][0], a[1][0], 0);
-  __syncthreads();
-#pragma unroll 1
-  for (int p = 0; p < kb; ++p) {
-    // place j holds column 8w + ((p + j) & 7)
-    const int pv = s_pvp[p & 1];
-    const double2 g0 = s_g[p & 1][l], g1 = s_g[p & 1][l + 32];
-    const int pl = pv & 31, pi = pv >> 5;
-    if (l == pl) {  // publish u over this warp's columns, then mark row pv used
+  for (int q = 0; q < np; ++q) {
+    if (w == 0) {
+      // the panel's eight steps; place j of a[.][] holds column 8q + ((p + j) & 7)
+      double2 a[2][8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        double2 v = pi ? a[1][j] : a[0][j];
-        if (j == 0 && w == (p >> 3)) v.x += 1.0;
-        s_row[w][j] = v;
+        a[0][j] = As[8 * q + j][l];
+        a[1][j] = As[8 * q + j][l + 32];
       }
-      if (pi) used1 = true;
-      else used0 = true;
-    }
-    __syncwarp();
-    const double2 u1 = s_row[w][1], o0 = a[0][0], o1 = a[1][0];
-    a[0][0] = cfnma(a[0][1], g0, u1);
-    a[1][0] = cfnma(a[1][1], g1, u1);
-    if (p + 1 < kb && w == ((p + 1) >> 3)) search(a[0][0], a[1][0], p + 1);
+      // the unused row of largest |re| + |im| of the next column, as the largest 64-bit key, and 1/d;
+      // beside the argmax every lane takes the reciprocal of its own candidate
+      int pv;
+      double2 dinv;
+      auto search = [&](double2 x0, double2 x1) {
+        const unsigned long long k0 = used0 ? 0ull : pivot_key(cabs1(x0), l);
+        const unsigned long long k1 = used1 ? 0ull : pivot_key(cabs1(x1), l + 32);
+        const bool first = k0 > k1;
+        const double2 rl = reciprocal(first ? x0 : x1);
+        pv = min(pivot_row(first ? k0 : k1), kbp - 1);  // (a row < kbp: some are unused)
+        dinv.x = __shfl_sync(0xffffffffu, rl.x, pv & 31);
+        dinv.y = __shfl_sync(0xffffffffu, rl.y, pv & 31);
+      };
+      search(a[0][0], a[1][0]);
+#pragma unroll 1
+      for (int p = 0; p < 8; ++p) {
+        const int pc = pv, pl = pv & 31;
+        const bool hi = pv >= 32, is0 = l == pv, is1 = l + 32 == pv;
+        const double2 di = dinv, h0 = cmul(a[0][0], di), h1 = cmul(a[1][0], di);
+        const double2 one = make_double2(1.0 - di.x, -di.y);
+        const double2 g0 = is0 ? one : h0, g1 = is1 ? one : h1;
+        used0 |= is0;
+        used1 |= is1;
+        {
+          const double2 v = hi ? a[1][1] : a[0][1];
+          double2 u;
+          u.x = __shfl_sync(0xffffffffu, v.x, pl);
+          u.y = __shfl_sync(0xffffffffu, v.y, pl);
+          a[0][0] = cfnma(a[0][1], g0, u);
+          a[1][0] = cfnma(a[1][1], g1, u);
+        }
+        search(a[0][0], a[1][0]);  // (after the last step: a finished column, not used)
 #pragma unroll
-    for (int j = 2; j < 8; ++j) {
-      const double2 u = s_row[w][j];
-      a[0][j - 1] = cfnma(a[0][j], g0, u);
-      a[1][j - 1] = cfnma(a[1][j], g1, u);
+        for (int j = 2; j < 8; ++j) {
+          const double2 v = hi ? a[1][j] : a[0][j];
+          double2 u;
+          u.x = __shfl_sync(0xffffffffu, v.x, pl);
+          u.y = __shfl_sync(0xffffffffu, v.y, pl);
+          a[0][j - 1] = cfnma(a[0][j], g0, u);
+          a[1][j - 1] = cfnma(a[1][j], g1, u);
+        }
+        a[0][7] = is0 ? di : make_double2(-h0.x, -h0.y);
+        a[1][7] = is1 ? di : make_double2(-h1.x, -h1.y);
+        if (l == 0) {
+          s_pv[8 * q + p] = pc;
+          s_inv[pc] = 8 * q + p;
+          if (di.x == 0.0 && di.y == 0.0) s_sing = 1;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        As[8 * q + j][l] = a[0][j];
+        As[8 * q + j][l + 32] = a[1][j];
+      }
+    } else if (q > 0 && (w & 3)) {
+      // meanwhile the step before, on the columns past the next panel: one block column a warp
+      int nb = (w & 3) - 1 + (w > 4 ? 3 : 0);  // 0 .. 5 over the blocks other than q - 1 and q
+      if (nb >= q - 1) nb += 2;
+      if (nb < np)
+#pragma unroll 2
+        for (int mb = 0; mb < kMb; ++mb) update(mb, nb, q - 1);
     }
-    const double2 u0 = s_row[w][0];
-    a[0][7] = cfnma(o0, g0, u0);
-    a[1][7] = cfnma(o1, g1, u0);
+    __syncthreads();
+    // U = the pivot rows, which A's update then builds from zero
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int e = tid + i * kDiagThreads, c = e >> 3, pr = s_pv[8 * q + (e & 7)];
+      if ((c >> 3) != q) {
+        Us[c][e & 7] = As[c][pr];
+        As[c][pr] = make_double2(0.0, 0.0);
+      }
+    }
+    __syncthreads();
+    if (q + 1 < np) update(w, q + 1, q);
+    else
+      for (int nb = 0; nb < np - 1; ++nb) update(w, nb, q);
     __syncthreads();
   }
-  __syncthreads();
-  if (tid < kb) s_inv[s_pv[tid]] = tid;
-  __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int r = l + 32 * i, c = 8 * w + ((j + kb) & 7);
-      if (r < kb && c < kb) As[s_inv[r]][s_pv[c]] = a[i][j];
-    }
-  __syncthreads();
-  if (kb == NB) {
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int e = tid + i * kDiagThreads;
-      stc(Fk + (e % NB) + (size_t)(e / NB) * J.ld, As[e % NB][e / NB]);
-    }
-  } else {
-    for (int e = tid; e < kb * kb; e += kDiagThreads) {
-      const int cc = e / kb, r = e - cc * kb;
-      stc(Fk + r + (size_t)cc * J.ld, As[r][cc]);
-    }
+  for (int i = 0; i < kPer; ++i) {
+    const int e = tid + i * kDiagThreads, r = e % NB, c = e / NB;
+    if (r < kb && c < kb) stc(Fk + r + (size_t)c * J.ld, As[s_inv[c]][s_pv[r]]);
   }
   if (s_sing && tid == 0) atomicCAS(&info[blockIdx.x], 0, k + 1);
 }
