@@ -242,10 +242,10 @@ void launch_diag_inverse(bool packed, const JobDev *jobs, int njobs, int k, int 
 // (re, im) pair: a complex multiply-add is two packed FMAs (fma.rn.f32x2, the same four products and
 // roundings as scalar FMAs), which leaves half the issue slots to the operand loads.  The whole
 // K <= 64 of both operands is requested by cp.async at once, in four K chunks of 16 that are
-// multiplied as they land, so a CTA waits out one memory round trip.  (31 jobs of N = 2160: the
-// elimination's small products 8.97 -> 8.29 ms in all, from scalar FMAs and a two-stage ring.)  Thread (tx, ty) owns rows
-// 2 tx, 2 tx + 1, 32 + 2 tx, 33 + 2 tx (16-byte shared-memory loads and stores) and columns
-// ty + 16 j.
+// multiplied as they land, so a CTA waits out one memory round trip.  (31 mixed jobs of
+// N = 2160: the elimination took 8.97 ms with scalar FMAs and a two-stage ring, 8.29 with these.)
+// Thread (tx, ty) owns rows 2 tx, 2 tx + 1, 32 + 2 tx, 33 + 2 tx (16-byte shared-memory loads and
+// stores) and columns ty + 16 j.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTile = 64;
 constexpr int kKc = 16;

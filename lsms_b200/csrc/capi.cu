@@ -492,7 +492,12 @@ int ensure_split(b200tau_ctx *ctx, int ld, int slots) {
   t.steps = ld / kNb + 1;
   t.a_slot = (size_t)2 * ld * kSplitDigits * kSplitRowBytes;
   t.b_slot = (size_t)ld * kSplitDigits * kSplitRowBytes;
-  CK(cudaMalloc(&ctx->d_split, split_slot_bytes(ld) * slots + sizeof(int) * kSplitCounters * t.steps));
+  if (cudaMalloc(&ctx->d_split, split_slot_bytes(ld) * slots + sizeof(int) * kSplitCounters * t.steps) != cudaSuccess) {
+    cudaGetLastError();  // no room: the updates stay on the FP64 tensor cores
+    ctx->d_split = nullptr;
+    ctx->split_ld = ctx->split_slots = 0;
+    return B200TAU_OK;
+  }
   t.a = reinterpret_cast<signed char *>(ctx->d_split);
   t.b = t.a + t.a_slot * slots;
   t.a_scale = reinterpret_cast<double *>(t.b + t.b_slot * slots);
@@ -520,12 +525,13 @@ int ensure_split(b200tau_ctx *ctx, int ld, int slots) {
   return B200TAU_OK;
 }
 
-// The digit planes for a wave of FP64 factors, or null where no update is large enough for them.
+// The digit planes for a wave of FP64 factors, or null where no update is large enough for them or they
+// find no room.
 int split_for(b200tau_ctx *ctx, FactorKind fk, int maxN, int ld, int nw, const SplitBufs **out) {
   *out = nullptr;
   if (fk != kFactorFP64 || !split_pays(maxN, maxN, nw)) return B200TAU_OK;
   const int rc = ensure_split(ctx, ld, std::max(nw, ctx->slots));
-  if (rc == B200TAU_OK) *out = &ctx->split;
+  if (rc == B200TAU_OK && ctx->d_split) *out = &ctx->split;
   return rc;
 }
 

