@@ -60,7 +60,8 @@ using namespace cx;
 // scheduler of the panel's stays idle).
 // A full block takes 47.5 k cycles, 742 a step, against 75.7 k with every step over all 64 columns, where the
 // eight warps wait for row pv to pass through shared memory (300 cycles of a step) and for a barrier; panels
-// of four columns take 54.0 k.  One mixed solve of N = 2160: 5.25 -> 4.85 ms; one of N = 240: 0.43 -> 0.38 ms.
+// of four columns take 54.0 k.  A launch takes 33 us (45 us).  One mixed solve
+// of N = 2160: 5.25 -> 4.85 ms; one of N = 240: 0.43 -> 0.38 ms.
 // ---------------------------------------------------------------------------------------------
 constexpr int kDiagThreads = 256;
 static_assert(kDiagThreads == 256 && kNb == 64, "diagonal inverse layout: 2 rows per lane, 8 panels, 8 row tiles");

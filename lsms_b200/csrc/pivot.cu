@@ -39,8 +39,9 @@
 namespace b200 {
 namespace {
 
-constexpr int kSelThreads = 1024;                  // (candidate, 16-column group) per thread
-constexpr int kGroups = kSelThreads / kPivCands;   // column groups of the panel
+constexpr int kSelThreads = 512;                   // two candidates, one 16-column group per thread
+constexpr int kHalf = kPivCands / 2;               // a thread's candidates are r and r + kHalf
+constexpr int kGroups = kSelThreads / kHalf;       // column groups of the panel
 constexpr int kGroupCols = kNb / kGroups;          // 16
 static_assert(kGroups * kGroupCols == kNb, "selection thread layout");
 
@@ -78,16 +79,16 @@ __device__ __forceinline__ int block_scan(int v, int *s_warp, int &excl) {
   if (lane == 31) s_warp[warp] = x;
   __syncthreads();
   if (warp == 0) {
-    int w = s_warp[lane];
+    int w = lane < kSelThreads / 32 ? s_warp[lane] : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, w, o);
       if (lane >= o) w += y;
     }
-    s_warp[lane] = w;  // inclusive over warps
+    if (lane < kSelThreads / 32) s_warp[lane] = w;  // inclusive over warps
   }
   __syncthreads();
-  const int total = s_warp[31];
+  const int total = s_warp[kSelThreads / 32 - 1];
   excl = (warp > 0 ? s_warp[warp - 1] : 0) + x - v;
   __syncthreads();  // s_warp is reused by the next scan
   return total;
@@ -104,13 +105,16 @@ __global__ void __launch_bounds__(kSelThreads) panel_select_kernel(const JobDev 
   int *__restrict__ piv = J.piv;
   const unsigned *__restrict__ mags = reinterpret_cast<const unsigned *>(piv + pivot_mags_offset(ld));
   __shared__ float2 s_col[2][kPivCands];  // the step's column, by step parity
-  __shared__ float2 s_row[kNb];           // the pivot row's columns, in the threads' places
-  __shared__ unsigned long long s_best[2][kPivCands / 32];
-  __shared__ int s_dst[2 * kNb], s_src[2 * kNb], s_cnt;
+  __shared__ __align__(16) float2 s_row[kNb];  // the pivot row's columns, in the threads' places
+  __shared__ unsigned long long s_best[2][kHalf / 32];
+  __shared__ int s_dst[2 * kNb], s_src[2 * kNb];
+  __shared__ int s_vac[kNb];
+  __shared__ unsigned s_in[2], s_moved[2], s_below[2];
+  __shared__ int s_ok;
   __shared__ int s_cand[kPivCands];
   __shared__ int s_out[kNb];
   __shared__ int s_hist[256];
-  __shared__ int s_warp[32];
+  __shared__ int s_warp[kSelThreads / 32];
   __shared__ unsigned s_prefix;
   __shared__ int s_remain;
   const int tid = threadIdx.x;
@@ -133,14 +137,22 @@ __global__ void __launch_bounds__(kSelThreads) panel_select_kernel(const JobDev 
         if ((key & mask) == prefix) atomicAdd(&s_hist[(key >> shift) & 255u], 1);
       }
       __syncthreads();
-      if (tid == 0) {
-        int cum = 0, d = 0;
-        for (d = 255; d > 0; --d) {
-          if (cum + s_hist[d] >= remain) break;
-          cum += s_hist[d];
+      if (tid < 32) {  // the digit of the remain-th largest key: lane l has bins 255 - 8 l down
+        int sum = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += s_hist[255 - 8 * tid - i];
+        int x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, x, o);
+          if (tid >= o) x += y;
         }
-        s_prefix = prefix | ((unsigned)d << shift);
-        s_remain = remain - cum;
+        if (x >= remain && x - sum < remain) {  // (one lane: at least `remain` keys match the prefix)
+          int cum = x - sum, d = 255 - 8 * tid;
+          for (; d > 0 && cum + s_hist[d] < remain; --d) cum += s_hist[d];
+          s_prefix = prefix | ((unsigned)d << shift);
+          s_remain = remain - cum;
+        }
       }
       __syncthreads();
       prefix = s_prefix;
@@ -179,94 +191,135 @@ __global__ void __launch_bounds__(kSelThreads) panel_select_kernel(const JobDev 
     __syncthreads();
   } else {
     const T *__restrict__ F = static_cast<const T *>(J.F);
-    // Thread (candidate r, column group g) holds its 16 columns in registers.  A step writes the columns
-    // of the group that holds the step's column one place down, so that group's column to rank is
-    // always in place 0; the others stay put.  (A launch takes 128 us; 173 us with the rows in shared
-    // memory and one thread finding the row moves.)
-    const int r = tid & (kPivCands - 1), g = tid / kPivCands, c0 = g * kGroupCols;
-    const int cand = r < R ? s_cand[r] : -1;
-    float2 a[kGroupCols];
+    // Thread (candidates r and r + kHalf, column group g) holds its 2 x 16 elements in registers.  What bounds
+    // a step is the shared-memory reads of the pivot row, the same 128 bytes for every row of a group,
+    // so a thread has two rows for them (a launch takes 100 us; 124 us with one row to each of 1024 threads, and
+    // the moves and the radix digits found by one thread).  A step writes the columns of the group that
+    // holds the step's column one place down, so that group's column to rank is always in place 0; the
+    // others stay put.
+    const int r = tid & (kHalf - 1), g = tid / kHalf, c0 = g * kGroupCols;
+    int cand[2];
+    float2 a[2][kGroupCols];
 #pragma unroll
-    for (int j = 0; j < kGroupCols; ++j)
-      a[j] = (cand >= 0 && c0 + j < kb) ? to_f2(F[(size_t)cand + (size_t)(k + c0 + j) * ld]) : make_float2(0.f, 0.f);
-    bool taken = false;
+    for (int h = 0; h < 2; ++h) {
+      cand[h] = r + h * kHalf < R ? s_cand[r + h * kHalf] : -1;
+#pragma unroll
+      for (int j = 0; j < kGroupCols; ++j)
+        a[h][j] = (cand[h] >= 0 && c0 + j < kb) ? to_f2(F[(size_t)cand[h] + (size_t)(k + c0 + j) * ld])
+                                                : make_float2(0.f, 0.f);
+    }
+    bool taken[2] = {false, false};
     for (int p = 0; p < kb; ++p) {
       const int par = p & 1;
       const bool mine = g == p / kGroupCols;  // (uniform over a warp)
       if (mine) {  // rank the rows: the largest |re| + |im| (its bits order as integers), ties low
-        float v = cabs1f(a[0]);
-        if (!(v == v)) v = 0.f;  // a NaN ranks as zero, so a row in range is still chosen
-        const bool on = cand >= 0 && !taken;
-        const unsigned hi = on ? __float_as_uint(v) + 1u : 0u;
+        unsigned key[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float v = cabs1f(a[h][0]);
+          if (!(v == v)) v = 0.f;  // a NaN ranks as zero, so a row in range is still chosen
+          key[h] = cand[h] >= 0 && !taken[h] ? __float_as_uint(v) + 1u : 0u;
+          s_col[par][r + h * kHalf] = a[h][0];
+        }
+        const unsigned hi = max(key[0], key[1]), row = key[0] >= key[1] ? r : r + kHalf;
         const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-        const unsigned lo = __reduce_max_sync(0xffffffffu, hi == mhi ? (unsigned)(kPivCands - 1 - r) : 0u);
+        const unsigned lo = __reduce_max_sync(0xffffffffu, hi == mhi ? kPivCands - 1 - row : 0u);
         if ((tid & 31) == 0) s_best[par][r >> 5] = ((unsigned long long)mhi << 32) | lo;
-        s_col[par][r] = a[0];
       }
       __syncthreads();
       unsigned long long best = s_best[par][0];
 #pragma unroll
-      for (int w = 1; w < kPivCands / 32; ++w) best = s_best[par][w] > best ? s_best[par][w] : best;
+      for (int w = 1; w < kHalf / 32; ++w) best = s_best[par][w] > best ? s_best[par][w] : best;
       // R > kb > p candidates remain untaken, each ranked above the taken ones: bi is one of them
       const int bi = kPivCands - 1 - (int)(unsigned)best;
-      if (r == bi) {
-        taken = true;
+      const float2 d = s_col[par][bi];
+      const float dd = d.x * d.x + d.y * d.y;
+      float2 f[2];
 #pragma unroll
-        for (int j = 0; j < kGroupCols; ++j) s_row[c0 + j] = a[j];
+      for (int h = 0; h < 2; ++h) {
+        if (r + h * kHalf == bi) {
+          taken[h] = true;
+#pragma unroll
+          for (int j = 0; j < kGroupCols; j += 2)
+            *reinterpret_cast<float4 *>(&s_row[c0 + j]) =
+                make_float4(a[h][j].x, a[h][j].y, a[h][j + 1].x, a[h][j + 1].y);
+        }
+        const float2 x0 = s_col[par][r + h * kHalf];
+        f[h] = make_float2(0.f, 0.f);
+        if (dd > 0.f && !taken[h])
+          f[h] = make_float2((x0.x * d.x + x0.y * d.y) / dd, (x0.y * d.x - x0.x * d.y) / dd);
       }
       if (tid == 0) s_out[p] = s_cand[bi];
-      const float2 d = s_col[par][bi], x0 = s_col[par][r];
-      const float dd = d.x * d.x + d.y * d.y;
-      float2 f = make_float2(0.f, 0.f);
-      if (dd > 0.f && !taken) f = make_float2((x0.x * d.x + x0.y * d.y) / dd, (x0.y * d.x - x0.x * d.y) / dd);
       __syncthreads();
-      auto sub = [&](float2 x, float2 pj) {
-        x.x -= f.x * pj.x - f.y * pj.y;
-        x.y -= f.x * pj.y + f.y * pj.x;
+      auto sub = [&](int h, float2 x, float2 pj) {
+        x.x -= f[h].x * pj.x - f[h].y * pj.y;
+        x.y -= f[h].x * pj.y + f[h].y * pj.x;
         return x;
       };
-      if (mine) {
+      if (mine || p < c0) {
 #pragma unroll
-        for (int j = 1; j < kGroupCols; ++j) a[j - 1] = sub(a[j], s_row[c0 + j]);
-        a[kGroupCols - 1] = make_float2(0.f, 0.f);  // (the step's own column is not needed again)
-      } else if (p < c0) {
+        for (int j = 0; j < kGroupCols; j += 2) {
+          const float4 q = *reinterpret_cast<const float4 *>(&s_row[c0 + j]);
+          const float2 q0 = make_float2(q.x, q.y), q1 = make_float2(q.z, q.w);
 #pragma unroll
-        for (int j = 0; j < kGroupCols; ++j) a[j] = sub(a[j], s_row[c0 + j]);
+          for (int h = 0; h < 2; ++h) {
+            const float2 v0 = sub(h, a[h][j], q0), v1 = sub(h, a[h][j + 1], q1);
+            if (mine) {
+              if (j > 0) a[h][j - 1] = v0;
+              a[h][j] = v1;
+            } else {
+              a[h][j] = v0;
+              a[h][j + 1] = v1;
+            }
+          }
+        }
+        if (mine) a[0][kGroupCols - 1] = a[1][kGroupCols - 1] = make_float2(0.f, 0.f);  // (not needed again)
       }
     }
     __syncthreads();
   }
   // the moves that bring the pivot rows to k..k+kb-1 (pivot order) and the displaced rows to the
-  // vacated positions; a permutation of at most 2 kb positions, also applied to perm
-  if (tid == 0) {
+  // vacated positions, the q-th displaced row to the q-th vacated position in pivot order; a permutation of
+  // at most 2 kb positions, also applied to perm.  Thread i < 64: step i and position k + i.
+  if (tid == 0) s_ok = 1;
+  if (tid < 2) s_in[tid] = 0u;
+  __syncthreads();
+  const int out = tid < kb ? s_out[tid] : k + tid;
+  if (tid < kNb) {
     // kb distinct rows in [k, n) by construction; anything else leaves the rows in place
-    bool ok = true;
-    unsigned long long in_s = 0ull;
-    for (int p = 0; p < kb; ++p) {
-      ok = ok && s_out[p] >= k && s_out[p] < n;
-      if (s_out[p] - k < kb) in_s |= 1ull << (s_out[p] - k);
+    if (tid < kb && (out < k || out >= n)) s_ok = 0;
+    if (tid < kb && out >= k && out - k < kb) atomicOr(&s_in[(out - k) >> 5], 1u << ((out - k) & 31));
+    const unsigned mv = __ballot_sync(0xffffffffu, tid < kb && out != k + tid);
+    const unsigned vac = __ballot_sync(0xffffffffu, tid < kb && out >= k + kb);
+    if ((tid & 31) == 0) {
+      s_moved[tid >> 5] = mv;
+      s_below[tid >> 5] = vac;
     }
-    int cnt = 0;
-    for (int i = 0; i < kb; ++i)
-      if (s_out[i] != k + i) {
-        s_dst[cnt] = k + i;
-        s_src[cnt] = s_out[i];
-        ++cnt;
-      }
-    int vj = 0;
-    for (int i = 0; i < kb; ++i)
-      if (!((in_s >> i) & 1ull)) {
-        while (vj < kb && s_out[vj] < k + kb) ++vj;  // the next vacated position, in pivot order
-        if (vj == kb) break;  // (as many vacated positions as displaced rows: not reached)
-        s_dst[cnt] = s_out[vj];
-        s_src[cnt] = k + i;
-        ++cnt;
-        ++vj;
-      }
-    s_cnt = ok ? cnt : 0;
   }
   __syncthreads();
-  const int cnt = s_cnt;
+  const unsigned long long moved = (unsigned long long)s_moved[1] << 32 | s_moved[0];
+  const unsigned long long vacated = (unsigned long long)s_below[1] << 32 | s_below[0];
+  const unsigned long long stay = (unsigned long long)s_in[1] << 32 | s_in[0];
+  const unsigned long long lower = tid < kNb ? (1ull << tid) - 1 : 0ull;
+  const int nmv = __popcll(moved), nvac = __popcll(vacated);
+  if (tid < kb) {
+    if (moved >> tid & 1) {
+      const int i = __popcll(moved & lower);
+      s_dst[i] = k + tid;
+      s_src[i] = out;
+    }
+    if (vacated >> tid & 1) s_vac[__popcll(vacated & lower)] = out;
+  }
+  __syncthreads();
+  if (tid < kb && !(stay >> tid & 1)) {
+    const int i = __popcll(~stay & lower);
+    if (i < nvac) {  // (as many vacated positions as displaced rows)
+      s_dst[nmv + i] = s_vac[i];
+      s_src[nmv + i] = k + tid;
+    }
+  }
+  __syncthreads();
+  const int cnt = s_ok ? nmv + nvac : 0;
   int *mv = piv + pivot_moves_offset(ld);
   if (tid == 0) mv[0] = cnt;
   int old = 0;
