@@ -217,7 +217,7 @@ constexpr size_t split_slot_bytes(int ld) {
 }
 // The integer tensor cores take an FP64 update of at least kSplitMin rows and columns and kSplitElems
 // elements of C over the wave: the packs and the fill of the pipeline cost some 35 us a launch, which the
-// faster products (30 against 50 to 60 TF/s) save from about 5 M elements on (a 64-column step; 31 jobs:
+// faster products (30 against 47 TF/s) save from about 5 M elements on (a 64-column step; 31 jobs:
 // 400 x 400; one job of N = 2160 stays on the FP64 tensor cores).
 constexpr int kSplitMin = 256;
 constexpr long kSplitElems = 5L << 20;
