@@ -1186,8 +1186,11 @@ cudaError_t sweep_solve(const JobDev *jobs, int njobs, int b, int max_N, int mod
 // host re-solves such jobs, and those not converged after the last round, by FP64 block LU.  The error left
 // after applying the correction is about c times the contraction factor of the refinement,
 // estimated as c / c_prev from the previous round; the job is converged when c * min(1, c / c_prev)
-// is below tol, and later rounds skip it.
-__global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__restrict__ jobs, double tol) {
+// is below tol, and later rounds skip it.  Accelerated rounds take a tol below kRefineTol, which a job may
+// meet its rounding floor before it reaches: a job whose estimate was once below kRefineTol (*cnorm is then
+// -c) counts as converged where its correction stops shrinking, or at the last round.
+__global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__restrict__ jobs, double tol, double grow,
+                                                             bool last) {
   const JobDev &J = jobs[blockIdx.x];
   if (J.conv == nullptr || converged(J) || J.inactive) return;
   const int b = J.b, n = J.n, ld = J.ld;
@@ -1211,11 +1214,12 @@ __global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__res
   }
   if (threadIdx.x == 0) {
     const double c = sx[0] > 0.0 ? sy[0] / sx[0] : 0.0;
-    const double prev = J.cnorm ? *J.cnorm : 0.0;
+    const double before = J.cnorm ? *J.cnorm : 0.0, prev = fabs(before);
     const double est = prev > 0.0 ? c * fmin(1.0, c / prev) : c;
-    if (est <= tol) *J.conv = kConverged;
-    else if (prev > 0.0 && c >= prev) *J.conv = kDiverged;  // no contraction: stop refining
-    if (J.cnorm) *J.cnorm = c;
+    const bool good = before < 0.0 || est <= kRefineTol, stalled = prev > 0.0 && c >= prev;
+    if (est <= tol || (good && (stalled || last))) *J.conv = kConverged;
+    else if (stalled && c >= grow * prev) *J.conv = kDiverged;  // no contraction: stop refining
+    if (J.cnorm) *J.cnorm = good ? -c : c;
   }
 }
 
@@ -1233,6 +1237,7 @@ __global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__res
 // results are as close to 64 bits as those of plain refinement (5e-13 to 1.5e-12 over whole batches).
 // hist: 0 the iterate X_i; 1, 2 P of odd and even rounds; 3, 4 Y of odd and even rounds.
 constexpr double kAccTol = 0.2;     // of kRefineTol
+constexpr double kAccGrow = 4.0;    // corrections of accelerated rounds do not shrink monotonically
 constexpr int kAccThreads = 1024;
 __global__ void __launch_bounds__(kAccThreads) accelerate_kernel(const JobDev *__restrict__ jobs, int round) {
   const JobDev &J = jobs[blockIdx.y];
@@ -1442,7 +1447,7 @@ cudaError_t launch_accelerate(const JobDev *jobs, int njobs, int b, int round, c
 
 cudaError_t launch_refine_round(FactorKind fk, const JobDev *jobs, int njobs, int max_n, int max_N, int b,
                                 bool check, int *info, cudaStream_t s, long *launches, bool fp32_sweep,
-                                const CUtensorMap *fmap, int active_hint, int *active, int accelerate) {
+                                const CUtensorMap *fmap, int active_hint, int *active, int accelerate, bool last) {
   (void)max_n;
   const cudaError_t e0 = b <= 16 ? launch_residual<16>(jobs, njobs, max_N, active, s)
                                  : launch_residual<32>(jobs, njobs, max_N, active, s);
@@ -1457,7 +1462,8 @@ cudaError_t launch_refine_round(FactorKind fk, const JobDev *jobs, int njobs, in
     if (ea != cudaSuccess) return ea;
   }
   if (check) {
-    converge_check_kernel<<<njobs, 256, 0, s>>>(jobs, accelerate > 0 ? kAccTol * kRefineTol : kRefineTol);
+    const bool acc = accelerate > 0;
+    converge_check_kernel<<<njobs, 256, 0, s>>>(jobs, acc ? kAccTol * kRefineTol : kRefineTol, acc ? kAccGrow : 1.0, last);
     if (launches) *launches += 1;
   }
   return cudaGetLastError();

@@ -764,7 +764,7 @@ int run_refinement(b200tau_ctx *ctx, const std::vector<JobDev> &h, int nw, int m
   for (int it = 0; it < p.steps; ++it) {
     const int hint = it >= kHintAfterRounds ? ctx->active_hint : 0;
     CK(launch_refine_round(p.fk, ctx->d_jobs, nw, maxn, maxN, b, true, ctx->d_info, ctx->stream, &ctx->launches,
-                           fp32_sweep, fmap, hint, ctx->d_active, accelerate ? it + 1 : 0));
+                           fp32_sweep, fmap, hint, ctx->d_active, accelerate ? it + 1 : 0, it + 1 == p.steps));
     if (it + 1 == kHintAfterRounds && p.steps > kHintAfterRounds && !ctx->hint_pending) {
       if (ctx->h_hint_cap < nw) {  // (no copy into the old buffer is pending)
         if (ctx->h_hint) cudaFreeHost(ctx->h_hint);
@@ -873,7 +873,7 @@ int wave_graph(b200tau_ctx *ctx, int nw, int maxL, int maxn, int maxN, int ld, c
       for (int it = 0; it < p.steps && e == cudaSuccess; ++it) {
         e = launch_refine_round(p.fk, ctx->d_jobs, nw, maxn, maxN, ctx->b, true, ctx->d_info, cs, &n, fp32_sweep,
                                 fmap, it >= kHintAfterRounds ? std::max(1, (nw + 3) / 4) : 0, ctx->d_active,
-                                accelerate ? it + 1 : 0);
+                                accelerate ? it + 1 : 0, it + 1 == p.steps);
       }
       if (e == cudaSuccess) e = launch_refine_end(ctx->d_jobs, nw, ctx->ns, ctx->kkrsz, cs, &n);
     } else if (e == cudaSuccess) {

@@ -307,9 +307,10 @@ cudaError_t launch_refine_begin(FactorKind fk, const JobDev *jobs, int njobs, in
 cudaError_t launch_refine_round(FactorKind fk, const JobDev *jobs, int njobs, int max_n, int max_N, int b,
                                 bool check, int *info, cudaStream_t s, long *launches, bool fp32_sweep = false,
                                 const CUtensorMap *fmap = nullptr, int active_hint = 0, int *active = nullptr,
-                                int accelerate = 0);
+                                int accelerate = 0, bool last = false);
 // The accelerated step of a round (MIXED records with history): round 0 is the initial solve.  Rounds
-// take it by launch_refine_round's `accelerate` (the round's number from 1, or 0 for a plain round).
+// take it by launch_refine_round's `accelerate` (the round's number from 1, or 0 for a plain round); `last`: no
+// round follows.
 cudaError_t launch_accelerate(const JobDev *jobs, int njobs, int b, int round, cudaStream_t s, long *launches);
 cudaError_t launch_refine_end(const JobDev *jobs, int njobs, int ns, int kkrsz, cudaStream_t s, long *launches);
 // One block sweep of the correction solve for all jobs, one thread-block cluster per job
