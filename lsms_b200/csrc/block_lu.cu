@@ -895,7 +895,7 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
     // row k2 only after its row moves, so that at the moves every row below step k still owes
     // step k's update right of block column k2 (done for all of them by the combined pass) and
     // the moves carry A21_k's rows with them.
-    if (panel && la.pair_min_rest > 0 && k2 < la.min_n && k2 + kNb < max_n &&
+    if (panel && la.pair_min_rest > 0 && k2 + kNb <= la.min_n && k2 + kNb < max_n &&
         max_N - k2 - kNb >= la.pair_min_rest) {
       const int tiles2 = (max_N - k2 - 1 + kTile - 1) / kTile;
       const int split2 = k2 + kNb + kTcTileCols;
@@ -947,7 +947,9 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
       k = k2;  // the loop's increment moves past k2
       continue;
     }
-    if (!panel && la.pair_min_rest > 0 && k2 < la.min_n && k2 + kNb < max_n &&
+    // (only where step k2 is a full block of every job: in a wave of 1392 and 2160 a pair whose second step
+    // was the smaller jobs' last, partial one left their factors too poor to refine)
+    if (!panel && la.pair_min_rest > 0 && k2 + kNb <= la.min_n && k2 + kNb < max_n &&
         max_N - k2 - kNb >= la.pair_min_rest) {
       const int tiles2 = (max_N - k2 - 1 + kTile - 1) / kTile;
       const bool next2 = k2 + kNb < max_n;

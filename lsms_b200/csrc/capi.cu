@@ -592,7 +592,7 @@ double trailing_flops(const std::vector<JobDev> &h, const Lookahead &la, int max
     for (int k = 0; k < J.n; k += kNb) {
       const int k2 = k + kNb;
       const double kb = std::min(kNb, J.n - k);
-      if (la.pair_min_rest > 0 && k2 < la.min_n && k2 + kNb < max_n && max_N - k2 - kNb >= la.pair_min_rest) {
+      if (la.pair_min_rest > 0 && k2 + kNb <= la.min_n && k2 + kNb < max_n && max_N - k2 - kNb >= la.pair_min_rest) {
         const double kb2 = std::min(kNb, J.n - k2);
         const double rest2 = J.N - k2 - kb2;
         f += 8.0 * rest2 * rest2 * (kb + kb2);
