@@ -522,10 +522,10 @@ __global__ void __launch_bounds__(dm::kThreads, 2) zgemm64_w_kernel(const JobDev
 // without look-ahead).
 template <int W>
 __global__ void __launch_bounds__(dm::kThreads, 4) zgemm64_update_kernel(const JobDev *__restrict__ jobs, int k, int tx,
-                                                                         int ty, int nj, int part, int len) {
+                                                                         int ty, int nj, int part, int len, bool sparse) {
   extern __shared__ __align__(16) double2 zsm64[];
   using TL = dm::Tile<W, W>;
-  if (gridDim.z == (unsigned)nj) {
+  if (!sparse) {  // grid (tx, ty, nj)
     const JobDev &J = jobs[blockIdx.z];
     const int bx = blockIdx.x;
     int by = blockIdx.y * len, l = len;
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(dm::kThreads, 4) zgemm64_update_kernel(const J
     update64_column<W>(J, k, bx, by, l, zsm64);
     return;
   }
-  // a 1-D grid smaller than the tiles (the FP64 re-solve of a mixed wave, where most jobs are
+  // sparse: a 1-D grid, smaller than the tiles (the FP64 re-solve of a mixed wave, where most jobs are
   // inactive and a full grid would spend its time launching CTAs that exit at once): jobs one
   // after another (an inactive job costs one check), its columns spread over the CTAs
   for (int z = 0; z < nj; ++z) {
@@ -1095,7 +1095,7 @@ void launch_update64_tiles(const JobDev *jobs, int njobs, int k, int max_N, int 
   const int len = sparse ? 1 : dm::column_tiles((long)tx * tr * njobs);
   const int ty = (tr + len - 1) / len;
   const dim3 grid = sparse ? dim3(std::min(tx * ty * njobs, kSparseGrid)) : dim3(tx, ty, njobs);
-  zgemm64_update_kernel<W><<<grid, dm::kThreads, TL::kSmem, s>>>(jobs, k, tx, ty, njobs, part, len);
+  zgemm64_update_kernel<W><<<grid, dm::kThreads, TL::kSmem, s>>>(jobs, k, tx, ty, njobs, part, len, sparse);
 }
 
 void launch_update64(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, cudaStream_t s) {

@@ -201,3 +201,27 @@ def test_updates_by_digit_products(solver_factory, n_reduced):
             want = -np.linalg.solve(t, inv[off[j]:off[j + 1], off[j]:off[j + 1]] - np.eye(k)).T
             err = [max(e, np.abs(d[j][:k, :k] - want).max()) for e, d in zip(err, (ld[i], ld1[0]))]
         assert err[0] <= 8 * err[1] + 10 * bound * np.abs(ld1[0]).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lattice,shells,njobs", [("bcc", 2, 1), ("fcc", 3, 1), ("fcc", 7, 1), ("fcc", 7, 2), ("bcc", 2, 65)])
+def test_fp64_resolve_job_counts(solver_factory, lattice, shells, njobs):
+    """One round converges no job, so every one is re-solved by FP64 block LU, whose update kernel takes
+    the wave's tiles on a small looping grid: a wave of one job (alone, or the last one of 65), and of two."""
+    from oracle import port
+    a = {"bcc": 5.42, "fcc": 6.82}[lattice]
+    prob = W.make_problem(lattice, a, shells, 3, W.semicircle_contour(-0.3, 0.7, njobs) if njobs > 1 else [0.35 + 0.15j],
+                          31, n_species=2)
+    s = solver_factory(3, 1, 1)
+    s.load_problem(prob)
+    jobs = T.make_jobs([(0, i, 0, e) for i, e in enumerate(prob.energies)])
+    want = s.solve_jobs(jobs, T.PREC_FP64)
+    s.set_refinement(T.PREC_MIXED, 1)
+    try:
+        got = s.solve_jobs(jobs, T.PREC_MIXED)
+        assert s.last_fallback_count == njobs
+    finally:
+        s.set_refinement(T.PREC_MIXED, 10)
+    for i in range(njobs):
+        t0 = -port.tau00_l(prob, np.zeros((16, 16), np.complex128), i)
+        assert np.abs(got[i] - want[i]).max() <= 1e-12 * np.abs(want[i] + t0).max()
