@@ -31,6 +31,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
     srcs = [os.path.join(CSRC, s) for s in SOURCES]
     deps = srcs + [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "cplx.cuh"), os.path.join(CSRC, "gj.cuh"),
                    os.path.join(CSRC, "dmma.cuh"), os.path.join(CSRC, "split8.cuh"), os.path.join(CSRC, "cluster.cuh"), os.path.join(CSRC, "umma.cuh"),
+                   os.path.join(CSRC, "refine_rule.h"),
                    os.path.join(HERE, "..", "include", "b200tau.h")]
     if (not force and os.path.exists(LIB_PATH)
             and all(os.path.getmtime(LIB_PATH) >= os.path.getmtime(d) for d in deps)):

@@ -1183,15 +1183,10 @@ cudaError_t sweep_solve(const JobDev *jobs, int njobs, int b, int max_N, int mod
   return cudaSuccess;
 }
 
-// After a refinement round: c = max|correction| / max|tau00| on the tau00 block.  A job whose
-// correction stops shrinking (c >= c_prev) is marked kDiverged and skipped from then on; the
-// host re-solves such jobs, and those not converged after the last round, by FP64 block LU.  The error left
-// after applying the correction is about c times the contraction factor of the refinement,
-// estimated as c / c_prev from the previous round; the job is converged when c * min(1, c / c_prev)
-// is below tol, and later rounds skip it.  Accelerated rounds take a tol below kRefineTol, which a job may
-// meet its rounding floor before it reaches: a job whose estimate was once below kRefineTol (*cnorm is then
-// -c) counts as converged where its correction stops shrinking, or at the last round.
-__global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__restrict__ jobs, double tol, double grow,
+// After a refinement round: c = max|correction| / max|tau00| on the tau00 block, and what refine_state
+// (refine_rule.h) makes of it and the two corrections before it.  A job that is kConverged or kDiverged is
+// skipped from then on; every job that is not kConverged after the last round is re-solved by FP64 block LU.
+__global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__restrict__ jobs, bool accelerated,
                                                              bool last) {
   const JobDev &J = jobs[blockIdx.x];
   if (J.conv == nullptr || converged(J) || J.inactive) return;
@@ -1216,12 +1211,12 @@ __global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__res
   }
   if (threadIdx.x == 0) {
     const double c = sx[0] > 0.0 ? sy[0] / sx[0] : 0.0;
-    const double before = J.cnorm ? *J.cnorm : 0.0, prev = fabs(before);
-    const double est = prev > 0.0 ? c * fmin(1.0, c / prev) : c;
-    const bool good = before < 0.0 || est <= kRefineTol, stalled = prev > 0.0 && c >= prev;
-    if (est <= tol || (good && (stalled || last))) *J.conv = kConverged;
-    else if (stalled && c >= grow * prev) *J.conv = kDiverged;  // no contraction: stop refining
-    if (J.cnorm) *J.cnorm = good ? -c : c;
+    const double prev = J.cnorm ? J.cnorm[0] : 0.0, prev2 = J.cnorm ? J.cnorm[1] : 0.0;
+    *J.conv = refine_state(c, prev, prev2, accelerated, last);
+    if (J.cnorm) {
+      J.cnorm[0] = c;
+      J.cnorm[1] = prev;
+    }
   }
 }
 
@@ -1234,12 +1229,9 @@ __global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__res
 // taken out instead of shrunk.  Rounds are a chain of two sweeps each, whose time hardly falls with the
 // jobs left: 256 jobs of N = 688 to 2160, one point next to the real axis, 31.0 -> 21.5 ms of refinement
 // (and no FP64 re-solve where there was one); 16 jobs of N = 4320, 32.5 -> 30.7 ms.  A round's step is
-// accelerated before the convergence check, and checked against a fifth of the plain rounds' tolerance: the
-// contraction between two accelerated rounds says less about the error that is left, and with this the
-// results are as close to 64 bits as those of plain refinement (5e-13 to 1.5e-12 over whole batches).
+// accelerated before the convergence check, which takes a fifth of the plain rounds' tolerance and the larger
+// of the last two contractions (refine_rule.h).
 // hist: 0 the iterate X_i; 1, 2 P of odd and even rounds; 3, 4 Y of odd and even rounds.
-constexpr double kAccTol = 0.2;     // of kRefineTol
-constexpr double kAccGrow = 4.0;    // corrections of accelerated rounds do not shrink monotonically
 constexpr int kAccThreads = 1024;
 __global__ void __launch_bounds__(kAccThreads) accelerate_kernel(const JobDev *__restrict__ jobs, int round) {
   const JobDev &J = jobs[blockIdx.y];
@@ -1464,8 +1456,7 @@ cudaError_t launch_refine_round(FactorKind fk, const JobDev *jobs, int njobs, in
     if (ea != cudaSuccess) return ea;
   }
   if (check) {
-    const bool acc = accelerate > 0;
-    converge_check_kernel<<<njobs, 256, 0, s>>>(jobs, acc ? kAccTol * kRefineTol : kRefineTol, acc ? kAccGrow : 1.0, last);
+    converge_check_kernel<<<njobs, 256, 0, s>>>(jobs, accelerate > 0, last);
     if (launches) *launches += 1;
   }
   return cudaGetLastError();

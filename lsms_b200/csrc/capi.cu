@@ -96,7 +96,7 @@ struct b200tau_ctx {
   int *d_info = nullptr;   // 2 x slots: the wave's jobs, then their FP64 re-solve records
   int *d_conv = nullptr;   // per slot: refinement converged
   int *d_active = nullptr;  // slots + 1: the jobs still refining (residual launches)
-  double *d_cnorm = nullptr;  // per slot: relative size of the last refinement correction
+  double *d_cnorm = nullptr;  // per slot: relative sizes of the last two refinement corrections
   int *d_err = nullptr;    // device error flags
   double2 *d_out = nullptr;
   size_t out_cap = 0;
@@ -275,7 +275,7 @@ int ensure_workspace(b200tau_ctx *ctx, int ld, int slots, const Plan &p) {
   CK(cudaMalloc(&ctx->d_info, sizeof(int) * 2 * sl));
   CK(cudaMalloc(&ctx->d_conv, sizeof(int) * sl));
   CK(cudaMalloc(&ctx->d_active, sizeof(int) * (sl + 1)));
-  CK(cudaMalloc(&ctx->d_cnorm, sizeof(double) * sl));
+  CK(cudaMalloc(&ctx->d_cnorm, sizeof(double) * 2 * sl));
   ctx->m_elems = m_el;
   ctx->f_bytes = f_b;
   ctx->vec_elems = v_el;
@@ -325,7 +325,7 @@ void fill_slot(b200tau_ctx *ctx, JobDev &J, int slot, int ld, const Plan &p) {
   J.hist = p.fk == kFactorFP32 ? v + (size_t)3 * ld * kMaxB : nullptr;
   J.ld = ld;
   J.conv = ctx->d_conv + slot;
-  J.cnorm = ctx->d_cnorm + slot;
+  J.cnorm = ctx->d_cnorm + 2 * slot;
   J.slot = slot;
   J.err = ctx->d_err;
   J.piv = nullptr;
@@ -360,12 +360,12 @@ TmatView tmat_view(const b200tau_ctx *ctx) {
 int *slot_piv(const b200tau_ctx *ctx, int slot) { return ctx->d_piv + (size_t)slot * ctx->piv_ints; }
 
 // Clears the per-slot status of the first nw slots: singular-pivot info, converged flag, last
-// correction size.
+// correction sizes.
 int reset_slot_status(b200tau_ctx *ctx, int nw) {
   CK(cudaMemsetAsync(ctx->d_info, 0, sizeof(int) * nw, ctx->stream));
   CK(cudaMemsetAsync(ctx->d_info + ctx->slots, 0, sizeof(int) * nw, ctx->stream));
   CK(cudaMemsetAsync(ctx->d_conv, 0, sizeof(int) * nw, ctx->stream));
-  CK(cudaMemsetAsync(ctx->d_cnorm, 0, sizeof(double) * nw, ctx->stream));
+  CK(cudaMemsetAsync(ctx->d_cnorm, 0, sizeof(double) * 2 * nw, ctx->stream));
   return B200TAU_OK;
 }
 

@@ -7,6 +7,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "refine_rule.h"
+
 namespace b200 {
 
 constexpr int kMaxLmax = 3;                                     // maxlmax supported
@@ -29,16 +31,9 @@ __host__ __device__ constexpr int pivot_mags_offset(int ld) { return 2 * ld + 1 
 __host__ __device__ constexpr int pivot_ints(int ld) { return pivot_mags_offset(ld) + ld; }
 // Columns of one tile of the tensor-core trailing update (tc_update.cu).
 constexpr int kTcTileCols = 256;
-// A refining job stops once its estimated remaining error on tau00 is below this fraction of
-// max|tau00|: 100x below the mixed path's 1e-10 accuracy target.
-constexpr double kRefineTol = 1e-12;
 // N x b vectors that the accelerated refinement of FP32 factors keeps: the iterate before the round, and
 // the corrected iterates and corrections of two earlier rounds (accelerate_kernel, block_lu.cu).
 constexpr int kHistory = 5;
-// JobDev::conv values (0: still refining)
-constexpr int kConverged = 1;
-constexpr int kDiverged = 2;  // the corrections stopped shrinking (numerical)
-constexpr int kAborted = 3;   // a bounded wait of a dataflow sweep ran out on this job
 // Bits of the context's device error word: a bounded wait ran out in the KKR build's table copy,
 // in the tensor-core trailing update, or in a dataflow sweep of the refinement.
 constexpr int kErrBuildWait = 1;
@@ -101,7 +96,7 @@ struct JobDev {
   const double2 *t0;     // central t-matrix (b x b, ld t0_ld)
   double2 *out;          // b*b complex result
   int *conv;             // refinement converged flag (set on the device, skips later rounds)
-  double *cnorm;         // relative size of the previous refinement correction (0 before round 1)
+  double *cnorm;         // relative sizes of the last two refinement corrections, latest first (0: none)
   double2 ubr[4];
   double2 ubrd[4];
   int L, N, n, b;
