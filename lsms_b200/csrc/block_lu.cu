@@ -1183,7 +1183,8 @@ cudaError_t sweep_solve(const JobDev *jobs, int njobs, int b, int max_N, int mod
   return cudaSuccess;
 }
 
-// After a refinement round: c = max|correction| / max|tau00| on the tau00 block, and what refine_state
+// After a refinement round: c = max|correction| / max|tau00| on the tau00 block (NaN where an element of
+// either is not finite, which refinement cannot mend), and what refine_state
 // (refine_rule.h) makes of it and the two corrections before it.  A job that is kConverged or kDiverged is
 // skipped from then on; every job that is not kConverged after the last round is re-solved by FP64 block LU.
 __global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__restrict__ jobs, bool accelerated,
@@ -1192,16 +1193,19 @@ __global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__res
   if (J.conv == nullptr || converged(J) || J.inactive) return;
   const int b = J.b, n = J.n, ld = J.ld;
   double my = 0.0, mx = 0.0;
+  int finite = 1;
   for (int e = threadIdx.x; e < b * b; e += blockDim.x) {
     const int r = e % b, c = e / b;
     const size_t idx = (size_t)(n + r) + (size_t)c * ld;
-    my = fmax(my, cabs1(J.Y[idx]));
-    mx = fmax(mx, cabs1(J.X[idx]));
+    const double y = cabs1(J.Y[idx]), x = cabs1(J.X[idx]);
+    my = fmax(my, y);
+    mx = fmax(mx, x);
+    finite = finite && isfinite(y) && isfinite(x);  // (fmax passes over a NaN)
   }
   __shared__ double sy[256], sx[256];
   sy[threadIdx.x] = my;
   sx[threadIdx.x] = mx;
-  __syncthreads();
+  finite = __syncthreads_and(finite);
   for (int o = 128; o > 0; o >>= 1) {
     if ((int)threadIdx.x < o) {
       sy[threadIdx.x] = fmax(sy[threadIdx.x], sy[threadIdx.x + o]);
@@ -1210,7 +1214,7 @@ __global__ void __launch_bounds__(256) converge_check_kernel(const JobDev *__res
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    const double c = sx[0] > 0.0 ? sy[0] / sx[0] : 0.0;
+    const double c = !finite ? nan("") : sx[0] > 0.0 ? sy[0] / sx[0] : 0.0;
     const double prev = J.cnorm ? J.cnorm[0] : 0.0, prev2 = J.cnorm ? J.cnorm[1] : 0.0;
     *J.conv = refine_state(c, prev, prev2, accelerated, last);
     if (J.cnorm) {

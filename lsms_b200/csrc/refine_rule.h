@@ -34,6 +34,7 @@ constexpr int kAborted = 3;   // a bounded wait of a dataflow sweep ran out on t
 // A job that stops shrinking, or has had its last round, is at its rounding floor if the correction itself is
 // below kRefineTol; any other is left to the FP64 re-solve.
 B200_HD int refine_state(double c, double prev, double prev2, bool accelerated, bool last) {
+  if (!(c <= 1e300)) return kDiverged;  // not finite
   const bool stalled = prev > 0.0 && c >= prev;
   double ratio = prev > 0.0 ? c / prev : 1.0;
   if (accelerated && prev2 > 0.0 && prev / prev2 > ratio) ratio = prev / prev2;
