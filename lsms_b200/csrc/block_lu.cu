@@ -66,19 +66,6 @@ using namespace cx;
 constexpr int kDiagThreads = 256;
 static_assert(kDiagThreads == 256 && kNb == 64, "diagonal inverse layout: 2 rows per lane, 8 panels, 8 row tiles");
 
-// 1 / d = conj(d) / |d|^2 (pivots of these blocks are far from the FP64 range limits); 0 for a zero.
-// 1 / |d|^2 by two Newton steps from the hardware's 20-bit approximation (2^-20, 2^-40, 2^-80 before
-// rounding), without the branches of a division, which kept the compiler from filling the chain's
-// latencies with the rest of the update (180 cycles a step).
-__device__ __forceinline__ double2 reciprocal(double2 d) {
-  const double q = d.x == 0.0 && d.y == 0.0 ? 1.0 : d.x * d.x + d.y * d.y;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(q));
-  r = fma(r, fma(-q, r, 1.0), r);
-  r = fma(r, fma(-q, r, 1.0), r);
-  return make_double2(d.x * r, -d.y * r);
-}
-
 // PER_SM = blocks per SM the register budget allows: 1 (for the elimination that keeps one SM per job
 // free for the inverses) or 2 (for the elimination with panel pivoting, which leaves fewer SMs to them).
 template <typename T, int PER_SM>

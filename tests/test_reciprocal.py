@@ -1,0 +1,99 @@
+"""The reciprocal of the elimination's pivots (lsms_b200/csrc/cplx.cuh) over the whole exponent range."""
+
+import ctypes
+import subprocess
+
+import numpy as np
+import pytest
+
+from lsms_b200 import build as B
+
+SRC = r'''
+#include "cplx.cuh"
+using namespace b200::cx;
+// ours, and the same by CUDA's division
+__global__ void recip(const double2 *d, double2 *ours, double2 *div, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  ours[i] = reciprocal(d[i]);
+  int e;
+  frexp(fmax(fabs(d[i].x), fabs(d[i].y)), &e);
+  const double x = ldexp(d[i].x, -e), y = ldexp(d[i].y, -e), r = 1.0 / (x * x + y * y);
+  div[i] = make_double2(ldexp(x * r, -e), ldexp(-y * r, -e));
+}
+extern "C" int run(const double *d, double *ours, double *div, int n) {
+  double2 *p;
+  if (cudaMalloc(&p, 3 * n * sizeof(double2)) != cudaSuccess) return 1;
+  cudaMemcpy(p, d, n * sizeof(double2), cudaMemcpyHostToDevice);
+  recip<<<(n + 255) / 256, 256>>>(p, p + n, p + 2 * n, n);
+  cudaMemcpy(ours, p + n, n * sizeof(double2), cudaMemcpyDeviceToHost);
+  cudaMemcpy(div, p + 2 * n, n * sizeof(double2), cudaMemcpyDeviceToHost);
+  cudaFree(p);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+'''
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    d = tmp_path_factory.mktemp("recip")
+    (d / "recip.cu").write_text(SRC)
+    so = str(d / "recip.so")
+    subprocess.run([B.nvcc(), "-shared", "-Xcompiler", "-fPIC", "-O3", "-std=c++17", *B.ARCH, "-I", B.CSRC,
+                    str(d / "recip.cu"), "-o", so], check=True)
+    lib = ctypes.CDLL(so)
+
+    def call(d):
+        out = [np.empty_like(d), np.empty_like(d)]
+        assert lib.run(*(ctypes.c_void_p(a.ctypes.data) for a in (d, *out)), ctypes.c_int(d.size)) == 0
+        return out
+
+    return call
+
+
+@pytest.mark.gpu
+def test_reciprocal_over_the_exponent_range(run):
+    rng = np.random.default_rng(0)
+    n = 200000
+    e = rng.integers(-1022, 1022, size=n)
+    x, y = rng.uniform(1.0, 2.0, size=(2, n)) * rng.choice([-1.0, 1.0], size=(2, n))
+    other = np.where(rng.random(n) < 0.8, rng.integers(0, 4, size=n), rng.integers(0, 1000, size=n))
+    a, b = np.ldexp(x, e), np.ldexp(y, np.maximum(e - other, -1074))
+    swap = rng.random(n) < 0.5
+    d = np.where(swap, b, a) + 1j * np.where(swap, a, b)
+    ours, div = run(d)
+    xl, yl = d.real.astype(np.longdouble), d.imag.astype(np.longdouble)
+    q = xl * xl + yl * yl
+    size = 1 / np.sqrt(q)
+    # the sum of squares is off by at most 2 u, its reciprocal by 1.5 u more, each product by u (u = 2^-53); a
+    # result below 2^-1022 also by half its last place, 2^-1075
+    for got, bound in ((ours.real - xl / q, 5), (ours.imag + yl / q, 5), (ours - div, 5)):
+        assert np.all(np.abs(got) <= bound * 2.0 ** -53 * size + 2.0 ** -1074)
+
+
+@pytest.mark.gpu
+def test_reciprocal_of_special_values(run):
+    tiny, top = 2.0 ** -1022, np.finfo(np.float64).max
+    d = np.array([0.0, -0.0, complex(np.inf, 1.0), complex(1.0, -np.inf), complex(np.nan, 1.0), complex(tiny, tiny),
+                  complex(1e-162, 0.0), complex(0.0, 1e-200), complex(top, -top), complex(7e153, 0.0)])
+    got = run(d)[0]
+    assert np.all(got[:2] == 0)
+    assert np.all(np.isnan(got[2:5].real) & np.isnan(got[2:5].imag))
+    want = 1 / d[5:].astype(np.clongdouble)
+    assert np.all(np.abs(got[5:] - want) <= 5 * 2.0 ** -53 * np.abs(want) + 2.0 ** -1074)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1e-170, 1e-154, 1.2e-154, 1e-100])
+def test_pivots_with_squares_out_of_range(solver_factory, scale):
+    """Pivots whose squares underflow or are subnormal are neither lost nor reported as singular."""
+    from lsms_b200 import tau as T
+    rng = np.random.default_rng(5)
+    n = 96
+    m = scale * (np.eye(n) + 0.04 * (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))))
+    t0 = scale * (rng.normal(size=(16, 16)) + 1j * rng.normal(size=(16, 16)))
+    rhs = np.zeros((n, 16), np.complex128)
+    rhs[:16] = t0
+    want = np.linalg.solve(m / scale, rhs / scale)[:16]
+    got = solver_factory(3, 1, 1).solve_tau00_dense(m, t0, T.PREC_FP64)
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
