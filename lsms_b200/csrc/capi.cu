@@ -841,7 +841,7 @@ int wave_graph(b200tau_ctx *ctx, int nw, int maxL, int maxn, int maxN, int ld, c
       (long long)(uintptr_t)ctx->d_info, (long long)(uintptr_t)ctx->d_active, (long long)(uintptr_t)ctx->d_err,
       (long long)(uintptr_t)ctx->d_tmat, (long long)(uintptr_t)ctx->d_tdiag, (long long)(uintptr_t)ctx->d_F,
       (long long)(uintptr_t)ctx->d_pack, ctx->tc_ld, ctx->tc_slots, ctx->la.min_n, ctx->la.pair_min_rest,
-      (long long)(uintptr_t)(split ? ctx->d_split : nullptr), ctx->split_ld};
+      (long long)(uintptr_t)(split ? ctx->d_split : nullptr), ctx->split_ld, ctx->split_slots};
   for (size_t i = 0; i < ctx->wg.size(); ++i)
     if (ctx->wg[i].key == key) {
       const WaveGraph g = ctx->wg[i];  // most recently used last
