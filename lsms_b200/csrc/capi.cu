@@ -150,6 +150,8 @@ struct b200tau_ctx {
   SplitBufs split;
   unsigned char *d_split = nullptr;
   int split_ld = 0, split_slots = 0;
+  // the smallest request that found no room, and the free memory it found
+  size_t split_failed_bytes = SIZE_MAX, split_failed_free = 0;
   // the mixed path's FP64 re-solve as graphs with a conditional body (fallback_graph)
   cudaStream_t cap_stream = nullptr;
   std::vector<FallbackGraph> fb;  // most recently used last
@@ -479,26 +481,38 @@ int ensure_tc(b200tau_ctx *ctx, int ld, int slots) {
   return B200TAU_OK;
 }
 
-// The digit planes of the FP64 update, for `slots` jobs of leading dimension up to ld.
-int ensure_split(b200tau_ctx *ctx, int ld, int slots) {
-  if (ctx->d_split && ld <= ctx->split_ld && slots <= ctx->split_slots) return B200TAU_OK;
-  CK(cudaStreamSynchronize(ctx->stream));
-  cudaFree(ctx->d_split);
-  ctx->d_split = nullptr;
+size_t split_bytes(int ld, int slots) {
+  return split_slot_bytes(ld) * slots + sizeof(int) * kSplitCounters * (ld / kNb + 1);
+}
+
+bool split_fits(const b200tau_ctx *ctx, int ld, int nw) {
+  return ctx->d_split && ld <= ctx->split_ld && nw <= ctx->split_slots;
+}
+
+// The digit planes of the FP64 update, for a wave of nw jobs of leading dimension ld.  Where there is no
+// room for them the planes stay as they are, for the waves that they do hold, and the same
+// request is not tried again until more memory is free.
+int ensure_split(b200tau_ctx *ctx, int ld, int nw) {
+  if (split_fits(ctx, ld, nw)) return B200TAU_OK;
   ld = std::max(ld, ctx->split_ld);
-  slots = std::max(slots, ctx->split_slots);
-  SplitBufs &t = ctx->split;
+  const int slots = std::max({nw, ctx->slots, ctx->split_slots});
+  const size_t bytes = split_bytes(ld, slots);
+  size_t freeb = 0, totalb = 0;
+  CK(cudaMemGetInfo(&freeb, &totalb));
+  if (freeb < bytes || (bytes >= ctx->split_failed_bytes && freeb <= ctx->split_failed_free)) return B200TAU_OK;
+  unsigned char *mem = nullptr;
+  if (cudaMalloc(&mem, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->split_failed_bytes = bytes;
+    ctx->split_failed_free = freeb;
+    return B200TAU_OK;
+  }
+  SplitBufs t;
   t.ld = ld;
   t.steps = ld / kNb + 1;
   t.a_slot = (size_t)2 * ld * kSplitDigits * kSplitRowBytes;
   t.b_slot = (size_t)ld * kSplitDigits * kSplitRowBytes;
-  if (cudaMalloc(&ctx->d_split, split_slot_bytes(ld) * slots + sizeof(int) * kSplitCounters * t.steps) != cudaSuccess) {
-    cudaGetLastError();  // no room: the updates stay on the FP64 tensor cores
-    ctx->d_split = nullptr;
-    ctx->split_ld = ctx->split_slots = 0;
-    return B200TAU_OK;
-  }
-  t.a = reinterpret_cast<signed char *>(ctx->d_split);
+  t.a = reinterpret_cast<signed char *>(mem);
   t.b = t.a + t.a_slot * slots;
   t.a_scale = reinterpret_cast<double *>(t.b + t.b_slot * slots);
   t.b_scale = t.a_scale + (size_t)ld * slots;
@@ -506,22 +520,35 @@ int ensure_split(b200tau_ctx *ctx, int ld, int slots) {
   t.counters = t.balance + (size_t)kNb * slots;
   void *fn = nullptr;
   cudaDriverEntryPointQueryResult q;
-  CK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q));
-  if (!fn || q != cudaDriverEntryPointSuccess) return fail(ctx, B200TAU_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-  EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(fn);
-  const cuuint32_t estr[3] = {1, 1, 1};
-  for (int i = 0; i < 2; ++i) {
-    const cuuint64_t rows = (cuuint64_t)(i == 0 ? 2 : 1) * ld * kSplitDigits;
-    const cuuint64_t dims[3] = {(cuuint64_t)kSplitRowBytes, rows, (cuuint64_t)slots};
-    const cuuint64_t strides[2] = {(cuuint64_t)kSplitRowBytes, rows * kSplitRowBytes};
-    const cuuint32_t box[3] = {(cuuint32_t)kSplitRowBytes, (cuuint32_t)(i == 0 ? 128 : 32), 1};
-    const CUresult r = enc(i == 0 ? &t.tA : &t.tB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, i == 0 ? t.a : t.b, dims, strides,
-                           box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(ctx, B200TAU_ERR_CUDA, "cuTensorMapEncodeTiled (digits) failed (%d)", (int)r);
+  CUresult r = CUDA_ERROR_NOT_FOUND;
+  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) == cudaSuccess && fn &&
+      q == cudaDriverEntryPointSuccess) {
+    EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(fn);
+    const cuuint32_t estr[3] = {1, 1, 1};
+    r = CUDA_SUCCESS;
+    for (int i = 0; i < 2 && r == CUDA_SUCCESS; ++i) {
+      const cuuint64_t rows = (cuuint64_t)(i == 0 ? 2 : 1) * ld * kSplitDigits;
+      const cuuint64_t dims[3] = {(cuuint64_t)kSplitRowBytes, rows, (cuuint64_t)slots};
+      const cuuint64_t strides[2] = {(cuuint64_t)kSplitRowBytes, rows * kSplitRowBytes};
+      const cuuint32_t box[3] = {(cuuint32_t)kSplitRowBytes, (cuuint32_t)(i == 0 ? 128 : 32), 1};
+      r = enc(i == 0 ? &t.tA : &t.tB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, i == 0 ? t.a : t.b, dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
   }
+  if (r != CUDA_SUCCESS) {
+    cudaFree(mem);
+    return fail(ctx, B200TAU_ERR_CUDA, "cuTensorMapEncodeTiled (digits) failed (%d)", (int)r);
+  }
+  unsigned char *old = ctx->d_split;
+  ctx->split = t;
+  ctx->d_split = mem;
   ctx->split_ld = ld;
   ctx->split_slots = slots;
+  if (old) {
+    CK(cudaStreamSynchronize(ctx->stream));  // no launch still uses the old planes
+    cudaFree(old);
+  }
   return B200TAU_OK;
 }
 
@@ -530,8 +557,8 @@ int ensure_split(b200tau_ctx *ctx, int ld, int slots) {
 int split_for(b200tau_ctx *ctx, FactorKind fk, int maxN, int ld, int nw, const SplitBufs **out) {
   *out = nullptr;
   if (fk != kFactorFP64 || !split_pays(maxN, maxN, nw)) return B200TAU_OK;
-  const int rc = ensure_split(ctx, ld, std::max(nw, ctx->slots));
-  if (rc == B200TAU_OK && ctx->d_split) *out = &ctx->split;
+  const int rc = ensure_split(ctx, ld, nw);
+  if (rc == B200TAU_OK && split_fits(ctx, ld, nw)) *out = &ctx->split;
   return rc;
 }
 
