@@ -303,11 +303,17 @@ int ensure_out(b200tau_ctx *ctx, size_t n) {
   return B200TAU_OK;
 }
 
+size_t split_bytes(int ld, int slots) {
+  return split_slot_bytes(ld) * slots + sizeof(int) * kSplitCounters * (ld / kNb + 1);
+}
+
 int choose_slots(b200tau_ctx *ctx, int ld, int njobs, const Plan &p, size_t extra_per_slot = 0) {
   size_t freeb = 0, totalb = 0;
   if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) freeb = (size_t)8 << 30;
   // memory already held by the context's workspace counts as available to it
   freeb += ctx->m_elems * ctx->slots * sizeof(double2) + ctx->f_bytes * ctx->slots;
+  // (for FP64 factors the digit planes too, which extra_per_slot counts)
+  if (p.fk == kFactorFP64 && ctx->d_split) freeb += split_bytes(ctx->split_ld, ctx->split_slots);
   const size_t per = (size_t)ld * ld * (sizeof(double2) + (p.f_separate ? f_elem_bytes(p) : 0)) +
                      vec_elems_for(p, ld) * sizeof(double2) + extra_per_slot;
   const size_t budget = freeb / 2;
@@ -479,10 +485,6 @@ int ensure_tc(b200tau_ctx *ctx, int ld, int slots) {
   ctx->tc_ld = ld;
   ctx->tc_slots = slots;
   return B200TAU_OK;
-}
-
-size_t split_bytes(int ld, int slots) {
-  return split_slot_bytes(ld) * slots + sizeof(int) * kSplitCounters * (ld / kNb + 1);
 }
 
 bool split_fits(const b200tau_ctx *ctx, int ld, int nw) {

@@ -76,3 +76,21 @@ def test_planes_that_find_no_room():
     finally:
         w.s.close()
         _release(held)
+
+
+@pytest.mark.gpu
+def test_waves_do_not_depend_on_the_planes_held():
+    """The same call twice with little memory: the planes allocated by the first count as available to the
+    second, so both take the same waves."""
+    w = _Waves((6,), 16)
+    held = []
+    try:
+        w.solve(6, 1)  # what a context allocates besides the wave's slots
+        ld = 1408
+        slot = 32 * ld * ld + 3 * ld * 32 * 16 + ld * (3 * 8 * 128 + 16) + 256
+        held = _hog(2 * 6.16 * slot - 32 * ld * ld)  # six slots and a sixth (one is held)
+        counts = [w.solve(6, 16)[1] for _ in range(3)]
+        assert len(set(counts)) == 1
+    finally:
+        w.s.close()
+        _release(held)
