@@ -676,17 +676,18 @@ __global__ void active_list_kernel(const JobDev *__restrict__ jobs, int njobs, i
 
 // Work item i is row block i / count of the i % count-th job: of the jobs listed in `active`
 // (active_list_kernel), so that the jobs still refining spread evenly over the SMs, or of all njobs.
-// With few items, `split` CTAs of a cluster share one item, each over its share of K.
+// With few items, `split` CTAs of a cluster share one item, each over its share of K; `whole`: always all
+// of them (FP64 factors, whose results then do not depend on how many jobs share the wave).
 template <int BC>
 __global__ void __cluster_dims__(kResCluster, 1, 1) __launch_bounds__(kResThreads, 4)
-    residual_kernel(const JobDev *__restrict__ jobs, const int *__restrict__ active, int njobs, int rowblocks) {
+    residual_kernel(const JobDev *__restrict__ jobs, const int *__restrict__ active, int njobs, int rowblocks, bool whole) {
   constexpr int ROWS = residual_rows<BC>();  // rows per CTA
   constexpr int RT = ROWS / 32;              // 8-row tiles per warp (four warps)
   constexpr int NB = BC / 8;                 // 8-column blocks
   static_assert(kResThreads == 128 && RT * 32 == ROWS && NB * 8 == BC && kResK % 4 == 0, "residual layout");
   const int cnt = active != nullptr ? active[0] : njobs;
   int split = kResCluster;  // the same in every CTA
-  while (split > 1 && cnt * rowblocks * split > kResWave) split >>= 1;
+  while (!whole && split > 1 && cnt * rowblocks * split > kResWave) split >>= 1;
   const int item = blockIdx.x / split, slice = blockIdx.x % split;
   if ((int)(blockIdx.x / kResCluster) * (kResCluster / split) >= cnt * rowblocks) return;  // (the whole cluster)
   const bool valid = item < cnt * rowblocks;
@@ -695,7 +696,7 @@ __global__ void __cluster_dims__(kResCluster, 1, 1) __launch_bounds__(kResThread
   const int N = J.N, ld = J.ld, b = J.b;
   const int row0 = rb * ROWS;
   const bool live = valid && !converged(J) && !J.inactive && row0 < N;
-  if (split == 1 && !live) return;
+  if ((split == 1 || split == kResCluster) && !live) return;  // (at kResCluster the whole cluster)
   extern __shared__ __align__(16) unsigned char rsm[];
   double2(*Ms)[kResK][ROWS + kResPad] = reinterpret_cast<double2(*)[kResK][ROWS + kResPad]>(rsm);
   double2(*Xs)[kResK][BC + kResPad] = reinterpret_cast<double2(*)[kResK][BC + kResPad]>(
@@ -1408,16 +1409,17 @@ cudaError_t launch_refine_begin(FactorKind fk, const JobDev *jobs, int njobs, in
 }
 
 template <int BC>
-cudaError_t launch_residual(const JobDev *jobs, int njobs, int max_N, int *active, cudaStream_t s) {
+cudaError_t launch_residual(const JobDev *jobs, int njobs, int max_N, int *active, bool whole, cudaStream_t s) {
   constexpr int sm = residual_smem_bytes<BC>();
   const cudaError_t e = ensure_smem(residual_kernel<BC>, sm);
   if (e != cudaSuccess) return e;
   const int rowblocks = (max_N + residual_rows<BC>() - 1) / residual_rows<BC>();
   if (active) active_list_kernel<<<1, 32, 0, s>>>(jobs, njobs, active);
   // room for every item alone, or for the split of the few items that are split
-  int grid = std::max(njobs * rowblocks, std::min(njobs * rowblocks * kResCluster, kResWave));
+  int grid = whole ? njobs * rowblocks * kResCluster
+                   : std::max(njobs * rowblocks, std::min(njobs * rowblocks * kResCluster, kResWave));
   grid = (grid + kResCluster - 1) / kResCluster * kResCluster;
-  residual_kernel<BC><<<grid, kResThreads, sm, s>>>(jobs, active, njobs, rowblocks);
+  residual_kernel<BC><<<grid, kResThreads, sm, s>>>(jobs, active, njobs, rowblocks, whole);
   return cudaGetLastError();
 }
 
@@ -1434,8 +1436,8 @@ cudaError_t launch_refine_round(FactorKind fk, const JobDev *jobs, int njobs, in
                                 bool check, int *info, cudaStream_t s, long *launches, bool fp32_sweep,
                                 const CUtensorMap *fmap, int active_hint, int *active, int accelerate, bool last) {
   (void)max_n;
-  const cudaError_t e0 = b <= 16 ? launch_residual<16>(jobs, njobs, max_N, active, s)
-                                 : launch_residual<32>(jobs, njobs, max_N, active, s);
+  const cudaError_t e0 = b <= 16 ? launch_residual<16>(jobs, njobs, max_N, active, fk == kFactorFP64, s)
+                                 : launch_residual<32>(jobs, njobs, max_N, active, fk == kFactorFP64, s);
   if (e0 != cudaSuccess) return e0;
   if (launches) *launches += active ? 2 : 1;
   const cudaError_t e = fk == kFactorFP64 ? sweep_solve<double2>(jobs, njobs, b, max_N, 1, info, s, launches, false, nullptr)

@@ -225,3 +225,37 @@ def test_fp64_resolve_job_counts(solver_factory, lattice, shells, njobs):
     for i in range(njobs):
         t0 = -port.tau00_l(prob, np.zeros((16, 16), np.complex128), i)
         assert np.abs(got[i] - want[i]).max() <= 1e-12 * np.abs(want[i] + t0).max()
+
+
+def _register(s, shells, energies, cant=1, seed=17):
+    """Atoms 0, 1, ... with these numbers of fcc shells over one t-matrix store."""
+    probs = [W.make_problem("fcc", 6.82, sh, 3, energies, seed, n_species=2, n_spin_cant=cant, n_spin_pola=cant)
+             for sh in shells]
+    s.upload_tmat(probs[0].tmat_store)
+    for a, p in enumerate(probs):
+        p.tmat_store, p.liz_store_idx = probs[0].tmat_store, np.minimum(p.liz_store_idx, 1)
+        s.set_atom(a, p.liz_pos, p.liz_lmax, p.liz_store_idx, p.ubr, p.ubrd)
+    return probs
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shells,cant,nen,pivoting", [
+    ((2,), 1, 40, T.PIVOT_BLOCK),           # N = 304: the residual's split
+])
+def test_fp64_results_do_not_depend_on_the_batch(solver_factory, shells, cant, nen, pivoting):
+    """Every job of a batch, bit for bit the result of the job alone, and against the oracle."""
+    from oracle import port
+    s = solver_factory(3, cant, cant)
+    energies = W.semicircle_contour(-0.2, 0.7, nen)
+    probs = _register(s, shells, energies, cant)
+    specs = [(a, i, 0, e) for i, e in enumerate(energies) for a in range(len(shells))]
+    s.set_pivoting(pivoting)
+    try:
+        out = s.solve_jobs(T.make_jobs(specs), T.PREC_FP64)
+        for j, spec in enumerate(specs):
+            assert np.array_equal(out[j], s.solve_jobs(T.make_jobs([spec]), T.PREC_FP64)[0])
+    finally:
+        s.set_pivoting(T.PIVOT_AUTO)
+    for a in range(len(shells) if len(shells) > 1 else 0):
+        bound = max(1e-12, 8 * np.linalg.cond(port.build_kkr(probs[a], 1)) * 2.0 ** -53)
+        assert _tau_err(probs[a], 1, out[len(shells) + a]) <= bound
