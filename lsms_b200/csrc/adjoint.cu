@@ -39,12 +39,12 @@ using GemmView = s8::View;
 // Tiles of 16 WM x 16 WN on the FP64 tensor cores (dmma.cuh), in columns of `len`.
 template <class Op, int WM, int WN, int MODE>
 __global__ void __launch_bounds__(dm::kThreads, WM == 4 ? 3 : 4)
-    zgemm_view_kernel(const JobDev *__restrict__ jobs, int k, Op op, int len) {
+    zgemm_view_kernel(const JobDev *__restrict__ jobs, int k, Op op, int len, bool small) {
   extern __shared__ __align__(16) double2 vsm64[];
   using TL = dm::Tile<WM, WN>;
   const JobDev &J = jobs[blockIdx.z];
   GemmView g;
-  if (!op(J, k, g)) return;
+  if (!op(J, k, g) || (small && split_pays(g.m, g.n, kSplitInverse))) return;
   const int row0 = blockIdx.y * len * TL::kRows, col0 = blockIdx.x * TL::kCols;
   if (row0 >= g.m || col0 >= g.n) return;
   dm::zgemm_column<WM, WN, MODE>(g.A + row0, g.lda, g.B + (size_t)col0 * g.ldb, g.ldb,
@@ -151,14 +151,14 @@ __global__ void __launch_bounds__(256) schur_inverse_kernel(const JobDev *__rest
 }
 
 template <class Op, int WM, int WN, int MODE>
-cudaError_t gemm_launch_tile(const JobDev *jobs, int njobs, int k, int max_m, int max_n, cudaStream_t s) {
+cudaError_t gemm_launch_tile(const JobDev *jobs, int njobs, int k, int max_m, int max_n, bool small, cudaStream_t s) {
   using TL = dm::Tile<WM, WN>;
   const cudaError_t e = ensure_smem(zgemm_view_kernel<Op, WM, WN, MODE>, TL::kSmem);
   if (e != cudaSuccess) return e;
   const int tx = (max_n + TL::kCols - 1) / TL::kCols, ty = (max_m + TL::kRows - 1) / TL::kRows;
   const int len = dm::column_tiles((long)tx * ty * njobs);
   zgemm_view_kernel<Op, WM, WN, MODE>
-      <<<dim3(tx, (ty + len - 1) / len, njobs), dm::kThreads, TL::kSmem, s>>>(jobs, k, Op(), len);
+      <<<dim3(tx, (ty + len - 1) / len, njobs), dm::kThreads, TL::kSmem, s>>>(jobs, k, Op(), len, small);
   return cudaGetLastError();
 }
 
@@ -166,24 +166,29 @@ cudaError_t gemm_launch_tile(const JobDev *jobs, int njobs, int k, int max_m, in
 // elimination's update.
 template <class Op, int MODE>
 cudaError_t gemm_launch(const JobDev *jobs, int njobs, int k, int max_m, int max_n, cudaStream_t s,
-                        long *launches) {
+                        long *launches, bool small = false) {
   if (max_m <= 0 || max_n <= 0) return cudaSuccess;
   if (launches) *launches += 1;
-  return gemm_launch_tile<Op, MODE == kOverwrite ? 4 : 2, 2, MODE>(jobs, njobs, k, max_m, max_n, s);
+  return gemm_launch_tile<Op, MODE == kOverwrite ? 4 : 2, 2, MODE>(jobs, njobs, k, max_m, max_n, small, s);
 }
 
-// A pass's update at step k: on the integer tensor cores where it is large enough.
+// A pass's update at step k, m x n of at most max_m x max_n and, for every job, at least min_m x min_n: on
+// the integer tensor cores for the jobs whose own is large enough (split_pays).
 template <class Op>
-cudaError_t subtract_launch(const JobDev *jobs, int njobs, int k, int max_m, int max_n, const SplitBufs *split, int pass,
-                            int *err, cudaStream_t s, long *launches) {
-  if (!split || !split_pays(max_m, max_n, njobs))
-    return gemm_launch<Op, kSubtract>(jobs, njobs, k, max_m, max_n, s, launches);
-  const Op op;
-  const cudaError_t e = s8::launch_split_pack(*split, jobs, njobs, k, max_m, max_n, s, op);
-  if (e != cudaSuccess) return e;
-  if (launches) *launches += 3;
-  return s8::launch_split_update(*split, jobs, njobs, k, max_m, max_n, false,
-                                 split->counters + pass * split->steps + k / kNb, err, s, op);
+cudaError_t subtract_launch(const JobDev *jobs, int njobs, int k, int min_m, int min_n, int max_m, int max_n,
+                            const SplitBufs *split, int pass, int *err, cudaStream_t s, long *launches) {
+  const bool large = split && split_pays(max_m, max_n, kSplitInverse);
+  if (large) {
+    const s8::Large<Op, kSplitInverse> op;
+    cudaError_t e = s8::launch_split_pack(*split, jobs, njobs, k, max_m, max_n, s, op);
+    if (e == cudaSuccess)
+      e = s8::launch_split_update(*split, jobs, njobs, k, max_m, max_n, false,
+                                  split->counters + pass * split->steps + k / kNb, err, s, op);
+    if (e != cudaSuccess) return e;
+    if (launches) *launches += 4;
+    if (split_pays(min_m, min_n, kSplitInverse)) return cudaSuccess;
+  }
+  return gemm_launch<Op, kSubtract>(jobs, njobs, k, max_m, max_n, s, launches, large);
 }
 
 // One CTA per (LIZ position p, job): with G in M's storage, X refined and V = M^-1,
@@ -345,17 +350,19 @@ cudaError_t launch_tau_full(const JobDev *jobs, int njobs, int max_L, int max_N,
   return cudaGetLastError();
 }
 
-cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, const SplitBufs *split, int *err,
-                           cudaStream_t s, long *launches) {
+cudaError_t launch_inverse(const JobDev *jobs, int njobs, int min_n, int max_n, int max_N, const SplitBufs *split,
+                           int *err, cudaStream_t s, long *launches) {
   if (njobs <= 0) return cudaSuccess;
   cudaError_t e;
+  const int min_N = min_n + max_N - max_n;
   if (split && (e = cudaMemsetAsync(split->counters + split->steps, 0, 2 * sizeof(int) * split->steps, s)) != cudaSuccess)
     return e;
   identity_kernel<<<dim3(max_N, njobs), 256, 0, s>>>(jobs);
   if (launches) *launches += 1;
   for (int k = 0; k < max_n; k += kNb) {
     if ((e = gemm_launch<OpInvDiag, kOverwrite>(jobs, njobs, k, kNb, k + kNb, s, launches)) != cudaSuccess) return e;
-    if ((e = subtract_launch<OpInvLower>(jobs, njobs, k, max_N - k - 1, k + kNb, split, 1, err, s, launches)) != cudaSuccess)
+    if ((e = subtract_launch<OpInvLower>(jobs, njobs, k, min_N - k - kNb, k + kNb, max_N - k - 1, k + kNb, split, 1, err,
+                                         s, launches)) != cudaSuccess)
       return e;
   }
   schur_inverse_kernel<<<njobs, 256, 0, s>>>(jobs);
@@ -363,7 +370,9 @@ cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, 
   if ((e = gemm_launch<OpSchurApply, kOverwrite>(jobs, njobs, 0, kMaxB, max_N, s, launches)) != cudaSuccess) return e;
   if ((e = gemm_launch<OpInvUpper, kSubtract>(jobs, njobs, -1, max_n, max_N, s, launches)) != cudaSuccess) return e;
   for (int k = ((max_n - 1) / kNb) * kNb; k >= 0 && max_n > 0; k -= kNb)
-    if ((e = subtract_launch<OpInvUpper>(jobs, njobs, k, k, max_N, split, 2, err, s, launches)) != cudaSuccess) return e;
+    if ((e = subtract_launch<OpInvUpper>(jobs, njobs, k, k < min_n ? k : 0, min_N, k, max_N, split, 2, err, s, launches)) !=
+        cudaSuccess)
+      return e;
   return cudaGetLastError();
 }
 

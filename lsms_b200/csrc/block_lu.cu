@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(dm::kThreads, 2) zgemm64_w_kernel(const JobDev
 // without look-ahead).
 template <int W>
 __global__ void __launch_bounds__(dm::kThreads, 4) zgemm64_update_kernel(const JobDev *__restrict__ jobs, int k, int tx,
-                                                                         int ty, int nj, int part, int len, bool sparse) {
+                                                                         int ty, int nj, int part, int len, bool sparse, bool small) {
   extern __shared__ __align__(16) double2 zsm64[];
   using TL = dm::Tile<W, W>;
   if (!sparse) {  // grid (tx, ty, nj)
@@ -517,6 +517,10 @@ __global__ void __launch_bounds__(dm::kThreads, 4) zgemm64_update_kernel(const J
     const int bx = blockIdx.x;
     int by = blockIdx.y * len, l = len;
     if (k >= J.n || J.inactive) return;
+    if (small) {  // only the jobs that the digit products leave
+      const int m = J.N - k - min(kNb, J.n - k);
+      if (split_pays(m, m, kSplitTrailing)) return;
+    }
     if (part == kOtherTiles && bx * TL::kCols < kNb) {  // without the first 64 rows
       const int skip = max(0, min(l, kNb / TL::kRows - by));
       by += skip;
@@ -1076,19 +1080,23 @@ cudaError_t eliminate32(const JobDev *jobs, int njobs, int max_n, int max_N, int
 }
 
 template <int W>
-void launch_update64_tiles(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, cudaStream_t s) {
+void launch_update64_tiles(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, bool small,
+                           cudaStream_t s) {
   using TL = dm::Tile<W, W>;
-  const int rows = part == kFirstBlock ? kNb : max_N - k - 1;
+  const int rows = part == kFirstBlock ? kNb : small ? std::min(kSplitSide - 1, max_N - k - 1) : max_N - k - 1;
   const int tx = (rows + TL::kCols - 1) / TL::kCols, tr = (rows + TL::kRows - 1) / TL::kRows;
   const int len = sparse ? 1 : dm::column_tiles((long)tx * tr * njobs);
   const int ty = (tr + len - 1) / len;
   const dim3 grid = sparse ? dim3(std::min(tx * ty * njobs, kSparseGrid)) : dim3(tx, ty, njobs);
-  zgemm64_update_kernel<W><<<grid, dm::kThreads, TL::kSmem, s>>>(jobs, k, tx, ty, njobs, part, len, sparse);
+  zgemm64_update_kernel<W><<<grid, dm::kThreads, TL::kSmem, s>>>(jobs, k, tx, ty, njobs, part, len, sparse, small);
 }
 
-void launch_update64(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, cudaStream_t s) {
-  if (part == kFirstBlock && 16 * njobs <= 4 * 148) launch_update64_tiles<1>(jobs, njobs, k, max_N, part, sparse, s);
-  else launch_update64_tiles<2>(jobs, njobs, k, max_N, part, sparse, s);
+// `small`: only the jobs whose update split_pays leaves to these tiles.
+void launch_update64(const JobDev *jobs, int njobs, int k, int max_N, int part, bool sparse, bool small, cudaStream_t s) {
+  if (part == kFirstBlock && 16 * njobs <= 4 * 148)
+    launch_update64_tiles<1>(jobs, njobs, k, max_N, part, sparse, small, s);
+  else
+    launch_update64_tiles<2>(jobs, njobs, k, max_N, part, sparse, small, s);
 }
 
 // FP64 factors.  With a second stream (and pivots inside the diagonal blocks) the update of step k
@@ -1107,6 +1115,8 @@ cudaError_t eliminate64(const JobDev *jobs, int njobs, int max_n, int max_N, int
   if ((e = ensure_smem(zgemm64_w_kernel<1>, dm::Tile<4, 1>::kSmem)) != cudaSuccess) return e;
   const bool ahead = la != nullptr && la->s2 != nullptr && !sparse && !panel;
   if (sparse) split = nullptr;
+  // the smallest job's N (b is the same for all; 0: not known)
+  const int min_N = la != nullptr ? la->min_n + max_N - max_n : 0;
   if (split && (e = cudaMemsetAsync(split->counters, 0, sizeof(int) * split->steps, s)) != cudaSuccess) return e;
   if (panel && (e = launch_pivot_init(jobs, njobs, s, launches)) != cudaSuccess) return e;
   for (int k = 0; k < max_n; k += kNb) {
@@ -1129,25 +1139,31 @@ cudaError_t eliminate64(const JobDev *jobs, int njobs, int max_n, int max_N, int
     const bool timed = timer && timer->used + 2 <= timer->cap;
     if (timed) cudaEventRecord(timer->ev[timer->used++], s);
     if (next) {
-      launch_update64(jobs, njobs, k, max_N, kFirstBlock, false, s);
+      launch_update64(jobs, njobs, k, max_N, kFirstBlock, false, false, s);
       if ((e = cudaEventRecord(la->panel, s)) != cudaSuccess) return e;
       if ((e = cudaStreamWaitEvent(la->s2, la->panel, 0)) != cudaSuccess) return e;
       launch_diag_inverse<double2>(false, jobs, njobs, k + kNb, info, smem_diag, la->s2);
       if ((e = cudaEventRecord(la->diag, la->s2)) != cudaSuccess) return e;
     }
-    if (split && split_pays(rest, rest, njobs)) {
-      const OpTrailing op;
-      if ((e = s8::launch_split_pack(*split, jobs, njobs, k, rest, rest, s, op)) != cudaSuccess) return e;
-      if ((e = s8::launch_split_update(*split, jobs, njobs, k, rest, rest, next, split->counters + k / kNb, err, s, op)) !=
+    // every job's update by digit products or on the FP64 tensor cores, as its own size asks (split_pays);
+    // no launch for a side that no job takes
+    const int most = max_N - k - kNb, least = min_N - k - kNb;
+    const bool large = split && split_pays(most, most, kSplitTrailing);
+    if (large) {
+      const s8::Large<OpTrailing, kSplitTrailing> op;
+      if ((e = s8::launch_split_pack(*split, jobs, njobs, k, most, most, s, op)) != cudaSuccess) return e;
+      if ((e = s8::launch_split_update(*split, jobs, njobs, k, most, most, next, split->counters + k / kNb, err, s, op)) !=
           cudaSuccess)
         return e;
-      if (launches) *launches += 2;
-    } else {
-      launch_update64(jobs, njobs, k, max_N, next ? kOtherTiles : kAllTiles, sparse, s);
+      if (launches) *launches += 4;
+    }
+    if (!large || !split_pays(least, least, kSplitTrailing)) {
+      launch_update64(jobs, njobs, k, max_N, next ? kOtherTiles : kAllTiles, sparse, large, s);
+      if (launches) *launches += 1;
     }
     if (timed) cudaEventRecord(timer->ev[timer->used++], s);
     if (next && (e = cudaStreamWaitEvent(s, la->diag, 0)) != cudaSuccess) return e;
-    if (launches) *launches += next ? 4 : 2;
+    if (launches) *launches += next ? 3 : 1;
   }
   if (panel && (e = launch_pivot_finish(jobs, njobs, s, launches)) != cudaSuccess) return e;
   return cudaGetLastError();

@@ -558,7 +558,7 @@ int ensure_split(b200tau_ctx *ctx, int ld, int nw) {
 // find no room.
 int split_for(b200tau_ctx *ctx, FactorKind fk, int maxN, int ld, int nw, const SplitBufs **out) {
   *out = nullptr;
-  if (fk != kFactorFP64 || !split_pays(maxN, maxN, nw)) return B200TAU_OK;
+  if (fk != kFactorFP64 || !split_pays(maxN, maxN, kSplitTrailing)) return B200TAU_OK;
   const int rc = ensure_split(ctx, ld, nw);
   if (rc == B200TAU_OK && split_fits(ctx, ld, nw)) *out = &ctx->split;
   return rc;
@@ -815,7 +815,7 @@ int run_refinement(b200tau_ctx *ctx, const std::vector<JobDev> &h, int nw, int m
   // Jobs whose FP32-factor refinement did not converge (condition numbers beyond what FP32 block
   // factors can refine, e.g. energies next to the real axis) take the FP64 path instead: an FP64
   // copy of the unmodified M, FP64 block elimination, the FP64 refinement rounds, tau00 from X -
-  // the same kernels and arithmetic as a PREC_FP64 solve of the job.
+  // the arithmetic of a PREC_FP64 solve of the job, with every update on the FP64 tensor cores.
   cudaGraphExec_t fb = nullptr;
   int rc = ensure_fallback(ctx, h[0].ld);
   if (rc || (rc = fallback_graph(ctx, nw, h[0].ld, b, ns, kkrsz, use_panel(ctx, maxN, kFactorFP64), &fb))) return rc;
@@ -1008,7 +1008,7 @@ int run_wave(b200tau_ctx *ctx, const b200tau_job *jobs, const int *idx, int nw, 
     const SplitBufs *split = nullptr;
     int rc = split_for(ctx, kFactorFP64, maxN, ld, nw, &split);
     if (rc) return rc;
-    CK(launch_inverse(ctx->d_jobs, nw, maxn, maxN, split, ctx->d_err, ctx->stream, &ctx->launches));
+    CK(launch_inverse(ctx->d_jobs, nw, ctx->la.min_n, maxn, maxN, split, ctx->d_err, ctx->stream, &ctx->launches));
     CK(launch_vjp_assemble(ctx->d_jobs, nw, maxL, ctx->kkrsz, ctx->ns, ctx->stream, &ctx->launches));
     return B200TAU_OK;
   }
@@ -1050,7 +1050,7 @@ int run_wave(b200tau_ctx *ctx, const b200tau_job *jobs, const int *idx, int nw, 
   CK(launch_kkr_build(ctx->d_jobs, nw, maxL, gp, ctx->d_err, ctx->stream, &ctx->launches));
   const SplitBufs *split = nullptr;
   if ((rc = split_for(ctx, kFactorFP64, maxN, ld, nw, &split))) return rc;
-  CK(launch_inverse(ctx->d_jobs, nw, maxn, maxN, split, ctx->d_err, ctx->stream, &ctx->launches));
+  CK(launch_inverse(ctx->d_jobs, nw, ctx->la.min_n, maxn, maxN, split, ctx->d_err, ctx->stream, &ctx->launches));
   CK(launch_vjp_assemble(ctx->d_jobs, nw, maxL, ctx->kkrsz, ctx->ns, ctx->stream, &ctx->launches));
   return B200TAU_OK;
 }
@@ -1708,6 +1708,7 @@ int b200tau_solve_dense(b200tau_ctx *ctx, const double *m, int n, int ldm, const
   CK(cudaMemcpyAsync(ctx->d_jobs, &J, sizeof(J), cudaMemcpyHostToDevice, ctx->stream));
   if ((rc = reset_slot_status(ctx, 1))) return rc;
   ctx->launches = 0;
+  ctx->la.min_n = r;
   if ((rc = run_pipeline(ctx, std::vector<JobDev>{J}, 1, r, n, ld, 1, b, b, p, panel))) return rc;
   int info = 0;
   CK(cudaMemcpyAsync(&info, ctx->d_info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1827,9 +1828,10 @@ static int solve_tau_full(b200tau_ctx *ctx, const b200tau_job *job, double *tau_
   if ((rc = reset_slot_status(ctx, 1))) return rc;
   ctx->launches = 0;
   CK(launch_kkr_build(ctx->d_jobs, 1, a.L, build_params(ctx, p), ctx->d_err, ctx->stream, &ctx->launches));
+  ctx->la.min_n = J.n;
   CK(launch_eliminate(kFactorFP64, ctx->d_jobs, 1, J.n, J.N, ctx->d_info, ctx->stream, &ctx->launches, nullptr,
                       nullptr, ctx->d_err, false, &ctx->la, panel, split));
-  CK(launch_inverse(ctx->d_jobs, 1, J.n, J.N, split, ctx->d_err, ctx->stream, &ctx->launches));
+  CK(launch_inverse(ctx->d_jobs, 1, J.n, J.n, J.N, split, ctx->d_err, ctx->stream, &ctx->launches));
   CK(launch_tau_full(ctx->d_jobs, 1, a.L, a.N, tmat_view(ctx), rows, ctx->stream, &ctx->launches));
   CK(cudaMemcpyAsync(tau_full, J.M, sizeof(double2) * n * n, cudaMemcpyDeviceToHost, ctx->stream));
   int info = 0;

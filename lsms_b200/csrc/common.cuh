@@ -210,14 +210,19 @@ constexpr int kSplitCounters = 3;  // elimination, inverse lower pass, inverse u
 constexpr size_t split_slot_bytes(int ld) {
   return (size_t)ld * (3 * kSplitDigits * kSplitRowBytes + 2 * sizeof(double)) + kNb * sizeof(int);
 }
-// The integer tensor cores take an FP64 update of at least kSplitMin rows and columns and kSplitElems
-// elements of C over the wave: the packs and the fill of the pipeline cost some 35 us a launch, which the
-// faster products (30 against 47 TF/s) save from about 5 M elements on (a 64-column step; 31 jobs:
-// 400 x 400; one job of N = 2160 stays on the FP64 tensor cores).
+// The integer tensor cores take a job's FP64 update of at least kSplitMin rows and columns and `elems`
+// elements.  The rule asks about the job alone, so that its results do not depend on the jobs that share its
+// wave.  Where the lines lie: the packs and the fill of the pipeline cost some 35 us a launch, against
+// products at 47 instead of 30 TF/s.  In the elimination that time hides behind the next diagonal inverse:
+// from 384 x 384 on, 64 jobs of N = 688 to 2160 take 16.2 ms (16.6 from 512 x 512, 17.7 from 886 x 886) and
+// 31 of N = 2160 25.0 (30 without); a job of N = 2160 alone loses by any line (2.98 -> 3.08 ms).  In the
+// inverse's passes it does not: those of a single job of N = 880 stay below their line, those of 16 jobs of
+// N = 1392 gain above it (a gradient call 23.0 -> 22.3 ms from 1024 x 1024 to 640 x 640).
 constexpr int kSplitMin = 256;
-constexpr long kSplitElems = 5L << 20;
-constexpr bool split_pays(int m, int n, int njobs) {
-  return m >= kSplitMin && n >= kSplitMin && (long)m * n * njobs >= kSplitElems;
+constexpr int kSplitSide = 384;
+constexpr long kSplitTrailing = (long)kSplitSide * kSplitSide, kSplitInverse = 768L * 1024;
+__host__ __device__ constexpr bool split_pays(int m, int n, long elems) {
+  return m >= kSplitMin && n >= kSplitMin && (long)m * n >= elems;
 }
 // A second stream and two events for the elimination's look-ahead (all null: none).
 struct Lookahead {
@@ -342,8 +347,9 @@ cudaError_t launch_tau_full(const JobDev *jobs, int njobs, int max_L, int max_N,
                             cudaStream_t s, long *launches);
 // Adjoint (adjoint.cu), FP64 factors: V = M^-1 from the block factors in F, then per LIZ site the
 // tau00 cotangent pull-back and d ln det M / d t (needs G in M, X refined, V).
-cudaError_t launch_inverse(const JobDev *jobs, int njobs, int max_n, int max_N, const SplitBufs *split, int *err,
-                           cudaStream_t s, long *launches);
+// `min_n`: the smallest n of the jobs.
+cudaError_t launch_inverse(const JobDev *jobs, int njobs, int min_n, int max_n, int max_N, const SplitBufs *split,
+                           int *err, cudaStream_t s, long *launches);
 cudaError_t launch_vjp_assemble(const JobDev *jobs, int njobs, int max_L, int kkrsz, int ns, cudaStream_t s,
                                 long *launches);
 

@@ -70,6 +70,14 @@ struct View {
   int lda, ldb, ldc, m, n, K;
 };
 
+// Op's view where the integer tensor cores take it: at least ELEMS elements (split_pays).
+template <class Op, long ELEMS>
+struct Large {
+  __device__ bool operator()(const JobDev &J, int k, View &g) const {
+    return Op()(J, k, g) && split_pays(g.m, g.n, ELEMS);
+  }
+};
+
 struct __align__(1024) Smem {
   signed char a[kDigits][kABytes];
   signed char b[kStages][kDigits * kBBytes];

@@ -51,27 +51,26 @@ def _close(a, b):
 @pytest.mark.gpu
 def test_planes_that_find_no_room():
     """A wave whose planes do not fit runs without them, and a smaller one still uses the planes it had."""
-    w = _Waves((2, 5, 6), 16)  # N = 304, 1264, 1392
+    w = _Waves((2, 5), 16)  # N = 304, 1264
     try:
-        want_big = w.solve(6, 4)[0]
+        want_big = w.solve(5, 8)[0]
         want, launches = w.solve(5, 4)
     finally:
         w.s.close()
-    w = _Waves((2, 5, 6), 16)
+    w = _Waves((2, 5), 16)
     held = []
     try:
-        first, count = w.solve(5, 4)  # 4 x 1264^2 elements: planes for four slots
+        first, count = w.solve(5, 4)  # planes for four slots
         assert count == launches
-        w.solve(2, 16)                # sixteen slots, too few elements for planes
-        w.solve(6, 2)                 # a larger leading dimension, too few elements
-        held = _hog(32 * MB)          # the planes of sixteen slots take 63 MB or more
+        w.solve(2, 16)                # sixteen slots, but updates too small for planes
+        held = _hog(32 * MB)          # the planes of sixteen slots take 63 MB
         for _ in range(3):
-            assert _close(w.solve(6, 4)[0], want_big)
+            assert _close(w.solve(5, 8)[0], want_big)
         again, count = w.solve(5, 4)
         assert count == launches      # (a wave on the FP64 tensor cores alone takes fewer launches)
         assert np.array_equal(again, want) and np.array_equal(first, want)
         _release(held)
-        got, _ = w.solve(6, 4)
+        got, _ = w.solve(5, 8)
         assert np.array_equal(got, want_big)
     finally:
         w.s.close()
@@ -87,8 +86,9 @@ def test_waves_do_not_depend_on_the_planes_held():
     try:
         w.solve(6, 1)  # what a context allocates besides the wave's slots
         ld = 1408
-        slot = 32 * ld * ld + 3 * ld * 32 * 16 + ld * (3 * 8 * 128 + 16) + 256
-        held = _hog(2 * 6.16 * slot - 32 * ld * ld)  # six slots and a sixth (one is held)
+        planes = ld * (3 * 8 * 128 + 16) + 256
+        slot = 32 * ld * ld + 3 * ld * 32 * 16 + planes
+        held = _hog(2 * 6.16 * slot - 32 * ld * ld - planes)  # six slots and a sixth (one is held)
         counts = [w.solve(6, 16)[1] for _ in range(3)]
         assert len(set(counts)) == 1
     finally:

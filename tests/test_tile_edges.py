@@ -163,10 +163,9 @@ def test_build_non_collinear_t(solver_factory, outer, coupled):
 @pytest.mark.gpu
 @pytest.mark.parametrize("n_reduced", [0, 3, 10])
 def test_updates_by_digit_products(solver_factory, n_reduced):
-    """32 jobs of N = 816 and less: the steps with enough elements run on the integer tensor cores, their
+    """32 jobs of N = 816 and less: the steps with enough rows run on the integer tensor cores, their
     row panels, column tiles and the first block that the look-ahead takes out ending anywhere.  Against
-    the oracle, and against each job alone, which stays on the FP64 tensor cores; the gradients likewise
-    (the inverse's two passes)."""
+    the oracle, in the batch and alone; the gradients likewise (the inverse's two passes)."""
     from oracle import port
     njobs = 32
     L = W.lattice_shells("bcc", 5.42, 4).shape[1]
@@ -190,8 +189,8 @@ def test_updates_by_digit_products(solver_factory, n_reduced):
         _, tb1, ld1 = s.solve_vjp(T.make_jobs(specs[i:i + 1]), bar[i:i + 1], [prob.num_liz])
         assert np.abs(tb[i] - tb1[0]).max() <= 10 * bound * np.abs(tb1[0]).max()
         # d ln det M comes from the unrefined inverse, whose error is that of the block LU (pivots inside
-        # the diagonal blocks).  Against -((G M^-1)_jj)^T with t_j (G M^-1)_jj = (M^-1 - 1)_jj: the digits
-        # may not add to the error of the FP64 products, but for the spread of two such roundings.
+        # the diagonal blocks): up to 9 times cond(M) 2^-53 here, by digits as by FP64 products.  Against
+        # -((G M^-1)_jj)^T with t_j (G M^-1)_jj = (M^-1 - 1)_jj.
         inv = np.linalg.inv(port.build_kkr(prob, i))
         off = np.concatenate([[0], np.cumsum((lmax + 1) ** 2)])
         err = [0.0, 0.0]
@@ -201,6 +200,7 @@ def test_updates_by_digit_products(solver_factory, n_reduced):
             want = -np.linalg.solve(t, inv[off[j]:off[j + 1], off[j]:off[j + 1]] - np.eye(k)).T
             err = [max(e, np.abs(d[j][:k, :k] - want).max()) for e, d in zip(err, (ld[i], ld1[0]))]
         assert err[0] <= 8 * err[1] + 10 * bound * np.abs(ld1[0]).max()
+        assert err[0] <= 32 * np.linalg.cond(port.build_kkr(prob, i)) * 2.0 ** -53 * np.abs(ld1[0]).max()
 
 
 @pytest.mark.gpu
@@ -241,6 +241,11 @@ def _register(s, shells, energies, cant=1, seed=17):
 @pytest.mark.gpu
 @pytest.mark.parametrize("shells,cant,nen,pivoting", [
     ((2,), 1, 40, T.PIVOT_BLOCK),           # N = 304: the residual's split
+    ((7,), 1, 5, T.PIVOT_BLOCK),            # N = 2160, 688: digit products and FP64 tensor cores
+    ((3,), 1, 33, T.PIVOT_BLOCK),
+    ((5, 6, 3, 4), 1, 5, T.PIVOT_BLOCK),    # N = 1264, 1392, 688, 880 in one wave
+    ((5, 6, 3), 1, 3, T.PIVOT_PANEL),       # row moves between digit products
+    ((3, 2), 2, 4, T.PIVOT_BLOCK),          # b = 32, N = 1376 and 608
 ])
 def test_fp64_results_do_not_depend_on_the_batch(solver_factory, shells, cant, nen, pivoting):
     """Every job of a batch, bit for bit the result of the job alone, and against the oracle."""
@@ -259,3 +264,92 @@ def test_fp64_results_do_not_depend_on_the_batch(solver_factory, shells, cant, n
     for a in range(len(shells) if len(shells) > 1 else 0):
         bound = max(1e-12, 8 * np.linalg.cond(port.build_kkr(probs[a], 1)) * 2.0 ** -53)
         assert _tau_err(probs[a], 1, out[len(shells) + a]) <= bound
+
+
+@pytest.mark.gpu
+def test_gradients_do_not_depend_on_the_batch(solver_factory):
+    """The inverse's passes on both sides of the digit products' line, uneven sizes in one wave."""
+    s = solver_factory(3, 1, 1)
+    energies = W.semicircle_contour(-0.2, 0.7, 3)
+    probs = _register(s, (3, 6, 5), energies)
+    specs = [(a, i, 0, e) for i, e in enumerate(energies) for a in range(3)]
+    num = [probs[a].num_liz for a, _, _, _ in specs]
+    rng = np.random.default_rng(4)
+    bar = rng.normal(size=(9, 16, 16)) + 1j * rng.normal(size=(9, 16, 16))
+    tau, tb, dl = s.solve_vjp(T.make_jobs(specs), bar, num)
+    for j, spec in enumerate(specs):
+        t1, tb1, dl1 = s.solve_vjp(T.make_jobs([spec]), bar[j:j + 1], num[j:j + 1])
+        assert np.array_equal(tau[j], t1[0]) and np.array_equal(tb[j], tb1[0]) and np.array_equal(dl[j], dl1[0])
+
+
+@pytest.mark.gpu
+def test_digit_products_are_taken(solver_factory):
+    """A 64-column step that leaves at least 384 rows updates them by digit products: four launches
+    instead of one."""
+    s = solver_factory(3, 1, 1)
+    energies = W.semicircle_contour(-0.2, 0.7, 2)
+    probs = _register(s, (3, 5, 7), energies)
+    count = []
+    for a, p in enumerate(probs):
+        s.solve_jobs(T.make_jobs([(a, i, 0, e) for i, e in enumerate(energies)]), T.PREC_FP64)
+        steps = [p.nrmat_ns - k - 64 for k in range(0, p.nrmat_ns - 16, 64)]
+        # W, the next diagonal block, its inverse and the update for every step but the last
+        count.append((s.last_launch_count, 4 * len(steps) + 3 * sum(m >= 384 for m in steps)))
+    assert count[1][0] - count[0][0] == count[1][1] - count[0][1]
+    assert count[2][0] - count[0][0] == count[2][1] - count[0][1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("s", [0, 25, 60])
+def test_balance_of_the_inner_indices(solver_factory, s):
+    """The first block's rows and columns scaled against each other by 2^s and 2^-s in turn, which leaves
+    tau00 as it is.  Digits scaled by row and by column alone would keep 62 - 2 s bits of the small half
+    of the operands."""
+    rng = np.random.default_rng(s)
+    n, b = 1040, 16
+    m = np.eye(n) + 0.3 / np.sqrt(n) * (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n)))
+    first = slice(b, b + 64)  # the rows eliminated first
+    m[first, first] = np.eye(64)
+    t0 = rng.normal(size=(b, b)) + 1j * rng.normal(size=(b, b))
+    rhs = np.zeros((n, b), np.complex128)
+    rhs[:b] = t0
+    want = np.linalg.solve(m, rhs)[:b]
+    e = np.zeros(n, np.int64)
+    e[first] = np.where(np.arange(64) % 2 == 0, s, -s)
+    f = np.ldexp(1.0, e)
+    x = solver_factory(3, 1, 1)
+    x.set_refinement(T.PREC_FP64, 0)
+    try:
+        got = x.solve_tau00_dense(m * f[:, None] / f[None, :], t0, T.PREC_FP64)
+    finally:
+        x.set_refinement(T.PREC_FP64, 1)
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+def test_panel_pivoting_with_digit_products(solver_factory):
+    """Rows in random order at a size whose first steps take the digit products."""
+    m, t0, want = _dense(16 + 1101, 16, 7, shuffle=True)
+    s = solver_factory(3, 1, 1)
+    s.set_pivoting(T.PIVOT_PANEL)
+    try:
+        got = s.solve_tau00_dense(m, t0, T.PREC_FP64)
+    finally:
+        s.set_pivoting(T.PIVOT_AUTO)
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,rest", [(32, 321), (32, 700), (9, 321), (16, 65)])
+def test_accelerated_rounds_of_an_ill_conditioned_matrix(solver_factory, b, rest):
+    """Condition number 1e5: several accelerated rounds, odd N and 32 columns among them."""
+    n = b + rest
+    rng = np.random.default_rng(n)
+    q = [np.linalg.qr(rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n)))[0] for _ in range(2)]
+    m = (q[0] * np.logspace(0, -5, n)) @ q[1]
+    t0 = rng.normal(size=(b, b)) + 1j * rng.normal(size=(b, b))
+    rhs = np.zeros((n, b), np.complex128)
+    rhs[:b] = t0
+    want = np.linalg.solve(m, rhs)[:b]
+    got = solver_factory(3, 1, 1).solve_tau00_dense(m, t0, T.PREC_MIXED)
+    assert np.abs(got - want).max() <= TOL_MIXED * np.abs(want).max()
