@@ -939,8 +939,9 @@ cudaError_t eliminate_lookahead(const JobDev *jobs, int njobs, int max_n, int ma
       k = k2;  // the loop's increment moves past k2
       continue;
     }
-    // (only where step k2 is a full block of every job: in a wave of 1392 and 2160 a pair whose second step
-    // was the smaller jobs' last, partial one left their factors too poor to refine)
+    // (only where step k2 is a full block of every job: the strips below apply step k to 64 columns and
+    // rows from k2 on, and the combined pass starts behind step k2's own block, so after a partial block of
+    // kb2 the last 64 - kb2 of them would have step k subtracted twice)
     if (!panel && la.pair_min_rest > 0 && k2 + kNb <= la.min_n && k2 + kNb < max_n &&
         max_N - k2 - kNb >= la.pair_min_rest) {
       const int tiles2 = (max_N - k2 - 1 + kTile - 1) / kTile;

@@ -353,3 +353,25 @@ def test_accelerated_rounds_of_an_ill_conditioned_matrix(solver_factory, b, rest
     want = np.linalg.solve(m, rhs)[:b]
     got = solver_factory(3, 1, 1).solve_tau00_dense(m, t0, T.PREC_MIXED)
     assert np.abs(got - want).max() <= TOL_MIXED * np.abs(want).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pivoting", [T.PIVOT_BLOCK, T.PIVOT_PANEL])
+@pytest.mark.parametrize("min_rest", [1, 512])
+def test_paired_steps_of_uneven_waves(solver_factory, min_rest, pivoting):
+    """Mixed waves whose smaller jobs end in a partial block at what would be a pair's second step (N = 1392
+    beside 2160: n = 21 x 64 + 32): every job refines, and to the FP64 result."""
+    s = solver_factory(3, 1, 1)
+    energies = W.semicircle_contour(-0.2, 0.7, 4)
+    _register(s, (6, 7, 4), energies)
+    jobs = T.make_jobs([(a, i, 0, e) for i, e in enumerate(energies) for a in range(3)])
+    want = s.solve_jobs(jobs, T.PREC_FP64)
+    s.set_pivoting(pivoting)
+    s.set_paired_steps(min_rest)
+    try:
+        got = s.solve_jobs(jobs, T.PREC_MIXED)
+        assert s.last_fallback_count == 0
+    finally:
+        s.set_paired_steps(768)
+        s.set_pivoting(T.PIVOT_AUTO)
+    assert np.all(np.abs(got - want).max(axis=1) <= TOL_MIXED * np.abs(want).max(axis=1))
