@@ -13,6 +13,8 @@ reference's own KKR matrix:
 * central finite differences of the reference's own tau00 (calculateTauMatrix with the block-LU
   solver) re-solved at delta +/- eps, and of ln det of the reference's own M.
 
+Where the compiled reference is not there, both take M and tau00 from its restatement (port.py) instead.
+
 Phase-shift t-matrices (t_l = -(1/kappa) sin d_l e^{i d_l}, the workloads' recipe for collinear
 sites) give dt_l / d d_l = -(1/kappa) e^{2 i d_l} = -(1/kappa) (1 - 2 i kappa t_l), so the
 directional derivatives need only t itself.
@@ -24,7 +26,17 @@ import copy
 
 import numpy as np
 
-from . import reflib
+from . import port, reflib
+
+
+def _build(prob, iie: int, ispin: int) -> np.ndarray:
+    return (reflib if reflib.available() else port).build_kkr(prob, iie, ispin)
+
+
+def _tau(prob, iie: int, ispin: int) -> np.ndarray:
+    if reflib.available():
+        return reflib.calculate_tau(prob, iie, ispin, reflib.ZBLOCKLU_CPP)
+    return port.solve(prob, iie, ispin)
 
 
 class Bicomplex:
@@ -87,7 +99,7 @@ def structure_constants(prob, iie: int, ispin: int = 0) -> np.ndarray:
     p.tmat_store[:, :, :b * b] = eye
     if p.n_spin_pola != p.n_spin_cant:
         p.tmat_store[:, :, b * b:2 * b * b] = eye
-    return np.eye(prob.nrmat_ns, dtype=np.complex128) - reflib.build_kkr(p, iie, ispin)
+    return np.eye(prob.nrmat_ns, dtype=np.complex128) - _build(p, iie, ispin)
 
 
 def site_layout(prob):
@@ -166,9 +178,9 @@ def finite_difference(prob, iie: int, taubar: np.ndarray, site: int, l: int, isp
             delta = np.angle(1.0 - 2j * kappa * t) / 2.0 + sign * eps
             blk[k + k * b] = -(1.0 / kappa) * np.sin(delta) * np.exp(1j * delta)
         p.tmat_store[store, iie] = blk
-        tau = reflib.calculate_tau(p, iie, ispin, reflib.ZBLOCKLU_CPP).reshape(b, b).T
+        tau = _tau(p, iie, ispin).reshape(b, b).T
         tau = tau + p.t_block(int(p.liz_store_idx[0]), iie, ispin)
-        sign_, ld = np.linalg.slogdet(reflib.build_kkr(p, iie, ispin))
+        sign_, ld = np.linalg.slogdet(_build(p, iie, ispin))
         return np.sum(taubar * tau), np.log(sign_) + ld
 
     (lp, dp), (lm, dm) = at(+1), at(-1)

@@ -43,6 +43,17 @@ def test_complex_step_agrees_with_reference_finite_differences(ref):
         assert abs(dd - fd) <= TOL_FD * max(abs(dd), 1e-3), (site, l, dd, fd)
 
 
+def test_complex_step_agrees_with_finite_differences():
+    """The same wherever the tests run: without the compiled reference, on its restatement."""
+    prob = _problem_small(5)
+    rng = np.random.default_rng(4)
+    tb = rng.normal(size=(16, 16)) + 1j * rng.normal(size=(16, 16))
+    for (site, l), (dl, dd) in zip([(0, 1), (9, 2)], A.complex_step(prob, 1, tb, [(0, 1), (9, 2)])):
+        fl, fd = A.finite_difference(prob, 1, tb, site, l)
+        assert abs(dl - fl) <= TOL_FD * abs(dl), (site, l, dl, fl)
+        assert abs(dd - fd) <= TOL_FD * max(abs(dd), 1e-3), (site, l, dd, fd)
+
+
 def test_bicomplex_solve_is_exact_arithmetic():
     rng = np.random.default_rng(5)
     a = rng.normal(size=(6, 6)) + 1j * rng.normal(size=(6, 6)) + 4 * np.eye(6)
