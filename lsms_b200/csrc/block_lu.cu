@@ -82,10 +82,13 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
   // four steps) hit eight 16-byte banks
   __shared__ double2 Us[NB][12];
   __shared__ int s_sing;
-  __shared__ int s_pv[NB], s_inv[NB];
+  __shared__ int s_pv[NB], s_inv[NB], s_hi[kDiagThreads / 32];
   T *__restrict__ Fk = static_cast<T *>(J.F) + (size_t)k + (size_t)k * J.ld;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   constexpr int kPer = NB * NB / kDiagThreads;  // entries per thread of a full block
+  // the block is inverted times a power of two that brings its largest element to 1 .. 2: the squares of
+  // its pivots stay in range, and 1 - 1/d does not lose the digits of a large d
+  double scale;
   {
     // all of a thread's loads in flight at once (a loop over them waits out one DRAM round trip
     // per entry)
@@ -93,12 +96,24 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       const int e = tid + i * kDiagThreads, r = e % NB, c = e / NB;
-      v[i] = r < kb && c < kb ? ldc(Fk + r + (size_t)c * J.ld) : make_double2(r == c ? 1.0 : 0.0, 0.0);
+      v[i] = r < kb && c < kb ? ldc(Fk + r + (size_t)c * J.ld) : make_double2(0.0, 0.0);
     }
+    int hi = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+      hi = max(hi, max(__double2hiint(v[i].x) & 0x7fffffff, __double2hiint(v[i].y) & 0x7fffffff));
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (l == 0) s_hi[w] = hi;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kDiagThreads / 32; ++i) hi = max(hi, s_hi[i]);
+    const int e2 = hi >> 20;  // (0x7ff: an element is not finite)
+    scale = e2 == 0x7ff ? 1.0 : __hiloint2double(max(1, 2046 - e2) << 20, 0);
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const int e = tid + i * kDiagThreads;
-      As[e / NB][e % NB] = v[i];
+      const int e = tid + i * kDiagThreads, r = e % NB, c = e / NB;
+      As[c][r] = r < kb && c < kb ? make_double2(v[i].x * scale, v[i].y * scale)
+                                  : make_double2(r == c ? 1.0 : 0.0, 0.0);
     }
   }
   if (tid < NB) s_pv[tid] = s_inv[tid] = tid;  // every entry in range whatever the pivots
@@ -212,7 +227,10 @@ __global__ void __launch_bounds__(kDiagThreads, PER_SM) diag_inverse_kernel(cons
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
     const int e = tid + i * kDiagThreads, r = e % NB, c = e / NB;
-    if (r < kb && c < kb) stc(Fk + r + (size_t)c * J.ld, As[s_inv[c]][s_pv[r]]);
+    if (r < kb && c < kb) {
+      const double2 v = As[s_inv[c]][s_pv[r]];
+      stc(Fk + r + (size_t)c * J.ld, make_double2(v.x * scale, v.y * scale));
+    }
   }
   if (s_sing && tid == 0) atomicCAS(&info[blockIdx.x], 0, k + 1);
 }

@@ -25,22 +25,18 @@ __device__ __forceinline__ double2 crecip(double2 a) {
   const double d = ar * ar + ai * ai;
   return make_double2(ar / (d * s), -ai / (d * s));
 }
-// 1 / d = conj(d) / |d|^2; 0 for a zero, NaN for an infinity or a NaN.  d is first scaled by a power of two,
-// so that |d|^2 is between 1 and 8 and neither it nor its reciprocal leaves the normal range (one FP64 solve
-// of N = 2160 takes 3.00 ms with the scaling, 2.98 without).  The reciprocal is Newton's iteration r <- r + r (1 - q r) from the hardware's 20-bit approximation (2^-20,
-// 2^-40, 2^-80 before rounding), without the branches of a division, which kept the compiler from filling
-// the diagonal inverse's chain with the rest of its update (180 cycles a step).
+// 1 / d = conj(d) / |d|^2 for |d|^2 in FP64's normal range (a block's pivots, scaled with it); 0 for a zero,
+// NaN for an infinity or a NaN.  1 / |d|^2 is Newton's iteration r <- r + r (1 - q r) from the hardware's 20-bit
+// approximation (2^-20, 2^-40, 2^-80 before rounding), without the branches of a division, which kept the
+// compiler from filling the diagonal inverse's chain with the rest of its update (180 cycles a step).
+// (Scaling every pivot here cost 3 us of the inverse's 33.)
 __device__ __forceinline__ double2 reciprocal(double2 d) {
-  const int h = max(__double2hiint(d.x) & 0x7fffffff, __double2hiint(d.y) & 0x7fffffff);
-  const double sc = __hiloint2double(max(1, 2046 - (h >> 20)) << 20, 0);  // 2^-e of the larger part
-  const double x = d.x * sc, y = d.y * sc;
-  const double q = x == 0.0 && y == 0.0 ? 1.0 : x * x + y * y;
+  const double q = d.x == 0.0 && d.y == 0.0 ? 1.0 : d.x * d.x + d.y * d.y;
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(q));
   r = fma(r, fma(-q, r, 1.0), r);
   r = fma(r, fma(-q, r, 1.0), r);
-  r *= sc;
-  return make_double2(x * r, -y * r);
+  return make_double2(d.x * r, -d.y * r);
 }
 // Loads and stores of the factor storage (FP64 or FP32), arithmetic in FP64.
 __device__ __forceinline__ double2 ldc(const double2 *p) { return *p; }

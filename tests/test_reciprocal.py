@@ -1,4 +1,4 @@
-"""The reciprocal of the elimination's pivots (lsms_b200/csrc/cplx.cuh) over the whole exponent range."""
+"""The reciprocal of the elimination's pivots (lsms_b200/csrc/cplx.cuh), and diagonal blocks of any scale."""
 
 import ctypes
 import subprocess
@@ -52,10 +52,11 @@ def run(tmp_path_factory):
 
 
 @pytest.mark.gpu
-def test_reciprocal_over_the_exponent_range(run):
+def test_reciprocal_over_its_range(run):
+    """Squares between 2^-1020 and 2^1020."""
     rng = np.random.default_rng(0)
     n = 200000
-    e = rng.integers(-1022, 1022, size=n)
+    e = rng.integers(-510, 509, size=n)
     x, y = rng.uniform(1.0, 2.0, size=(2, n)) * rng.choice([-1.0, 1.0], size=(2, n))
     other = np.where(rng.random(n) < 0.8, rng.integers(0, 4, size=n), rng.integers(0, 1000, size=n))
     a, b = np.ldexp(x, e), np.ldexp(y, np.maximum(e - other, -1074))
@@ -65,28 +66,23 @@ def test_reciprocal_over_the_exponent_range(run):
     xl, yl = d.real.astype(np.longdouble), d.imag.astype(np.longdouble)
     q = xl * xl + yl * yl
     size = 1 / np.sqrt(q)
-    # the sum of squares is off by at most 2 u, its reciprocal by 1.5 u more, each product by u (u = 2^-53); a
-    # result below 2^-1022 also by half its last place, 2^-1075
+    # the sum of squares is off by at most 2 u, its reciprocal by 1.5 u more, each product by u (u = 2^-53)
     for got, bound in ((ours.real - xl / q, 5), (ours.imag + yl / q, 5), (ours - div, 5)):
-        assert np.all(np.abs(got) <= bound * 2.0 ** -53 * size + 2.0 ** -1074)
+        assert np.all(np.abs(got) <= bound * 2.0 ** -53 * size)
 
 
 @pytest.mark.gpu
 def test_reciprocal_of_special_values(run):
-    tiny, top = 2.0 ** -1022, np.finfo(np.float64).max
-    d = np.array([0.0, -0.0, complex(np.inf, 1.0), complex(1.0, -np.inf), complex(np.nan, 1.0), complex(tiny, tiny),
-                  complex(1e-162, 0.0), complex(0.0, 1e-200), complex(top, -top), complex(7e153, 0.0)])
+    d = np.array([0.0, -0.0, complex(np.inf, 1.0), complex(1.0, -np.inf), complex(np.nan, 1.0)])
     got = run(d)[0]
     assert np.all(got[:2] == 0)
-    assert np.all(np.isnan(got[2:5].real) & np.isnan(got[2:5].imag))
-    want = 1 / d[5:].astype(np.clongdouble)
-    assert np.all(np.abs(got[5:] - want) <= 5 * 2.0 ** -53 * np.abs(want) + 2.0 ** -1074)
+    assert np.all(np.isnan(got[2:].real) & np.isnan(got[2:].imag))
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("scale", [1e-170, 1e-154, 1.2e-154, 1e-100])
-def test_pivots_with_squares_out_of_range(solver_factory, scale):
-    """Pivots whose squares underflow or are subnormal are neither lost nor reported as singular."""
+@pytest.mark.parametrize("scale", [1e-300, 1e-170, 1e-154, 1.2e-154, 1e-100, 1e10])
+def test_matrices_of_any_scale(solver_factory, scale):
+    """Pivots whose squares leave the range are neither lost nor reported as singular."""
     from lsms_b200 import tau as T
     rng = np.random.default_rng(5)
     n = 96
