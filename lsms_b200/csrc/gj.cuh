@@ -45,14 +45,29 @@ __device__ __forceinline__ double2 cfnma(double2 x, double2 g, double2 u) {
 __device__ inline bool gj_solve_smem(double2 (*A)[2 * kMaxB + 1], int b) {
   __shared__ double2 s_g[2][32];
   __shared__ double2 s_row[8][8];
-  __shared__ int s_pv[2], s_inv[32], s_sing;
+  __shared__ int s_pv[2], s_inv[32], s_hi[8], s_sing;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   double2 a[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) a[j] = (l < b && 8 * w + j < 2 * b) ? A[l][8 * w + j] : make_double2(0.0, 0.0);
   if (tid < 32) s_inv[tid] = tid;
   if (tid == 0) s_sing = 0;
+  // A is taken times a power of two that brings its largest element to 1 .. 2: 1 - 1/d would lose the digits
+  // of a large d
+  int hi = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (8 * w + j < b) hi = max(hi, max(__double2hiint(a[j].x) & 0x7fffffff, __double2hiint(a[j].y) & 0x7fffffff));
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (l == 0) s_hi[w] = hi;
   __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) hi = max(hi, s_hi[i]);
+  const int e2 = hi >> 20;  // (0x7ff: an element is not finite)
+  const double scale = e2 == 0x7ff ? 1.0 : __hiloint2double(max(1, 2046 - e2) << 20, 0);
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (8 * w + j < b) a[j] = make_double2(a[j].x * scale, a[j].y * scale);
   bool used = l >= b;
   auto search = [&](double2 x, int p) {
     const double v = cabs1(x);
@@ -99,7 +114,7 @@ __device__ inline bool gj_solve_smem(double2 (*A)[2 * kMaxB + 1], int b) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int c = 8 * w + ((j + b) & 7);
-    if (l < b && c >= b && c < 2 * b) A[s_inv[l]][c] = a[j];
+    if (l < b && c >= b && c < 2 * b) A[s_inv[l]][c] = make_double2(a[j].x * scale, a[j].y * scale);
   }
   __syncthreads();
   return s_sing != 0;

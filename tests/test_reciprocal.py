@@ -80,7 +80,7 @@ def test_reciprocal_of_special_values(run):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("scale", [1e-300, 1e-170, 1e-154, 1.2e-154, 1e-100, 1e10])
+@pytest.mark.parametrize("scale", [1e-300, 1e-170, 1e-154, 1.2e-154, 1e-100, 1e10, 1e20, 7e153, 1e200])
 def test_matrices_of_any_scale(solver_factory, scale):
     """Pivots whose squares leave the range are neither lost nor reported as singular."""
     from lsms_b200 import tau as T
@@ -93,3 +93,22 @@ def test_matrices_of_any_scale(solver_factory, scale):
     want = np.linalg.solve(m / scale, rhs / scale)[:16]
     got = solver_factory(3, 1, 1).solve_tau00_dense(m, t0, T.PREC_FP64)
     assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec,tol", [(0, 1e-12), (1, 1e-10)])
+@pytest.mark.parametrize("scale", [1e-12, 1e6, 1e12])
+@pytest.mark.parametrize("b", [9, 32])
+def test_central_block_of_any_scale(solver_factory, b, scale, prec, tol):
+    """The central site's rows and t0 scaled together leave tau00 as it is: the solve with the b x b Schur
+    complement keeps its digits."""
+    rng = np.random.default_rng(b)
+    n = b + 150
+    m = np.eye(n) + 0.03 * (rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n)))
+    t0 = rng.normal(size=(b, b)) + 1j * rng.normal(size=(b, b))
+    rhs = np.zeros((n, b), np.complex128)
+    rhs[:b] = t0
+    want = np.linalg.solve(m, rhs)[:b]
+    m[:b] *= scale
+    got = solver_factory(3, 1, 1).solve_tau00_dense(m, t0 * scale, prec)
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()
