@@ -106,8 +106,10 @@ int b200tau_set_atom(b200tau_ctx *ctx, int atom, int num_liz,
  * system).  Defaults: FP64 1 step, MIXED 10 steps, of which each job runs only as many as it
  * needs: after every step, a job whose estimated remaining error (the relative size c of the
  * correction just applied times its contraction c / c_previous) is below 1e-12 of tau00 stops.
- * A MIXED job whose corrections stop shrinking, or that has not converged after the last step,
- * is re-solved by FP64 block LU (b200tau_last_fallback_count).  FP64 with 0 steps takes tau00
+ * With more than two MIXED steps they are accelerated (Anderson, depth 2); these stop at 2e-13, the
+ * contraction being the larger of the last two, or at a correction below 1e-12 that shrinks no more.
+ * A MIXED job whose corrections stop shrinking or are not finite, or that has not converged after the
+ * last step, is re-solved by FP64 block LU (b200tau_last_fallback_count).  FP64 with 0 steps takes tau00
  * directly from the Schur complement like zblock_lu. */
 int b200tau_set_refinement(b200tau_ctx *ctx, int prec, int steps);
 
@@ -121,7 +123,9 @@ int b200tau_set_mixed_sweep(b200tau_ctx *ctx, int sweep);
 /* Solve `njobs` (atom, energy, spin) problems in one batched device pass and
  * write each job's tau00_l (kkrsz_ns^2 complex, the layout calculateTauMatrix
  * writes through its tau00_l argument) to host memory at
- * tau00_l + 2 * kkrsz_ns^2 * j.  `prec` is B200TAU_PREC_*. */
+ * tau00_l + 2 * kkrsz_ns^2 * j.  `prec` is B200TAU_PREC_*.
+ * A PREC_FP64 job's result is bit for bit the same alone and in any batch, as long as the workspace of the
+ * integer tensor-core updates (about 3 KB per row of a job) finds room on the device. */
 int b200tau_solve(b200tau_ctx *ctx, const b200tau_job *jobs, int njobs,
                   int prec, double *tau00_l);
 

@@ -322,7 +322,7 @@ cudaError_t launch_sweep(FactorKind fk, const JobDev *jobs, int njobs, int b, in
 // to work (the others leave at once), which sizes the clusters.
 cudaError_t launch_sweep64(FactorKind fk, const JobDev *jobs, int njobs, int b, bool forward, int mode, int want,
                            cudaStream_t s);
-// The dataflow sweeps for FP32 factors in FP32 arithmetic with b <= 16 (sweep_flow.cu), operand
+// The dataflow sweeps for FP32 factors in FP32 arithmetic (sweep_flow.cu; 16 columns per cluster), operand
 // units loaded through `fmap` (TcMaps::tFu over the jobs' factor slots).  Sets *launched when it
 // took the launch; false (and cudaSuccess) without a map or when the shape does not fit its
 // shared-memory layout, and the caller runs launch_sweep's step-synchronous kernels instead.

@@ -14,7 +14,8 @@
 // out.  On updates of KKR matrices (fcc, 43 sites) with energies on a contour from -0.3 to 0.7 Ry the
 // norm of the error is 0.4 to 1.4e-17 of that of |A| |B|, where FP64 has 0.4 to 1.9e-16; at E = 0.02 +
 // 0.02 i, where the digits without the balance lose to FP64 (0.9 to 3.5e-16), 0.3 to 2.2e-17 against 0.3
-// to 0.7e-16.
+// to 0.7e-16.  Whole solves, gradients and inverses are as close to 64 bits as with FP64 products (tau00 of
+// contours 6.3e-13 with either).
 //
 // A complex C (m x n) is the real matrix with rows 2r, 2r + 1 = (re, im): C = At Bh with Bh column c =
 // (Br[0], Bi[0], Br[1], ...) and At the 2 x 2 expansion [[ar, -ai], [ai, ar]] (as in tc_update.cu), K =

@@ -1,5 +1,5 @@
-// Dataflow block sweeps of the correction solve: FP32 factors, b <= 16, the products on the
-// tensor cores.
+// Dataflow block sweeps of the correction solve: FP32 factors, 16 right-hand-side columns a cluster (b = 32:
+// two clusters a job), the products on the tensor cores.
 //
 // Same contract as the step-synchronous sweeps of sweep.cu (forward: Y_k = D_k R_k,
 // R[k+kb:N] -= A21_k Y_k; backward: X_k (+)= Y_k, Y[0:k] -= W[0:k, k] Y_k, i.e. zgetrs on the
@@ -56,7 +56,7 @@ using namespace cl;
 constexpr int kThreads = 256;             // compute threads (8 warps)
 constexpr int kBlock = kThreads + 64;     // and the producer and MMA warps
 constexpr int kWarps = kThreads / 32;
-constexpr int kCols = 16;                  // right-hand-side columns held (b <= 16)
+constexpr int kCols = 16;                  // right-hand-side columns of a cluster
 constexpr int kUnit = 32;                  // factor columns per unit: the MMA's K
 constexpr int kUnitFloats = 128 * kUnit;   // 128 real rows (the MMA's M) x 32 columns
 constexpr unsigned kUnitBytes = kUnitFloats * 4;
